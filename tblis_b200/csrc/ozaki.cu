@@ -1723,9 +1723,9 @@ void crt_run(OzakiJob& j, int nm, cudaStream_t st)
         oz_crt_shifts<<<(unsigned)((v.l*v.n + 255)/256), 256, 0, st>>>(j.sB.as<double>(), v.l*v.n, P, shB.as<int>());
         check_launch("oz_crt_shifts");
     }
-    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, v.amode,
+    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
                     j.tab->a_m_step, j.tab->a_k_step};
-    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, v.bmode,
+    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
                     j.tab->b_n_step, j.tab->b_k_step};
     // 128-row tiles of A and B, an even number of each: a CTA pair takes
     // 256 rows of A and 256 columns (two B tiles) of the output
@@ -1816,9 +1816,9 @@ void ozaki_begin(OzakiJob& j, cudaStream_t st)
     j.eB = dbuf((size_t)v.l*v.n*sizeof(int), st);
     j.sA = dbuf((size_t)v.l*v.m*sizeof(double), st);
     j.sB = dbuf((size_t)v.l*v.n*sizeof(double), st);
-    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, v.amode,
+    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
                     j.tab->a_m_step, j.tab->a_k_step};
-    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, v.bmode,
+    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
                     j.tab->b_n_step, j.tab->b_k_step};
     stats(oa, j.eA.as<int>(), j.sA.as<double>(), st);
     stats(ob, j.eB.as<int>(), j.sB.as<double>(), st);
@@ -1903,9 +1903,9 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
     TB_CHECK(S >= 1 && S <= OZ_SMAX, TB_ERR_ARG, "Ozaki slice count must be 1..8");
     j.res.slices = S;
 
-    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, v.amode,
+    OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
                     j.tab->a_m_step, j.tab->a_k_step};
-    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, v.bmode,
+    OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
                     j.tab->b_n_step, j.tab->b_k_step};
     const int esz = elem_bytes(kind);
     const i64 ke = OZ_BK/esz;              // k elements per MMA step

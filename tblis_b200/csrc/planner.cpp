@@ -444,6 +444,61 @@ void gemm_pair_modes(const GemmView& v, const i64* a_m, const i64* a_k, const i6
     b_pairs[1] = lb && bk_adj >= q && bn_even >= q;
 }
 
+// Offsets of a row (or column) group in an order that serves both tensors it
+// indexes. The view's order starts at C's smallest stride; where the operand's
+// contiguous dimension is another one and the operand is gathered along its
+// rows, a tile of rows then holds that dimension at one index only and every
+// 8-byte copy takes a 32-byte sector of its own. Instead the two dimensions are
+// walked in blocks of 16 (operand) x 8 (C), the operand's fastest: the gather
+// reads runs of 16 elements and C is still written in runs of 8. Any order is a
+// GEMM view as long as both vectors follow it. Returns false where the view's
+// order already serves it.
+static bool blocked_rows(const ivec& len, const ivec& op, const ivec& c, i64* op_out, i64* c_out)
+{
+    const size_t nd = len.size();
+    size_t u = 0, w = 0;
+    for (size_t d = 1; d < nd; d++)
+    {
+        if (std::llabs(op[d]) < std::llabs(op[u])) u = d;
+        if (std::llabs(c[d]) < std::llabs(c[w])) w = d;
+    }
+    // (a dimension of stride 4 and up shares no sector either way)
+    if (nd < 2 || u == 0 || std::llabs(op[u]) >= 4) return false;
+    if (w == u) w = u == 0 ? 1 : 0;
+    i64 outer = 1;
+    for (size_t d = 0; d < nd; d++) if (d != u && d != w) outer *= len[d];
+    const i64 bu = std::min<i64>(16, len[u]), bw = std::max<i64>(8, 128/bu);
+    i64 at = 0;
+    for (i64 o = 0; o < outer; o++)
+    {
+        i64 x = o, po = 0, pc = 0;
+        for (size_t d = 0; d < nd; d++)
+        {
+            if (d == u || d == w) continue;
+            po += x % len[d]*op[d];
+            pc += x % len[d]*c[d];
+            x /= len[d];
+        }
+        for (i64 w0 = 0; w0 < len[w]; w0 += bw)
+            for (i64 u0 = 0; u0 < len[u]; u0 += bu)
+                for (i64 j = w0; j < std::min(w0 + bw, len[w]); j++)
+                    for (i64 i = u0; i < std::min(u0 + bu, len[u]); i++, at++)
+                    {
+                        op_out[at] = po + i*op[u] + j*op[w];
+                        c_out[at] = pc + i*c[u] + j*c[w];
+                    }
+    }
+    return true;
+}
+
+// gathered along the rows (0) or along k (1): whichever holds the operand's
+// smallest stride
+static int gather_mode(const ivec& rows, const ivec& k)
+{
+    auto least = [](const ivec& s) { i64 m = (i64)1 << 62; for (i64 x : s) m = std::min<i64>(m, std::llabs(x)); return m; };
+    return least(rows) < least(k) ? 0 : 1;
+}
+
 std::shared_ptr<GemmTables> gemm_tables(const GemmView& v, i64 BM, i64 BN, i64 BK,
                                         cudaStream_t stream)
 {
@@ -477,10 +532,17 @@ std::shared_ptr<GemmTables> gemm_tables(const GemmView& v, i64 BM, i64 BN, i64 B
     i64 *a_kbs = p; p += nkb; i64 *b_kbs = p; p += nkb;
 
     std::vector<i64> bs(std::max({v.m, v.n, v.k, v.l}));
-    fill_block_scatter(v.lenM, v.aM, BM, 0, v.m, a_m, bs.data(), v.pack_m_3d);
-    fill_block_scatter(v.lenM, v.cM, BM, 0, v.m, c_m, bs.data(), v.pack_m_3d);
-    fill_block_scatter(v.lenN, v.bN, BN, 0, v.n, b_n, bs.data(), v.pack_n_3d);
-    fill_block_scatter(v.lenN, v.cN, BN, 0, v.n, c_n, bs.data(), v.pack_n_3d);
+    const int amode = gather_mode(v.aM, v.aK), bmode = gather_mode(v.bN, v.bK);
+    if (amode != 0 || !blocked_rows(v.lenM, v.aM, v.cM, a_m, c_m))
+    {
+        fill_block_scatter(v.lenM, v.aM, BM, 0, v.m, a_m, bs.data(), v.pack_m_3d);
+        fill_block_scatter(v.lenM, v.cM, BM, 0, v.m, c_m, bs.data(), v.pack_m_3d);
+    }
+    if (bmode != 0 || !blocked_rows(v.lenN, v.bN, v.cN, b_n, c_n))
+    {
+        fill_block_scatter(v.lenN, v.bN, BN, 0, v.n, b_n, bs.data(), v.pack_n_3d);
+        fill_block_scatter(v.lenN, v.cN, BN, 0, v.n, c_n, bs.data(), v.pack_n_3d);
+    }
     fill_block_scatter(v.lenK, v.aK, BK, 0, v.k, a_k, bs.data(), v.pack_k_3d);
     for (i64 b = 0; b < nkb; b++) a_kbs[b] = bs[b*BK];
     fill_block_scatter(v.lenK, v.bK, BK, 0, v.k, b_k, bs.data(), v.pack_k_3d);
@@ -490,6 +552,8 @@ std::shared_ptr<GemmTables> gemm_tables(const GemmView& v, i64 BM, i64 BN, i64 B
     fill_block_scatter(v.lenL, v.cL, 1, 0, v.l, c_l, bs.data(), false);
 
     auto t = std::make_shared<GemmTables>();
+    t->amode = amode;
+    t->bmode = bmode;
     t->a_m_step = affine_step(a_m, v.m); t->a_k_step = affine_step(a_k, v.k);
     t->b_n_step = affine_step(b_n, v.n); t->b_k_step = affine_step(b_k, v.k);
     gemm_pair_modes(v, a_m, a_k, b_n, b_k, a_l, b_l, t->a_pairs, t->b_pairs);
