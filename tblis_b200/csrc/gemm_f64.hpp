@@ -22,7 +22,19 @@ struct GemmF64Args
     i64 k_per_split;         // set by the launcher
     double* partial;         // split-K workspace (splits*L*M*N doubles)
     int variant;             // tile configuration, 0 = automatic
+    // complex contraction (dense kernel only; offsets and extents in complex
+    // elements, every element 16-byte aligned)
+    int cplx, conj_a, conj_b, conj_c;
+    double alpha_im, beta_im;
     int pair_a, pair_b;      // gather the operand's contiguous dimension in pairs (16-byte copies)
+    // set by gemm_f64_dense_plan: k steps of a tile, tiles done whole, tiles
+    // whose k steps are cut into equal runs over sk_ctas CTAs, CTAs, workspace
+    // (tile: 0 = 128 x 128, 1 = 64 x 64, 2 = 128 x 32), and of the cut tiles the
+    // first of each class, its cost per k step and the cost per CTA
+    i64 kt, dp_tiles, sk_tiles;
+    int sk_ctas, cut, grid, tile;
+    unsigned sk_per, sk_extra, cls_first[5], cls_w[4];
+    size_t ws_bytes;
 };
 
 // one K segment of a grouped GEMM: the rows of A / columns of B it reads
@@ -107,5 +119,12 @@ i64 gemm_f64_tile_k();
 int gemm_f64_choose_splits(i64 M, i64 N, i64 K, i64 L, int num_sms);
 size_t gemm_f64_workspace_bytes(i64 M, i64 N, i64 L, int splits);
 void gemm_f64_launch(GemmF64Args a, cudaStream_t stream);
+
+// The dense kernel (gemm_f64_dense.cu): plan sets the work split for `sms` SMs
+// and a.ws_bytes, at most ws_limit bytes of workspace for a.partial; launch
+// runs it.
+void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit);
+void gemm_f64_dense_launch(const GemmF64Args& a, cudaStream_t stream);
+int gemm_f64_dense_error_flag();
 
 } // namespace tb

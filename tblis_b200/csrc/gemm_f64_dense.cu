@@ -1,0 +1,1101 @@
+// gemm_f64_dense.cu -- the dense FP64 contraction kernel: one persistent,
+// warp-specialised CTA per SM over the GEMM view of strided tensors.
+//
+// Replaces TBLIS's pack + microkernel + scatter-accumulate chain
+// (src/nodes/packm.hpp:79-124, src/kernels/3m/packm.hpp:292-403,
+// src/nodes/gemm_ukr.hpp:16-126) for one contraction: operand tiles are
+// gathered straight from the strided tensors through the scatter vectors, the
+// alpha/beta update of C is scattered back from the accumulators, and
+// beta == 0 never reads C.
+//
+// What bounds it: the FP64 tensor pipe (DMMA, 64 FMA per cycle and SM).
+// A 64 x 64 tile needs 16 operand bytes per cycle and SM from L2 at that
+// rate, 4.5 TB/s over the chip, and its CTA-wide barriers stop all warps once
+// per 16 k; it measured 29.7 TFLOP/s at 7680^3. Here a tile is 128 x 128 (8
+// bytes per cycle and SM), four producer warps gather it with cp.async into a
+// ring of 16-wide k stages whose mbarriers they alone feed, and eight consumer
+// warps (two per SM sub-core, so one's fragment loads hide behind the other's
+// MMAs) release each stage as soon as its fragments are in registers. No
+// barrier spans the CTA after the start. Measured: 7680^3 in 27.4 ms (30.4 before,
+// cuBLAS 25.3), 97 x 97 x 93217 in 102 us (283), 3007^3 with permuted operands in
+// 1.95 ms (2.97), complex 1728^3 in 1.38 ms (2.58 as four real contractions).
+//
+// Fragments are dealt to the warps cyclically (16-row fragment f of the tile
+// to row-warp f % WGM, 8-column fragment g to column-warp g % WGN), and
+// fragments past M or N are neither gathered nor multiplied, so a ragged
+// edge costs what it holds, evenly over the sub-cores, instead of a tile.
+//
+// Work split: whole waves of whole tiles go to the CTAs in launch order
+// (neighbouring CTAs share A and B panels in L2); the whole tiles left over, one
+// more wave of them and all ragged tiles are cut into runs of k steps of equal
+// cost, one per CTA, so no SM idles in the last wave and a contraction of few
+// tiles and a long sum still fills the chip. A run that covers part of a
+// tile leaves its accumulators in a workspace (at most two per CTA) and
+// gemm_f64_fixup sums them in CTA order: the result does not depend on
+// scheduling, and no kernel waits for another CTA.
+//
+// Every wait is bounded (2 s of wall clock): one that gives up ends the CTA's
+// work and records the error for the host (gemm_f64_dense_error_flag).
+#include "gemm_f64.hpp"
+#include "gemm_f64_dev.cuh"
+
+#include <algorithm>
+#include <cmath>
+#include <type_traits>
+
+namespace tb
+{
+
+namespace
+{
+
+using namespace f64dev;
+
+constexpr int DN_PRODUCERS = 4, DN_CONSUMERS = 8;           // warps (per team of producers)
+constexpr int DN_PT = DN_PRODUCERS*32, DN_CT = DN_CONSUMERS*32;
+constexpr unsigned long long DN_WAIT_NS = 2000000000ull;    // 2 s
+// registers per thread at launch, and after the split between the roles (a sum
+// over the warps above the launch's would wait forever)
+constexpr int dn_threads(int teams) { return teams*DN_PT + DN_CT; }
+constexpr int dn_reg_launch(int teams) { return teams == 1 ? 168 : 128; }
+constexpr int dn_reg_p(int teams) { return teams == 1 ? 104 : 72; }
+constexpr int dn_reg_c(int teams) { return teams == 1 ? 200 : 184; }
+static_assert(DN_PT*dn_reg_p(1) + DN_CT*dn_reg_c(1) <= dn_threads(1)*dn_reg_launch(1), "register split");
+static_assert(2*DN_PT*dn_reg_p(2) + DN_CT*dn_reg_c(2) <= dn_threads(2)*dn_reg_launch(2), "register split");
+
+__device__ int g_dn_error = 0;
+
+// smem position of element (row, k) of an operand tile of R rows and 16 k.
+// MODE 0 (gathered along the rows): k rows of R doubles; MODE 1 (along k):
+// rows of 16 doubles. XOR swizzles in units of four doubles keep the 8 x 4
+// fragment reads free of bank conflicts and element pairs adjacent.
+template <int R, int MODE>
+__device__ __forceinline__ int tile_pos(int row, int k)
+{
+    return MODE == 0 ? k*R + (row ^ ((k & 3) << 2)) : row*BK + (k ^ ((row & 3) << 2));
+}
+
+__device__ __forceinline__ bool dn_wait_slow(uint64_t* b, uint32_t parity, volatile int* abort_flag)
+{
+    const unsigned long long t0 = gtimer();
+    for (unsigned it = 0;; it++)
+    {
+        if (mb_try(b, parity)) return true;
+        if ((it & 63) == 0)
+        {
+            if (*abort_flag) return false;
+            if (gtimer() - t0 > DN_WAIT_NS)
+            {
+                *abort_flag = 1;
+                atomicExch(&g_dn_error, 1);
+                return false;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ bool dn_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag)
+{
+    const bool ok = mb_try(b, parity) || dn_wait_slow(b, parity, abort_flag);
+    return __all_sync(0xffffffffu, ok) != 0;
+}
+
+// one run of k steps of one tile
+struct Run
+{
+    unsigned tile;
+    int s0, s1;               // k steps [s0, s1)
+    int slot;                 // -1: the whole tile (C is updated), else the CTA's workspace slot
+};
+
+// Tiles are numbered class by class: whole tiles, the ragged last row of tiles,
+// the ragged last column, the corner; a class costs cls_w per k step. The k
+// steps ("units") of the cut tiles are dealt so that every CTA gets the same
+// cost: CTA c starts at the first unit at or past cost c*sk_per + min(c,
+// sk_extra).
+
+// cost of the units before unit u (of the cut tiles)
+__device__ __forceinline__ unsigned unit_cost(const GemmF64Args& p, unsigned u)
+{
+    const unsigned kt = (unsigned)p.kt, tile = u/kt, step = u - tile*kt;
+    unsigned cost = 0;
+    #pragma unroll
+    for (int c = 0; c < 4; c++)
+    {
+        // the cut tiles of class c, counted from the first cut one
+        const unsigned b = p.cls_first[c], e = p.cls_first[c + 1];
+        const unsigned n = min(max(tile, b), e) - b;
+        cost += n*kt*p.cls_w[c];
+        if (tile >= b && tile < e) cost += step*p.cls_w[c];
+    }
+    return cost;
+}
+
+// first unit of CTA c
+__device__ __forceinline__ unsigned first_unit(const GemmF64Args& p, unsigned c)
+{
+    unsigned at = c*p.sk_per + min(c, p.sk_extra);
+    const unsigned kt = (unsigned)p.kt;
+    #pragma unroll
+    for (int k = 0; k < 4; k++)
+    {
+        const unsigned b = p.cls_first[k], e = p.cls_first[k + 1], w = p.cls_w[k];
+        const unsigned all = (e - b)*kt*w;
+        if (at <= all && e > b) return b*kt + (at + w - 1)/w;
+        at -= all;
+    }
+    return p.cls_first[4]*kt;
+}
+
+// the CTA that holds unit u
+__device__ __forceinline__ unsigned cta_of_unit(const GemmF64Args& p, unsigned u)
+{
+    const unsigned at = unit_cost(p, u), big = p.sk_extra*(p.sk_per + 1);
+    return at < big ? at/(p.sk_per + 1) : p.sk_extra + (at - big)/p.sk_per;
+}
+
+// Run number r of CTA `cta`: its whole tiles, then its share of the k steps of
+// the cut tiles [dp_tiles, dp_tiles + sk_tiles). Computed anew from r where it
+// is needed, so that the accumulators have the registers. 32-bit arithmetic:
+// the plan keeps tiles and units below 2^31.
+__device__ __forceinline__ bool run_at(const GemmF64Args& p, unsigned cta, unsigned r, Run& out)
+{
+    const unsigned kt = (unsigned)p.kt, dp = (unsigned)p.dp_tiles;
+    const unsigned mine = r*gridDim.x + cta;
+    if (mine < dp)
+    {
+        out = Run{mine, 0, (int)kt, -1};
+        return true;
+    }
+    if (cta >= (unsigned)p.sk_ctas) return false;
+    const unsigned nd = dp > cta ? (dp - cta - 1)/gridDim.x + 1 : 0;
+    const unsigned u0 = first_unit(p, cta), u1 = first_unit(p, cta + 1);
+    const unsigned t0 = u0/kt, t = t0 + (r - nd);
+    const unsigned b = max(u0, t*kt), e = min(u1, (t + 1)*kt);
+    if (b >= e) return false;
+    out.tile = dp + t;
+    out.s0 = (int)(b - t*kt);
+    out.s1 = (int)(e - t*kt);
+    // a partial run takes slot 0, the second one (after a first run that is
+    // part of an earlier tile) slot 1
+    out.slot = e - b == kt ? -1 : t > t0 && u0 != t0*kt ? 1 : 0;
+    return true;
+}
+
+struct TileAt
+{
+    i64 m0, n0;
+    unsigned l;
+    int mrem, nrem;           // rows and columns of the tile inside the GEMM
+};
+
+// Whole tiles: groups of 8 tile rows sweep the tile columns together, so
+// concurrent CTAs share panels of both operands in L2; then the ragged tiles.
+template <int BM, int BN>
+__device__ __forceinline__ TileAt tile_at(const GemmF64Args& p, unsigned tile)
+{
+    const i64 N = p.cplx ? 2*p.N : p.N;                       // real columns
+    const unsigned fm = (unsigned)(p.M/BM), fn = (unsigned)(N/BN);
+    const unsigned L = (unsigned)p.L, whole = fm*fn, bottom = p.M % BM ? fn : 0, right = N % BN ? fm : 0;
+    TileAt t;
+    t.l = 0;
+    unsigned row = fm, col = fn;
+    auto split = [&](unsigned n) { if (L > 1) { t.l = tile/n; tile -= t.l*n; } };
+    if (tile < whole*L)
+    {
+        split(whole);
+        const unsigned gid = tile/(8*fn), first = gid*8, in = tile - gid*8*fn;
+        const unsigned gs = min(8u, fm - first);
+        col = in/gs;
+        row = first + in - col*gs;
+    }
+    else if ((tile -= whole*L) < bottom*L) { split(bottom); col = tile; }
+    else if ((tile -= bottom*L) < right*L) { split(right); row = tile; }
+    else t.l = tile - right*L;
+    t.m0 = (i64)row*BM;
+    t.n0 = (i64)col*BN;
+    t.mrem = (int)min((i64)BM, p.M - t.m0);
+    t.nrem = (int)min((i64)BN, N - t.n0);
+    return t;
+}
+
+// ---- producers -----------------------------------------------------------------------
+
+// copies of one element or of a pair of elements (16-byte aligned); not ok:
+// zero-filled. They write stages that only the consumers read: no memory clobber,
+// so that a producer's address loads and arithmetic batch across its copies.
+__device__ __forceinline__ void cp_elem(double* dst, const double* src, bool ok = true)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" :: "r"(su32(dst)), "l"(src), "r"(ok ? 8 : 0));
+}
+
+__device__ __forceinline__ void cp_pair16(double* dst, const double* src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(su32(dst)), "l"(src));
+}
+
+// One operand of a run: this thread's share of the gather of a stage. With
+// pairs (the host found nearly all pairs of the gathered dimension adjacent and
+// 16-byte aligned) a lane takes two neighbouring elements, one 16-byte copy
+// where they are adjacent and aligned, else two of 8; without, lanes take
+// consecutive elements, so that 8-byte copies still cover whole lines. In mode 0
+// a thread's rows are fixed and it copies them at J of the stage's k, in mode 1
+// its k are fixed and it copies J rows. The k offsets are loaded four stages at
+// a time, four stages ahead (one stage ahead, small tiles waited for them: 0.8
+// us a stage), two to a lane, and handed round by shuffles.
+//
+// A producer warp runs alone on its issue slots, so what bounds it is the
+// latency of each copy's address arithmetic: the common case (a warp whose
+// copies all lie inside the GEMM, at k of one stride, pairs adjacent and aligned)
+// is a run of copies from one pointer; per-copy predicates and shuffles cost 150
+// to 200 cycles a copy and capped the gather at 7 to 11 bytes per cycle and SM.
+// Rows past the GEMM are not copied: whatever the stage holds there meets no
+// stored element of C. k past the end is zero-filled.
+template <int R, int MODE>
+struct Gather
+{
+    template <int W>
+    struct Geom
+    {
+        static constexpr int LANES = (MODE == 0 ? R : BK)/W;   // threads along the gathered dimension
+        static constexpr int STEP = DN_PT/LANES;               // groups of threads along the other one
+        static constexpr int J = (MODE == 0 ? BK : R)/STEP;    // copy slots per thread and stage
+        static_assert(DN_PT % LANES == 0 && J >= 1 && J*STEP == (MODE == 0 ? BK : R), "gather geometry");
+    };
+    const double* X;
+    const i64* kvec;
+    i64 ro[2];                                                // mode 0: the thread's row offsets
+    i64* sro;                                                 // mode 1: row offsets, each read by one warp only
+    i64 ko[2], kn[2];                                         // offsets of k lane and lane + 32 of four stages, and of the next four
+    int rem;                                                  // rows inside the GEMM
+    bool even;                                                // mode 1: this warp's row offsets are even
+
+    template <int W>
+    __device__ __forceinline__ void rows(const i64* rvec)
+    {
+        constexpr int LANES = Geom<W>::LANES, STEP = Geom<W>::STEP, J = Geom<W>::J;
+        const int t = threadIdx.x % DN_PT;
+        if constexpr (MODE == 0)
+        {
+            const int r = W*(t % LANES);
+            ro[0] = r < rem ? __ldg(rvec + r) : 0;
+            if (W == 2) ro[1] = r + 1 < rem ? __ldg(rvec + r + 1) : 0;
+        }
+        else
+        {
+            // the rows this warp copies: PER consecutive ones at each of J steps
+            constexpr int PER = 32/LANES;
+            int odd = 0;
+            __syncwarp();
+            for (int x = t % 32; x < PER*J; x += 32)
+            {
+                const int r = (t/32)*PER + x % PER + x/PER*STEP;
+                const i64 o = r < rem ? __ldg(rvec + r) : 0;
+                sro[r] = o;
+                odd |= (int)(o & 1);
+            }
+            even = __all_sync(0xffffffffu, odd == 0) != 0;
+            __syncwarp();
+        }
+    }
+
+    // loads the k offsets of the four stages from k0 on (up to k1) into kn
+    __device__ __forceinline__ void fetch(i64 k0, i64 k1)
+    {
+        const int lane = threadIdx.x & 31;
+        kn[0] = k0 + lane < k1 ? __ldg(kvec + k0 + lane) : 0;
+        kn[1] = k0 + 32 + lane < k1 ? __ldg(kvec + k0 + 32 + lane) : 0;
+    }
+    __device__ __forceinline__ void advance() { ko[0] = kn[0]; ko[1] = kn[1]; }
+
+    __device__ __forceinline__ void start(const double* X_, const i64* rvec, const i64* kvec_, i64 r0, int rem_,
+                                          bool pairs)
+    {
+        X = X_; kvec = kvec_;
+        rem = rem_;
+        if (pairs) rows<2>(rvec + r0);
+        else rows<1>(rvec + r0);
+    }
+
+    // copies stage u of the current four
+    template <int W>
+    __device__ __forceinline__ void copy(double* Xs, int u, int kvalid) const
+    {
+        const i64 mine = u & 2 ? ko[1] : ko[0];               // this stage's offsets, from lane base on
+        const int base = (u & 1)*BK;
+        constexpr int LANES = Geom<W>::LANES, STEP = Geom<W>::STEP, J = Geom<W>::J;
+        const int t = threadIdx.x % DN_PT;
+        if (MODE == 0)
+        {
+            const int lane = t & 31, r = W*(t % LANES), k0 = t/LANES;
+            const bool in = r < rem, two = W == 2 && r + 1 < rem, adj = two && ro[1] == ro[0] + 1;
+            const i64 first = __shfl_sync(0xffffffffu, mine, base);
+            const i64 step = __shfl_sync(0xffffffffu, mine, base + 1) - first;
+            const double* src = X + ro[0] + first + k0*step;
+            const bool other = ((lane ^ base) & BK) != 0;      // the offset this lane holds belongs to another stage
+            const bool fast = kvalid == BK && (other || mine == first + (lane - base)*step) &&
+                              (W == 1 || !in || (adj && (((uintptr_t)src | (uintptr_t)(8*STEP*step)) & 15) == 0));
+            if (__all_sync(0xffffffffu, fast))
+            {
+                if (!in) return;
+                #pragma unroll
+                for (int j = 0; j < J; j++)
+                {
+                    double* dst = Xs + tile_pos<R, MODE>(r, k0 + j*STEP);
+                    if (W == 2) cp_pair16(dst, src);
+                    else cp_elem(dst, src);
+                    src += STEP*step;
+                }
+                return;
+            }
+            // any k offsets: all shuffles before the copies
+            i64 k[J];
+            #pragma unroll
+            for (int j = 0; j < J; j++) k[j] = __shfl_sync(0xffffffffu, mine, base + k0 + j*STEP);
+            const bool whole = kvalid == BK && (W == 1 || other || (mine & 1) == 0) &&
+                               (W == 1 || !in || (adj && ((uintptr_t)(X + ro[0]) & 15) == 0));
+            if (__all_sync(0xffffffffu, whole))
+            {
+                if (!in) return;
+                #pragma unroll
+                for (int j = 0; j < J; j++)
+                {
+                    double* dst = Xs + tile_pos<R, MODE>(r, k0 + j*STEP);
+                    if (W == 2) cp_pair16(dst, X + ro[0] + k[j]);
+                    else cp_elem(dst, X + ro[0] + k[j]);
+                }
+                return;
+            }
+            if (!in) return;
+            #pragma unroll
+            for (int j = 0; j < J; j++)
+            {
+                const int kl = k0 + j*STEP;
+                const bool ok = kl < kvalid;
+                src = X + ro[0] + k[j];
+                double* dst = Xs + tile_pos<R, MODE>(r, kl);
+                if (W == 2 && ok && adj && ((uintptr_t)src & 15) == 0) cp_pair16(dst, src);
+                else
+                {
+                    cp_elem(dst, src, ok);
+                    if (two) cp_elem(dst + 1, X + ro[1] + k[j], ok);
+                }
+            }
+        }
+        else
+        {
+            const int kl = W*(t % LANES);
+            const i64 o0 = __shfl_sync(0xffffffffu, mine, base + kl);
+            const i64 o1 = W == 2 ? __shfl_sync(0xffffffffu, mine, base + kl + W - 1) : 0;
+            const bool adj = W == 2 && o1 == o0 + 1;
+            const double* Xk = X + o0;
+            const bool fast = kvalid == BK && (W == 1 || (adj && even && ((uintptr_t)Xk & 15) == 0));
+            if (__all_sync(0xffffffffu, fast))
+            {
+                if (rem < R)
+                {
+                    #pragma unroll 4
+                    for (int r = t/LANES; r < rem; r += STEP)
+                    {
+                        double* dst = Xs + tile_pos<R, MODE>(r, kl);
+                        if (W == 2) cp_pair16(dst, Xk + sro[r]);
+                        else cp_elem(dst, Xk + sro[r]);
+                    }
+                    return;
+                }
+                #pragma unroll
+                for (int j = 0; j < J; j++)
+                {
+                    const int r = t/LANES + j*STEP;
+                    double* dst = Xs + tile_pos<R, MODE>(r, kl);
+                    if (W == 2) cp_pair16(dst, Xk + sro[r]);
+                    else cp_elem(dst, Xk + sro[r]);
+                }
+                return;
+            }
+            const bool ok0 = kl < kvalid, ok1 = W == 2 && kl + 1 < kvalid;
+            #pragma unroll 4
+            for (int j = 0; j < J; j++)
+            {
+                const int r = t/LANES + j*STEP;
+                if (r >= rem) break;
+                const i64 row = sro[r];
+                double* dst = Xs + tile_pos<R, MODE>(r, kl);
+                if (adj && ok1 && ((uintptr_t)(Xk + row) & 15) == 0) cp_pair16(dst, Xk + row);
+                else
+                {
+                    cp_elem(dst, Xk + row, ok0);
+                    if (W == 2) cp_elem(dst + 1, X + row + o1, ok1);
+                }
+            }
+        }
+    }
+
+    __device__ __forceinline__ void stage(double* Xs, int u, int kvalid, bool pairs) const
+    {
+        if (pairs) copy<2>(Xs, u, kvalid);
+        else copy<1>(Xs, u, kvalid);
+    }
+};
+
+// zero-filled when not ok
+__device__ __forceinline__ void cp_pair16(double* dst, const double* src, bool ok)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(su32(dst)), "l"(src), "r"(ok ? 16 : 0));
+}
+
+// The gather of a complex operand (R rows of BK/2 complex k; 16-byte aligned
+// elements, offsets in elements). Real and imaginary part stay together, so one
+// stage layout (tile_pos MODE 1, part p of complex k at real k 2k + p) and one
+// 16-byte copy per element serve both gather directions: rows = true takes
+// lanes along the rows, else along k.
+template <int R>
+struct GatherZ
+{
+    static constexpr int KS = BK/2;                           // complex k per stage
+    static constexpr int STEP0 = DN_PT/R, J0 = KS/STEP0;      // along the rows: k per pass, copies per thread
+    static constexpr int STEP1 = DN_PT/KS, J1 = R/STEP1;      // along k: rows per pass
+    static_assert(DN_PT % R == 0 && J0*STEP0 == KS && J1*STEP1 == R, "gather geometry");
+    const double* X;
+    const i64* kvec;
+    i64 ro;
+    i64* sro;                                                 // along k: row offsets, each read by one warp only
+    i64 ko, kn;                                               // offset of k lane of four stages, and of the next four
+    int rem;
+
+    __device__ __forceinline__ void fetch(i64 k0, i64 k1)
+    {
+        const int lane = threadIdx.x & 31;
+        kn = k0 + lane < k1 ? __ldg(kvec + k0 + lane) : 0;
+    }
+    __device__ __forceinline__ void advance() { ko = kn; }
+    __device__ __forceinline__ void start(const double* X_, const i64* rvec, const i64* kvec_, i64 r0, int rem_,
+                                          bool rows)
+    {
+        X = X_; kvec = kvec_;
+        rem = rem_;
+        rvec += r0;
+        const int t = threadIdx.x % DN_PT;
+        ro = rows && t % R < rem ? __ldg(rvec + t % R) : 0;
+        if (rows) return;
+        constexpr int PER = 32/KS;
+        __syncwarp();
+        for (int x = t % 32; x < PER*J1; x += 32)
+        {
+            const int r = (t/32)*PER + x % PER + x/PER*STEP1;
+            sro[r] = r < rem ? __ldg(rvec + r) : 0;
+        }
+        __syncwarp();
+    }
+    __device__ __forceinline__ void stage(double* Xs, int u, int kvalid, bool rows) const
+    {
+        const int t = threadIdx.x % DN_PT, base = u*KS;
+        if (rows)
+        {
+            const int r = t % R, k0 = t/R;
+            i64 k[J0];
+            #pragma unroll
+            for (int j = 0; j < J0; j++) k[j] = __shfl_sync(0xffffffffu, ko, base + k0 + j*STEP0);
+            if (r >= rem) return;
+            #pragma unroll
+            for (int j = 0; j < J0; j++)
+            {
+                const int kl = k0 + j*STEP0;
+                cp_pair16(Xs + tile_pos<R, 1>(r, 2*kl), X + 2*(ro + k[j]), kl < kvalid);
+            }
+        }
+        else
+        {
+            const int kl = t % KS;
+            const double* Xk = X + 2*__shfl_sync(0xffffffffu, ko, base + kl);
+            #pragma unroll
+            for (int j = 0; j < J1; j++)
+            {
+                const int r = t/KS + j*STEP1;
+                if (r >= rem) break;
+                cp_pair16(Xs + tile_pos<R, 1>(r, 2*kl), Xk + 2*sro[r], kl < kvalid);
+            }
+        }
+    }
+};
+
+// ---- kernel ---------------------------------------------------------------------------
+
+// Row-warp and column-warp of a consumer warp. Warps cw and cw + 4 share an SM
+// sub-core: shifting the columns of the second row-warp gives a ragged edge's
+// longer and shorter shares to the same sub-core.
+template <int WGN>
+__device__ __forceinline__ void warp_at(int cw, int& wm, int& wn)
+{
+    wm = cw/WGN;
+    wn = (cw + (WGN/2)*wm) % WGN;
+}
+
+template <int STAGES>
+struct DnShared
+{
+    uint64_t full[STAGES], empty[STAGES];
+    int abort;
+};
+
+template <int WGM, int WGN, int MF, int NF, int STAGES, int TEAMS>
+constexpr size_t dn_smem()
+{
+    return (size_t)(STAGES*BK + TEAMS)*(WGM*MF*16 + WGN*NF*8)*sizeof(double) + sizeof(DnShared<STAGES>);
+}
+
+// x with its sign bit flipped by the mask
+__device__ __forceinline__ double flip(double x, unsigned mask)
+{
+    return __hiloint2double(__double2hiint(x) ^ (int)mask, __double2loint(x));
+}
+
+// alpha*x + beta*op(c) over a complex element of C (beta == 0: c is not read)
+__device__ __forceinline__ void update_z(const GemmF64Args& p, double* dst, double re, double im)
+{
+    double vr = p.alpha*re - p.alpha_im*im, vi = p.alpha*im + p.alpha_im*re;
+    if (p.beta != 0.0 || p.beta_im != 0.0)
+    {
+        const double cr = dst[0], ci = p.conj_c ? -dst[1] : dst[1];
+        vr += p.beta*cr - p.beta_im*ci;
+        vi += p.beta*ci + p.beta_im*cr;
+    }
+    *reinterpret_cast<double2*>(dst) = make_double2(vr, vi);
+}
+
+// calls f with the fragment counts as constants: an MMA under a run-time
+// condition is predicated, and the pipe takes as long for one that is off
+template <int MF, int NF, typename F>
+__device__ __forceinline__ bool dn_fragments(int ni, int nj, F&& f)
+{
+    if (ni <= 0 || nj <= 0) return f(std::integral_constant<int, 0>(), std::integral_constant<int, 0>());
+    bool ok = true;
+    auto columns = [&](auto i)
+    {
+        if (nj == 1) ok = f(i, std::integral_constant<int, 1>());
+        else if (NF <= 2 || nj == 2) ok = f(i, std::integral_constant<int, (NF < 2 ? NF : 2)>());
+        else if (nj == 3) ok = f(i, std::integral_constant<int, (NF < 3 ? NF : 3)>());
+        else ok = f(i, std::integral_constant<int, NF>());
+    };
+    if (ni == 1) columns(std::integral_constant<int, 1>());
+    else if (MF <= 2 || ni == 2) columns(std::integral_constant<int, (MF < 2 ? MF : 2)>());
+    else if (ni == 3) columns(std::integral_constant<int, (MF < 3 ? MF : 3)>());
+    else columns(std::integral_constant<int, MF>());
+    return ok;
+}
+
+// CPLX: a complex contraction as a real one of M x 2N x 2K: the columns of C
+// and the k of A are (real, imaginary) pairs as they lie in memory, and the 2 x 2
+// real block of each element of B, ((re, im), (-im, re)), is formed from the one
+// stored copy as the fragments are read: column parity q and k parity p pick
+// part p ^ q and a sign. N, K and the scatter vectors stay in complex units in
+// the arguments; M x 2N tiles of 16 real k (8 complex) are what the tile loop
+// sees.
+template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS, int AMODE, int BMODE, bool CPLX>
+__global__ void __launch_bounds__(dn_threads(TEAMS), 1)
+gemm_f64_dense_kernel(const GemmF64Args p)
+{
+    static_assert(WGM*WGN == DN_CONSUMERS, "consumer warps");
+    static_assert(STAGES % TEAMS == 0 && LAG*TEAMS < STAGES, "ring");
+    constexpr bool SPLIT = MF*NF > 4;             // small accumulators: the launch's registers serve both roles
+    constexpr int BM = WGM*MF*16, BN = WGN*NF*8;
+    constexpr int STAGE = BK*(BM + BN);
+    extern __shared__ __align__(128) double smem[];
+    i64* sro = reinterpret_cast<i64*>(smem + STAGES*STAGE);        // each team's row offsets of A, then of B
+    DnShared<STAGES>& sh = *reinterpret_cast<DnShared<STAGES>*>(sro + TEAMS*(BM + BN));
+    volatile int* abort_flag = &sh.abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0)
+    {
+        for (int s = 0; s < STAGES; s++)
+        {
+            mb_init(&sh.full[s], DN_PRODUCERS);       // one arrival per producer warp, its copies landed
+            mb_init(&sh.empty[s], DN_CONSUMERS);      // one arrival per consumer warp
+        }
+        sh.abort = 0;
+    }
+    __syncthreads();
+    // from here on the roles never wait on a CTA-wide barrier
+
+    Run run;
+    uint32_t st = 0, phase = 0;                       // ring position
+    if (warp < TEAMS*DN_PRODUCERS)
+    {
+        if (SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" :: "n"(dn_reg_p(TEAMS)));
+        // two teams take the stages in turn
+        const int team = warp/DN_PRODUCERS;
+        int turn = 0;
+        // complex: the gather directions
+        const bool pair_a = CPLX ? p.amode == 0 : p.pair_a != 0, pair_b = CPLX ? p.bmode == 0 : p.pair_b != 0;
+        bool ok = true;
+        bool wrapped = false;                         // the first round of stages starts empty
+        // A warp publishes a stage LAG stages after it issued it, when its copies
+        // have landed: LAG stages are in flight. (An mbarrier arrival tied to the
+        // copies, cp.async.mbarrier.arrive, held the warp's later copies back
+        // until it had fired.) LAG covers the memory latency at the tile's cycles
+        // per stage; a longer one only delays a run's first stage.
+        int lag = 0;
+        uint32_t pub = team;                          // the team's next stage to publish
+        for (unsigned r = 0; ok && run_at(p, blockIdx.x, r, run); r++)
+        {
+            const TileAt t = tile_at<BM, BN>(p, run.tile);
+            constexpr int KS = CPLX ? BK/2 : BK;               // k of the scatter vectors per stage
+            typename std::conditional<CPLX, GatherZ<BM>, Gather<BM, AMODE>>::type ga;
+            typename std::conditional<CPLX, GatherZ<BN/2>, Gather<BN, BMODE>>::type gb;
+            ga.sro = sro + team*(BM + BN);
+            gb.sro = ga.sro + BM;
+            constexpr int ES = CPLX ? 2 : 1;                   // doubles per element
+            const i64 k_begin = (i64)run.s0*KS, k_end = min(p.K, (i64)run.s1*KS);
+            ga.start(p.A + ES*p.a_l[t.l], p.a_m, p.a_k, t.m0, t.mrem, pair_a);
+            gb.start(p.B + ES*p.b_l[t.l], p.b_n, p.b_k, t.n0/ES, t.nrem/ES, pair_b);
+            ga.fetch(k_begin, k_end);
+            gb.fetch(k_begin, k_end);
+            int u = 0;
+            for (i64 k0 = k_begin; k0 < k_end; k0 += KS)
+            {
+                if (u == 0)
+                {
+                    ga.advance();
+                    gb.advance();
+                    ga.fetch(k0 + 4*KS, k_end);
+                    gb.fetch(k0 + 4*KS, k_end);
+                }
+                if (turn == team)
+                {
+                    if (wrapped && !dn_wait(&sh.empty[st], phase ^ 1, abort_flag))
+                    {
+                        ok = false;
+                        break;
+                    }
+                    const int kvalid = (int)min((i64)KS, k_end - k0);
+                    double* As = smem + st*STAGE;
+                    ga.stage(As, u, kvalid, pair_a);
+                    gb.stage(As + BK*BM, u, kvalid, pair_b);
+                    cp_async_commit();
+                    if (lag < LAG) lag++;
+                    else
+                    {
+                        cp_async_wait<LAG>();
+                        __syncwarp();
+                        if (lane == 0) mb_arrive(&sh.full[pub]);
+                        pub = (pub + TEAMS) % STAGES;
+                    }
+                }
+                if (TEAMS > 1) turn ^= 1;
+                u = (u + 1) & 3;
+                if (++st == STAGES) { st = 0; phase ^= 1; wrapped = true; }
+            }
+        }
+        // the last stages (also after a wait that gave up: the copies land before
+        // the CTA is gone)
+        cp_async_wait<0>();
+        __syncwarp();
+        for (; ok && lag > 0; lag--)
+        {
+            if (lane == 0) mb_arrive(&sh.full[pub]);
+            pub = (pub + TEAMS) % STAGES;
+        }
+        return;
+    }
+
+    if (SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" :: "n"(dn_reg_c(TEAMS)));
+    int wm, wn;
+    warp_at<WGN>(warp - TEAMS*DN_PRODUCERS, wm, wn);
+    const int fr = lane >> 2, fc = lane & 3;
+    // (Ar + i sa Ai)(Br + i sb Bi): sign of the part of B at this lane's column
+    // parity fr & 1 (0: real) and k parity fc & 1 (0: Ar)
+    unsigned sign = 0;
+    if (CPLX)
+    {
+        const bool col_im = fr & 1, k_im = fc & 1;
+        const bool neg = k_im ? (col_im ? p.conj_a != 0 : (p.conj_a != 0) == (p.conj_b != 0)) : col_im && p.conj_b;
+        sign = neg ? 0x80000000u : 0u;
+    }
+    for (unsigned r = 0; run_at(p, blockIdx.x, r, run); r++)
+    {
+        TileAt t = tile_at<BM, BN>(p, run.tile);
+        // fragments of this warp inside the GEMM: 16-row fragment i*WGM + wm, 8-column fragment j*WGN + wn
+        const int ni = min(MF, max(0, ((t.mrem + 15)/16 - wm + WGM - 1)/WGM));
+        const int nj = min(NF, max(0, ((t.nrem + 7)/8 - wn + WGN - 1)/WGN));
+        double acc[MF][NF][4];
+        #pragma unroll
+        for (int i = 0; i < MF; i++)
+            #pragma unroll
+            for (int j = 0; j < NF; j++)
+                #pragma unroll
+                for (int q = 0; q < 4; q++) acc[i][j][q] = 0.0;
+
+        const bool ok = dn_fragments<MF, NF>(ni, nj, [&](auto ni_, auto nj_)
+        {
+            constexpr int NI = decltype(ni_)::value, NJ = decltype(nj_)::value;
+            for (int left = run.s1 - run.s0; left > 0; left--)
+            {
+                if (!dn_wait(&sh.full[st], phase, abort_flag)) return false;
+                if (NI*NJ > 0)
+                {
+                    const double* As = smem + st*STAGE;
+                    const double* Bs = As + BK*BM;
+                    #pragma unroll
+                    for (int kk = 0; kk < BK; kk += 8)
+                    {
+                        double af[NI > 0 ? NI : 1][4], bf[NJ > 0 ? NJ : 1][2];
+                        #pragma unroll
+                        for (int j = 0; j < NJ; j++)
+                            #pragma unroll
+                            for (int q = 0; q < 2; q++)
+                            {
+                                if (CPLX)
+                                    bf[j][q] = flip(Bs[tile_pos<BN/2, 1>((j*WGN + wn)*4 + (fr >> 1),
+                                                                         (kk + fc + 4*q) ^ (fr & 1))], sign);
+                                else bf[j][q] = Bs[tile_pos<BN, BMODE>((j*WGN + wn)*8 + fr, kk + fc + 4*q)];
+                            }
+                        #pragma unroll
+                        for (int i = 0; i < NI; i++)
+                            #pragma unroll
+                            for (int q = 0; q < 4; q++)
+                                af[i][q] = As[tile_pos<BM, AMODE>((i*WGM + wm)*16 + fr + 8*(q & 1),
+                                                                  kk + fc + 4*(q >> 1))];
+                        if (kk + 8 == BK)
+                        {
+                            // the stage's last fragments are read: it may be refilled
+                            __syncwarp();
+                            if (lane == 0) mb_arrive(&sh.empty[st]);
+                        }
+                        #pragma unroll
+                        for (int i = 0; i < NI; i++)
+                            #pragma unroll
+                            for (int j = 0; j < NJ; j++) dmma16(acc[i][j], af[i], bf[j]);
+                    }
+                }
+                else if (lane == 0) mb_arrive(&sh.empty[st]);
+                if (++st == STAGES) { st = 0; phase ^= 1; }
+            }
+            return true;
+        });
+        if (!ok) break;
+
+        // the run and its tile again (not kept over the loop above)
+        asm volatile("" : "+r"(r));
+        run_at(p, blockIdx.x, r, run);
+        t = tile_at<BM, BN>(p, run.tile);
+        if (run.slot >= 0)
+        {
+            // this run's sums, thread by thread, for gemm_f64_fixup
+            double* w = p.partial + ((i64)blockIdx.x*2 + run.slot)*(BM*BN) + (threadIdx.x - TEAMS*DN_PT);
+            #pragma unroll
+            for (int i = 0; i < MF; i++)
+                #pragma unroll
+                for (int j = 0; j < NF; j++)
+                    if (i < ni && j < nj)
+                    {
+                        #pragma unroll
+                        for (int q = 0; q < 4; q++) w[((i*NF + j)*4 + q)*DN_CT] = acc[i][j][q];
+                    }
+            continue;
+        }
+        double* C = p.C + (CPLX ? 2 : 1)*p.c_l[t.l];
+        const double alpha = p.alpha, beta = p.beta;
+        #pragma unroll
+        for (int j = 0; j < NF; j++)
+        {
+            const int n = (j*WGN + wn)*8 + 2*fc;
+            if (n >= t.nrem) continue;
+            if (CPLX)
+            {
+                double* C0 = C + 2*__ldg(p.c_n + (t.n0 + n)/2);
+                #pragma unroll
+                for (int i = 0; i < MF; i++)
+                    #pragma unroll
+                    for (int hh = 0; hh < 2; hh++)
+                    {
+                        const int m = (i*WGM + wm)*16 + 8*hh + fr;
+                        if (m < t.mrem)
+                            update_z(p, C0 + 2*__ldg(p.c_m + t.m0 + m), acc[i][j][2*hh], acc[i][j][2*hh + 1]);
+                    }
+                continue;
+            }
+            const bool two = n + 1 < t.nrem;
+            double* C0 = C + __ldg(p.c_n + t.n0 + n);
+            double* C1 = C + (two ? __ldg(p.c_n + t.n0 + n + 1) : 0);
+            #pragma unroll
+            for (int i = 0; i < MF; i++)
+                #pragma unroll
+                for (int hh = 0; hh < 2; hh++)
+                {
+                    const int m = (i*WGM + wm)*16 + 8*hh + fr;
+                    if (m >= t.mrem) continue;
+                    const i64 ro = __ldg(p.c_m + t.m0 + m);
+                    const double v0 = alpha*acc[i][j][2*hh], v1 = alpha*acc[i][j][2*hh + 1];
+                    C0[ro] = beta == 0.0 ? v0 : v0 + beta*C0[ro];
+                    if (two) C1[ro] = beta == 0.0 ? v1 : v1 + beta*C1[ro];
+                }
+        }
+    }
+}
+
+// Sums the runs of the cut tiles in CTA order and applies alpha and beta.
+// blockIdx.x: the tile; thread t of a group of DN_CT holds the elements of
+// consumer thread t, a few of the MF*NF*2 pairs per block. GROUPS groups of threads
+// take interleaved CTAs and combine in a fixed order: a tile cut over all SMs
+// then still has enough loads in flight.
+template <int WGM, int WGN, int MF, int NF, int GROUPS, bool CPLX>
+__global__ void __launch_bounds__(DN_CT*GROUPS)
+gemm_f64_fixup(const GemmF64Args p)
+{
+    constexpr int BM = WGM*MF*16, BN = WGN*NF*8;
+    __shared__ double sums[GROUPS][2][DN_CT];
+    const int tc = threadIdx.x % DN_CT, grp = threadIdx.x/DN_CT;
+    const int lane = tc & 31;
+    int wm, wn;
+    warp_at<WGN>(tc >> 5, wm, wn);
+    const TileAt t = tile_at<BM, BN>(p, p.dp_tiles + blockIdx.x);
+
+    // the CTAs [c0, c1) whose runs meet this tile's k steps [ub, ue)
+    const unsigned kt = (unsigned)p.kt, ub = blockIdx.x*kt, ue = ub + kt;
+    const unsigned c0 = cta_of_unit(p, ub), c1 = cta_of_unit(p, ue - 1) + 1;
+    if (c1 - c0 == 1) return;                        // one CTA did the whole tile
+    // the CTA's second slot when its first run is part of an earlier tile
+    // (whole tiles take no slot); only the first CTA can have such a run
+    const unsigned uf = first_unit(p, c0);
+    const double* first = p.partial + (i64)(c0*2 + (uf < ub && uf % kt != 0 ? 1 : 0))*(BM*BN) + tc;
+    // launched while the kernel above runs: its sums are complete from here on
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (int e = blockIdx.y; e < MF*NF*2; e += gridDim.y)
+    {
+        // elements 2e and 2e + 1: neighbouring columns of one row (complex: the
+        // parts of one element)
+        const int hh = e & 1, j = (e >> 1) % NF, i = e/(2*NF);
+        const int m = (i*WGM + wm)*16 + 8*hh + (lane >> 2), n = (j*WGN + wn)*8 + 2*(lane & 3);
+        const bool in = m < t.mrem && n < t.nrem;
+        double s0 = 0.0, s1 = 0.0;
+        if (in)
+        {
+            const i64 at = (i64)2*e*DN_CT;
+            if (grp == 0) { s0 = first[at]; s1 = first[at + DN_CT]; }
+            #pragma unroll 4
+            for (unsigned c = c0 + (grp == 0 ? GROUPS : grp); c < c1; c += GROUPS)
+            {
+                const double* w = p.partial + (i64)c*2*(BM*BN) + at + tc;
+                s0 += w[0];
+                s1 += w[DN_CT];
+            }
+        }
+        if (GROUPS > 1)
+        {
+            __syncthreads();
+            sums[grp][0][tc] = s0;
+            sums[grp][1][tc] = s1;
+            __syncthreads();
+            if (grp > 0) continue;
+            #pragma unroll
+            for (int g = 1; g < GROUPS; g++) { s0 += sums[g][0][tc]; s1 += sums[g][1][tc]; }
+        }
+        if (!in) continue;
+        if (CPLX)
+        {
+            update_z(p, p.C + 2*(p.c_l[t.l] + __ldg(p.c_m + t.m0 + m) + __ldg(p.c_n + (t.n0 + n)/2)), s0, s1);
+            continue;
+        }
+        double* Cm = p.C + p.c_l[t.l] + __ldg(p.c_m + t.m0 + m);
+        double* d0 = Cm + __ldg(p.c_n + t.n0 + n);
+        const double v0 = p.alpha*s0;
+        *d0 = p.beta == 0.0 ? v0 : v0 + p.beta*(*d0);
+        if (n + 1 < t.nrem)
+        {
+            double* d1 = Cm + __ldg(p.c_n + t.n0 + n + 1);
+            const double v1 = p.alpha*s1;
+            *d1 = p.beta == 0.0 ? v1 : v1 + p.beta*(*d1);
+        }
+    }
+}
+
+template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS>
+struct DenseTile
+{
+    static constexpr int BM = WGM*MF*16, BN = WGN*NF*8, GM = WGM, GN = WGN;
+    template <int AM, int BMd, bool CPLX = false>
+    static void go(const GemmF64Args& a, cudaStream_t s)
+    {
+        auto kern = gemm_f64_dense_kernel<WGM, WGN, MF, NF, STAGES, LAG, TEAMS, AM, BMd, CPLX>;
+        constexpr size_t bytes = dn_smem<WGM, WGN, MF, NF, STAGES, TEAMS>();
+        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        TimedLaunch t("gemm_f64_kernel", s);
+        kern<<<(unsigned)a.grid, dn_threads(TEAMS), bytes, s>>>(a);
+        check_launch("gemm_f64_dense_kernel");
+    }
+    // starts as the dense kernel's CTAs leave (its index arithmetic and launch
+    // overlap them), and waits for all of them before it reads their sums
+    template <int GROUPS>
+    static void fixup(const GemmF64Args& a, int y, cudaStream_t s)
+    {
+        cudaLaunchConfig_t c = {};
+        c.gridDim = dim3((unsigned)a.sk_tiles, (unsigned)y);
+        c.blockDim = dim3(DN_CT*GROUPS);
+        c.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        c.attrs = at;
+        c.numAttrs = 1;
+        if (a.cplx) TB_CUDA(cudaLaunchKernelEx(&c, gemm_f64_fixup<WGM, WGN, MF, NF, GROUPS, true>, a));
+        else TB_CUDA(cudaLaunchKernelEx(&c, gemm_f64_fixup<WGM, WGN, MF, NF, GROUPS, false>, a));
+    }
+    static void launch(const GemmF64Args& a, cudaStream_t s)
+    {
+        if (a.cplx) go<1, 1, true>(a, s);
+        else switch (a.amode*2 + a.bmode)
+        {
+            case 0: go<0, 0>(a, s); break;
+            case 1: go<0, 1>(a, s); break;
+            case 2: go<1, 0>(a, s); break;
+            default: go<1, 1>(a, s); break;
+        }
+        if (a.cut)
+        {
+            // few runs per tile: several elements a thread; many: the loads of
+            // one element spread over four groups of threads
+            if (a.sk_ctas >= 8*a.sk_tiles) fixup<4>(a, MF*NF*2, s);
+            else fixup<1>(a, MF*NF, s);
+            check_launch("gemm_f64_fixup");
+        }
+    }
+};
+
+typedef DenseTile<2, 4, 4, 4, 6, 1, 1> Tile128;      // 128 x 128, 192 KB of stages
+typedef DenseTile<2, 4, 2, 2, 12, 1, 2> Tile64;      // 64 x 64, the same ring in bytes
+typedef DenseTile<8, 1, 1, 4, 8, 2, 2> TileTall;     // 128 x 32, 180 KB
+
+// Cycles of one k step of a tile with m rows and n columns, as measured: 128 for
+// each 16 x 8 fragment pair of the busiest SM sub-core (the DMMA rate) and about
+// 350 more, at least the gather of its operands (12 bytes per cycle and SM) and
+// the time a producer warp takes to issue a stage (kFloor).
+template <typename T>
+double step_cycles(int m, int n)
+{
+    constexpr double kGather = 12.0, kFloor = T::BM == 128 && T::BN == 128 ? 1450.0 : 900.0;
+    double load[4] = {0, 0, 0, 0};
+    for (int cw = 0; cw < DN_CONSUMERS; cw++)
+    {
+        const int wm = cw/T::GN, wn = (cw + (T::GN/2)*wm) % T::GN;
+        const int ni = std::max(0, ((m + 15)/16 - wm + T::GM - 1)/T::GM);
+        const int nj = std::max(0, ((n + 7)/8 - wn + T::GN - 1)/T::GN);
+        load[cw % 4] += 128.0*ni*nj;
+    }
+    return std::max({350.0 + std::max({load[0], load[1], load[2], load[3]}), (double)(m + n)*BK*8/kGather, kFloor});
+}
+
+// the work split of one tile shape and its modelled cycles
+template <typename T>
+double split_work(GemmF64Args& a, int sms, size_t ws_limit)
+{
+    // cutting adds a second launch, the partial sums' way through L2 (about
+    // 1.2 KB per cycle) and another pipeline start; kRun: a tile's C update
+    constexpr double kCutCycles = 10000, kRun = 2000, kUnit = 32;
+    constexpr size_t kSlot = (size_t)T::BM*T::BN*sizeof(double);
+    const i64 N = a.cplx ? 2*a.N : a.N;
+    const i64 fm = a.M/T::BM, fn = N/T::BN, L = a.L;
+    const int rm = (int)(a.M - fm*T::BM), rn = (int)(N - fn*T::BN);
+    const i64 count[4] = {fm*fn*L, rm ? fn*L : 0, rn ? fm*L : 0, rm && rn ? L : 0};
+    const double cyc[4] = {step_cycles<T>(T::BM, T::BN), step_cycles<T>(std::max(rm, 1), T::BN),
+                           step_cycles<T>(T::BM, std::max(rn, 1)), step_cycles<T>(std::max(rm, 1), std::max(rn, 1))};
+    const double kt = (double)a.kt;
+    i64 tiles = 0;
+    double total = 0, longest = 0;
+    for (int c = 0; c < 4; c++)
+    {
+        tiles += count[c];
+        total += (double)count[c]*(kt*cyc[c] + kRun);
+        if (count[c]) longest = std::max(longest, kt*cyc[c] + kRun);
+    }
+    a.dp_tiles = tiles; a.sk_tiles = 0; a.sk_ctas = 0; a.cut = 0;
+    a.sk_per = a.sk_extra = 0;
+    a.grid = (int)std::min<i64>(tiles, sms);
+    a.ws_bytes = 0;
+    // tiles dealt in turn: about one longest tile above the mean
+    const double whole = tiles <= sms ? longest : std::max((double)((tiles + sms - 1)/sms)*total/(double)tiles,
+                                                           total/sms + 0.5*longest);
+    // cut: all but the last whole wave of whole tiles stays uncut
+    const i64 dp = std::max<i64>(0, (count[0]/sms - 1)*sms);
+    const double cut_total = total - (double)dp*(kt*cyc[0] + kRun);
+    double units = 0;
+    unsigned first = 0, wmax = 1;
+    for (int c = 0; c < 4; c++)
+    {
+        const unsigned n = (unsigned)(count[c] - (c == 0 ? dp : 0));
+        a.cls_first[c] = first;
+        a.cls_w[c] = (unsigned)std::max(1.0, std::round(cyc[c]/kUnit));
+        first += n;
+        units += (double)n*kt*a.cls_w[c];
+        if (n) wmax = std::max(wmax, a.cls_w[c]);
+    }
+    a.cls_first[4] = first;
+    // no run below 1500 cycles (its pipeline start) or two steps of any class
+    i64 ctas = std::min<i64>({(i64)sms, (i64)(units*kUnit/1500.0), (i64)(units/(2.0*wmax)), (i64)(ws_limit/(2*kSlot))});
+    if (units >= (double)(1ll << 31) || ctas < 2 || (dp > 0 && ctas < sms)) return whole;
+    const double cut = (double)(dp/sms)*(kt*cyc[0] + kRun) + cut_total/(double)ctas + kRun + kCutCycles +
+                       (double)ctas*(double)kSlot/1200.0;
+    if (cut >= whole) return whole;
+    a.dp_tiles = dp;
+    a.sk_tiles = tiles - dp;
+    a.sk_ctas = (int)ctas;
+    a.sk_per = (unsigned)units/(unsigned)ctas;
+    a.sk_extra = (unsigned)units - a.sk_per*(unsigned)ctas;
+    a.cut = 1;
+    a.grid = (int)ctas;
+    a.ws_bytes = (size_t)ctas*2*kSlot;
+    return cut;
+}
+
+} // namespace
+
+// The tile shape and work split of least modelled time: 128 x 128 for most; 64
+// x 64 (twice the operand bytes per FMA, a quarter of the partial sums) where a
+// GEMM has few tiles or ragged ones; 128 x 32 where one extent is small, the
+// operands swapped if that is the rows.
+void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit)
+{
+    const i64 per = a.cplx ? 2 : 1;                 // real columns and k per element
+    if (a.N > a.M && per*a.M <= TileTall::BN)
+    {
+        // C^T = B^T A^T: the small extent becomes the columns
+        std::swap(a.A, a.B);
+        std::swap(a.a_m, a.b_n); std::swap(a.a_k, a.b_k); std::swap(a.a_l, a.b_l);
+        std::swap(a.c_m, a.c_n); std::swap(a.M, a.N);
+        std::swap(a.amode, a.bmode); std::swap(a.pair_a, a.pair_b);
+        std::swap(a.conj_a, a.conj_b);
+    }
+    a.kt = (per*a.K + BK - 1)/BK;
+    GemmF64Args b = a, c = a;
+    a.tile = 0; b.tile = 1; c.tile = 2;
+    const double t128 = split_work<Tile128>(a, sms, ws_limit), t64 = split_work<Tile64>(b, sms, ws_limit);
+    const double tall = per*a.N <= TileTall::BN ? split_work<TileTall>(c, sms, ws_limit) : 1e300;
+    if (t64 < t128 && t64 <= tall) a = b;
+    else if (tall < t128) a = c;
+}
+
+void gemm_f64_dense_launch(const GemmF64Args& a, cudaStream_t stream)
+{
+    if (a.M == 0 || a.N == 0 || a.L == 0 || a.K == 0) return;
+    TB_CHECK(a.L <= 65535, TB_ERR_SIZE, "batch extent too large");
+    TB_CHECK(((a.M + 63)/64)*((a.N + 63)/64) < (1ll << 31), TB_ERR_SIZE, "tile grid too large");
+    TB_CHECK(!a.cut || a.partial, TB_ERR_ARG, "cut tiles need a workspace");
+    TB_CHECK(a.dp_tiles + a.sk_tiles < (1ll << 31), TB_ERR_SIZE, "tile grid too large");
+    if (a.tile == 0) Tile128::launch(a, stream);
+    else if (a.tile == 1) Tile64::launch(a, stream);
+    else TileTall::launch(a, stream);
+}
+
+int gemm_f64_dense_error_flag()
+{
+    int v = 0;
+    cudaMemcpyFromSymbol(&v, g_dn_error, sizeof(int));
+    if (v)
+    {
+        const int zero = 0;
+        cudaMemcpyToSymbol(g_dn_error, &zero, sizeof(int));
+    }
+    return v;
+}
+
+} // namespace tb

@@ -5,6 +5,8 @@
 
 #include "common.hpp"
 
+#include <cstdint>
+
 namespace tb
 {
 namespace f64dev
@@ -56,6 +58,35 @@ __device__ __forceinline__ void dmma16(double* c, const double* a, const double*
                  "{%0,%1,%2,%3};\n"
                  : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
                  : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
+}
+
+// ---- mbarriers ------------------------------------------------------------------
+
+__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+__device__ __forceinline__ void mb_init(uint64_t* b, uint32_t count)
+{
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(su32(b)), "r"(count) : "memory");
+}
+
+__device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(su32(b)), "r"(parity) : "memory");
+    return ok != 0;
+}
+
+__device__ __forceinline__ void mb_arrive(uint64_t* b)
+{
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(su32(b)) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long gtimer()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
 }
 
 // shared-memory geometry of one operand tile (ROWS = BM or BN)

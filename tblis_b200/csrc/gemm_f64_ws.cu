@@ -84,26 +84,6 @@ __device__ int g_f64_error = 0;
 __device__ unsigned long long g_f64_wait_ns = WS_WAIT_NS;
 __device__ int g_f64_skip_step = -1;       // test support: a stage whose copies are never issued
 
-__device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mb_init(uint64_t* b, uint32_t count)
-{
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(su32(b)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ bool mb_try(uint64_t* b, uint32_t parity)
-{
-    uint32_t ok;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-                 " selp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(su32(b)), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-__device__ __forceinline__ void mb_arrive(uint64_t* b)
-{
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(su32(b)) : "memory");
-}
-
 // arrives and adds the bytes that the copies of this phase will deliver
 __device__ __forceinline__ void mb_arrive_expect(uint64_t* b, uint32_t bytes)
 {
@@ -116,13 +96,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 {
     asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                  :: "r"(su32(dst)), "l"((uint64_t)src), "r"(bytes), "r"(su32(bar)) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long gtimer()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
 }
 
 // bounded wait of one thread on a phase of an mbarrier; false when the CTA

@@ -223,6 +223,26 @@ static void unstage(StagedOp& o, cudaStream_t s)
                             cudaMemcpyDeviceToHost, s));
 }
 
+// the dense kernel with its workspace; without room for one, tiles stay whole
+static void dense_gemm(GemmF64Args& a, cudaStream_t st)
+{
+    const GemmF64Args unplanned = a;
+    gemm_f64_dense_plan(a, device_sm_count(), SIZE_MAX);
+    dbuf ws;
+    if (a.ws_bytes)
+    {
+        try { ws = dbuf(a.ws_bytes, st); }
+        catch (const error&)
+        {
+            cudaGetLastError();
+            a = unplanned;
+            gemm_f64_dense_plan(a, device_sm_count(), 0);
+        }
+    }
+    a.partial = ws.as<double>();
+    gemm_f64_dense_launch(a, st);
+}
+
 // one contraction on device data (a GEMM view of device-resident operands)
 static void contract_device(const GemmView& v, const double* A, const double* B, double* C, double alpha,
                             double beta, int method, double tol, int slices, cudaStream_t st,
@@ -250,17 +270,14 @@ static void contract_device(const GemmView& v, const double* A, const double* B,
     a.a_m = tab->a_m; a.a_k = tab->a_k; a.b_k = tab->b_k; a.b_n = tab->b_n;
     // pairs of 16-byte copies where the layout gives them (the kernel checks
     // every pair; this only picks the gather code)
-    a.pair_a = tab->a_pairs[v.amode] && ((uintptr_t)A & 15) == 0;
-    a.pair_b = tab->b_pairs[v.bmode] && ((uintptr_t)B & 15) == 0;
+    a.pair_a = tab->a_pairs[tab->amode] && ((uintptr_t)A & 15) == 0;
+    a.pair_b = tab->b_pairs[tab->bmode] && ((uintptr_t)B & 15) == 0;
     a.c_m = tab->c_m; a.c_n = tab->c_n; a.a_l = tab->a_l; a.b_l = tab->b_l; a.c_l = tab->c_l;
     a.a_kbs = tab->a_kbs; a.b_kbs = tab->b_kbs;
     a.M = v.m; a.N = v.n; a.K = v.k; a.L = v.l;
     a.alpha = alpha; a.beta = beta;
-    a.amode = v.amode; a.bmode = v.bmode;
-    a.splits = gemm_f64_choose_splits(v.m, v.n, v.k, v.l, device_sm_count());
-    dbuf ws(gemm_f64_workspace_bytes(v.m, v.n, v.l, a.splits), st);
-    a.partial = ws.as<double>();
-    gemm_f64_launch(a, st);
+    a.amode = tab->amode; a.bmode = tab->bmode;
+    dense_gemm(a, st);
     used_slices = 0;
     est_error = 1.1e-16*std::sqrt((double)v.k);
 }
@@ -324,6 +341,51 @@ static void mult_complex(const tblis_config* cfg,
     stage(sA, &pa.whole, true, st);
     stage(sB, &pb.whole, true, st);
     pa.place(sA.dptr); pb.place(sB.dptr); pc.place(sC.dptr);
+
+    // FP64 with a product to form: one real contraction of twice the columns
+    // and twice the k (gemm_f64_dense.cu). It reads and writes whole elements, so
+    // they must be 16-byte aligned; the four real contractions below serve the
+    // rest and the split-precision methods.
+    const int method = opts && opts->method ? opts->method : (cfg ? cfg->method : 1);
+    const bool aligned = (((uintptr_t)sA.dptr | (uintptr_t)sB.dptr | (uintptr_t)sC.dptr) & 15) == 0;
+    if (method == 1 && aligned && (alr != 0.0 || ali != 0.0))
+    {
+        const GemmView v = gemm_view(mult_groups(A, idx_A, B, idx_B, C, idx_C));
+        if (v.m*v.n*v.l*v.k != 0)
+        {
+            auto tab = gemm_tables(v, gemm_f64_tile_m(), gemm_f64_tile_n(), gemm_f64_tile_k(), st);
+            GemmF64Args a = {};
+            a.A = static_cast<const double*>(sA.dptr);
+            a.B = static_cast<const double*>(sB.dptr);
+            a.C = static_cast<double*>(sC.dptr);
+            a.a_m = tab->a_m; a.a_k = tab->a_k; a.b_k = tab->b_k; a.b_n = tab->b_n;
+            a.c_m = tab->c_m; a.c_n = tab->c_n; a.a_l = tab->a_l; a.b_l = tab->b_l; a.c_l = tab->c_l;
+            a.M = v.m; a.N = v.n; a.K = v.k; a.L = v.l;
+            a.alpha = alr; a.alpha_im = ali;
+            a.beta = ber; a.beta_im = bei;
+            a.cplx = 1;
+            a.conj_a = A->conj != 0; a.conj_b = B->conj != 0; a.conj_c = C->conj != 0;
+            a.amode = tab->amode; a.bmode = tab->bmode;
+            dense_gemm(a, st);
+            unstage(sC, st);
+            if (sA.staged || sB.staged || sC.staged) TB_CUDA(cudaStreamSynchronize(st));
+            C->scalar.type = TYPE_DCOMPLEX;
+            C->scalar.data.z[0] = 1.0;
+            C->scalar.data.z[1] = 0.0;
+            C->conj = 0;
+            if (report)
+            {
+                // a complex alpha counts twice, as its four real products do below
+                const double per = alr != 0.0 && ali != 0.0 ? 16.0 : 8.0;
+                report->method = 1;
+                report->slices = 0;
+                report->est_error = 0.5*per*1.1e-16*std::sqrt((double)v.k);
+                report->flops = per*(double)v.m*(double)v.n*(double)v.k*(double)v.l;
+                report->kernels = (int)(g_kernel_count.load() - kernels_before);
+            }
+            return;
+        }
+    }
 
     auto real_add = [&](double alpha, tblis_tensor X, double beta, tblis_tensor Y)
     {
