@@ -449,6 +449,12 @@ int tblis_b200_dpd_mult_shard(const tblis_b200_dpd_tensor* A, const label_type* 
 int tblis_b200_dpd_block(const tblis_b200_dpd_tensor* A, const unsigned* irreps, len_type* len,
                          stride_type* stride, stride_type* offset);
 
+/* Offset and strides of every stored block at once: irrep tuples numbered with
+ * dimension 0 fastest, nirrep^ndim offsets (-1: not stored or empty) and
+ * nirrep^ndim * ndim strides (zeros there), as tblis_b200_dpd_block_table takes
+ * them. */
+int tblis_b200_dpd_blocks(const tblis_b200_dpd_tensor* A, stride_type* offset, stride_type* stride);
+
 /* Number of stored elements (all allowed blocks), or -1 on error. */
 len_type tblis_b200_dpd_size(const tblis_b200_dpd_tensor* A);
 

@@ -536,25 +536,21 @@ lib.tblis_b200_dpd_full_to_block.argtypes = [_P(tblis_tensor), _DT]
 
 def _dpd_table(T, scalar=1.0):
     """The block table of a DpdTensor (every stored block's offset and
-    strides, irrep tuples numbered with dimension 0 fastest)."""
+    strides, irrep tuples numbered with dimension 0 fastest). It follows from the
+    layout alone, so the tensor keeps it for the layout it was made for; data
+    and scalar are read on every call."""
     nd, n = len(T.lens), T.nirrep
-    nt = n ** nd
-    off = [-1] * nt
-    st = [0] * (nt * nd)
-    for t in range(nt):
-        irr = [(t // n ** d) % n for d in range(nd)]
-        x = 0
-        ext = 1
-        for d in range(nd):
-            x ^= irr[d]
-            ext *= T.lens[d][irr[d]]
-        if x != T.irrep or ext == 0:
-            continue
-        o, _, strides = T.block(irr)
-        off[t] = o
-        st[t * nd:(t + 1) * nd] = strides
-    keep = [(ctypes.c_ssize_t * (nd * n))(*[x for r in T.lens for x in r]), (ctypes.c_ssize_t * nt)(*off),
-            (ctypes.c_ssize_t * max(1, len(st)))(*st)]
+    layout = (n, T.irrep, T.layout, tuple(map(tuple, T.lens)))
+    kept = getattr(T, "_table", None)
+    if kept is None or kept[0] != layout:
+        nt = n ** nd
+        keep = [(ctypes.c_ssize_t * (nd * n))(*[x for r in T.lens for x in r]), (ctypes.c_ssize_t * nt)(),
+                (ctypes.c_ssize_t * max(1, nt * nd))()]
+        t = T.struct()
+        lib.tblis_b200_dpd_blocks(ctypes.byref(t), keep[1], keep[2])
+        _check()
+        T._table = kept = (layout, keep)
+    keep = kept[1]
     b = tblis_b200_dpd_block_table()
     b.type = T.code
     b.conj = 0

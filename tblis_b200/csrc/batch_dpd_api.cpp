@@ -390,6 +390,28 @@ int tblis_b200_dpd_block(const tblis_b200_dpd_tensor* A, const unsigned* irreps,
     });
 }
 
+int tblis_b200_dpd_blocks(const tblis_b200_dpd_tensor* A, stride_type* offset, stride_type* stride)
+{
+    return guarded([&]
+    {
+        TB_CHECK(offset && stride, TB_ERR_ARG, "null block table");
+        DpdLayout lay;
+        to_layout(A, lay);
+        size_t nt = 1;
+        for (unsigned d = 0; d < lay.ndim; d++) nt *= lay.nirrep;
+        std::fill(offset, offset + nt, (stride_type)-1);
+        std::fill(stride, stride + nt*lay.ndim, (stride_type)0);
+        lay.for_each_block([&](const std::vector<unsigned>& irr, const std::vector<i64>&, const std::vector<i64>& bs,
+                               i64 off)
+        {
+            size_t t = 0;
+            for (unsigned d = lay.ndim; d-- > 0;) t = t*lay.nirrep + irr[d];
+            offset[t] = off;
+            for (unsigned d = 0; d < lay.ndim; d++) stride[t*lay.ndim + d] = bs[d];
+        });
+    });
+}
+
 len_type tblis_b200_dpd_size(const tblis_b200_dpd_tensor* A)
 {
     len_type n = -1;

@@ -15,6 +15,8 @@
 //  * dot: sum over blocks of the blockwise dots (0 when the irreps differ);
 //  * reduce: blockwise reductions combined in block order, idx = offset of
 //    the extreme element from the tensor's data (first block wins ties);
+//    sums need no order, so permuting adds, dots and sum-type reductions take
+//    all blocks in one launch (level1_tiles.cuh);
 //  * scale / set / shift: every stored block.
 #include "common.hpp"
 #include "dpd.hpp"
@@ -215,6 +217,78 @@ void scale_all(int type, const DpdLayout& X, void* base, zd beta, bool conj, con
     });
 }
 
+// the index space of a pair of blocks: dimensions of extent 1 dropped, those
+// that continue one another in both tensors merged
+PieceSpec piece_of(const std::vector<i64>& len, const std::vector<i64>& sa, const std::vector<i64>& sb, i64 offa,
+                   i64 offb)
+{
+    TB_CHECK(len.size() <= (size_t)L1_MAX_DIM, TB_ERR_SIZE, "DPD: too many dimensions");
+    PieceSpec p;
+    p.offa = offa; p.offb = offb;
+    Strided2& s = p.ab;
+    for (size_t d = 0; d < len.size(); d++)
+    {
+        if (len[d] == 1) continue;
+        int at = s.ndim++;
+        for (; at > 0 && s.sa[at - 1] > sa[d]; at--)
+        {
+            s.len[at] = s.len[at - 1]; s.sa[at] = s.sa[at - 1]; s.sb[at] = s.sb[at - 1];
+        }
+        s.len[at] = len[d]; s.sa[at] = sa[d]; s.sb[at] = sb[d];
+    }
+    int n = 0;
+    for (int d = 0; d < s.ndim; d++)
+    {
+        if (n > 0 && s.sa[d] == s.sa[n - 1]*s.len[n - 1] && s.sb[d] == s.sb[n - 1]*s.len[n - 1]) s.len[n - 1] *= s.len[d];
+        else { s.len[n] = s.len[d]; s.sa[n] = s.sa[d]; s.sb[n] = s.sb[d]; n++; }
+    }
+    s.ndim = n;
+    return p;
+}
+
+// block irr of X: its extents and strides into len and stride (in X's dimension
+// order), offset returned; false for an empty block
+bool block_at(const DpdLayout& X, const std::vector<unsigned>& irr, std::vector<i64>& len, std::vector<i64>& stride,
+              i64& offset)
+{
+    i64 ext = 1;
+    for (unsigned d = 0; d < X.ndim; d++) ext *= X.len[d][irr[d]];
+    if (ext == 0) return false;
+    len.resize(X.ndim);
+    stride.resize(X.ndim);
+    X.block(irr.data(), len.data(), stride.data(), offset);
+    return true;
+}
+
+// calls f with an element of the type
+template <typename F>
+void with_element(int type, F&& f)
+{
+    switch (type)
+    {
+        case TYPE_FLOAT: f(float()); return;
+        case TYPE_DOUBLE: f(double()); return;
+        case TYPE_SCOMPLEX: f(cplx<float>(0.0f)); return;
+        case TYPE_DCOMPLEX: f(cplx<double>(0.0)); return;
+    }
+    throw error(TB_ERR_TYPE, "unknown element type");
+}
+void element(zd z, float& x) { x = (float)z.real(); }
+void element(zd z, double& x) { x = z.real(); }
+void element(zd z, cplx<float>& x) { x = cplx<float>((float)z.real(), (float)z.imag()); }
+void element(zd z, cplx<double>& x) { x = cplx<double>(z.real(), z.imag()); }
+zd to_zd(double x) { return zd(x, 0.0); }
+zd to_zd(cplx<double> x) { return zd(x.re, x.im); }
+template <typename T> struct SumOf { typedef double type; };
+template <typename R> struct SumOf<cplx<R>> { typedef cplx<double> type; };
+
+bool repeats(const std::string& labels)
+{
+    for (size_t i = 1; i < labels.size(); i++)
+        if (labels.find(labels[i]) < i) return true;
+    return false;
+}
+
 std::vector<unsigned> positions(const std::string& labels, const std::string& of)
 {
     std::vector<unsigned> p;
@@ -249,6 +323,32 @@ void dpd_add_dev_t(int type, zd alpha, const DpdLayout& A, const void* a, const 
     }
     const auto pA_AB = positions(AB, iA), pB_AB = positions(AB, iB), pA_only = positions(Aonly, iA);
     std::vector<unsigned> irrA(A.ndim, 0);
+    if (Aonly.empty() && Bonly.empty())
+    {
+        // a permutation: every B block has its one A block; all in one launch
+        // (a launch per block cost 2 us each, 512 of them for 8 irreps)
+        std::vector<PieceSpec> pieces;
+        std::vector<i64> la, sa, sb(A.ndim);
+        B.for_each_block([&](const std::vector<unsigned>& irrB, const std::vector<i64>&, const std::vector<i64>& bs,
+                             i64 offb)
+        {
+            i64 offa = 0;
+            for (size_t i = 0; i < AB.size(); i++) irrA[pA_AB[i]] = irrB[pB_AB[i]];
+            if (!block_at(A, irrA, la, sa, offa)) return;
+            for (size_t i = 0; i < AB.size(); i++) sb[pA_AB[i]] = bs[pB_AB[i]];
+            pieces.push_back(piece_of(la, sa, sb, offa, offb));
+        });
+        with_element(type, [&](auto t)
+        {
+            typedef decltype(t) T;
+            T al, be;
+            element(alpha, al);
+            element(beta, be);
+            l1_add_pieces<T>(static_cast<const T*>(a), static_cast<T*>(b), pieces, al, be, current_stream(), conj_a,
+                             conj_b);
+        });
+        return;
+    }
     B.for_each_block([&](const std::vector<unsigned>& irrB, const std::vector<i64>&, const std::vector<i64>&, i64)
     {
         BlockView bb(type, B, b, irrB, beta, conj_b);
@@ -298,15 +398,45 @@ zd dpd_dot_dev_t(int type, const DpdLayout& A, const void* a, const std::string&
     const auto pB = positions(iA, iB);
     std::vector<unsigned> irrB(B.ndim), all(A.ndim), irrA(A.ndim, 0);
     for (unsigned d = 0; d < A.ndim; d++) all[d] = d;
+    if (repeats(iA) || repeats(iB))
+    {
+        // diagonals: block by block through the dense entry point
+        for_each_combo(all, A.irrep, A.nirrep, irrA, [&]
+        {
+            for (unsigned d = 0; d < A.ndim; d++) irrB[pB[d]] = irrA[d];
+            BlockView ab(type, A, a, irrA, 1.0, conj_a), bb(type, B, b, irrB, 1.0, conj_b);
+            if (ab.empty || bb.empty) return;
+            tblis_scalar r;
+            r.type = (type_t)type;
+            checked([&] { tblis_tensor_dot(nullptr, nullptr, &ab.t, iA.c_str(), &bb.t, iB.c_str(), &r); });
+            sum += scalar_get(r);
+        });
+        return sum;
+    }
+    // every stored block pair in one launch, the sum in double precision
+    std::vector<PieceSpec> pieces;
+    std::vector<i64> la, sa, lb, sb, sbA(A.ndim);
     for_each_combo(all, A.irrep, A.nirrep, irrA, [&]
     {
         for (unsigned d = 0; d < A.ndim; d++) irrB[pB[d]] = irrA[d];
-        BlockView ab(type, A, a, irrA, 1.0, conj_a), bb(type, B, b, irrB, 1.0, conj_b);
-        if (ab.empty || bb.empty) return;
-        tblis_scalar r;
-        r.type = (type_t)type;
-        checked([&] { tblis_tensor_dot(nullptr, nullptr, &ab.t, iA.c_str(), &bb.t, iB.c_str(), &r); });
-        sum += scalar_get(r);
+        i64 offa = 0, offb = 0;
+        if (!block_at(A, irrA, la, sa, offa) || !block_at(B, irrB, lb, sb, offb)) return;
+        for (unsigned d = 0; d < A.ndim; d++) sbA[d] = sb[pB[d]];
+        pieces.push_back(piece_of(la, sa, sbA, offa, offb));
+    });
+    cudaStream_t st = current_stream();
+    with_element(type, [&](auto t)
+    {
+        typedef decltype(t) T;
+        typedef typename SumOf<T>::type Acc;
+        const bool cx = is_complex_type(type);
+        dbuf out(sizeof(Acc), st);
+        l1_dot_pieces<T, Acc>(static_cast<const T*>(a), static_cast<const T*>(b), pieces, out.as<Acc>(), st,
+                              conj_a && cx, conj_b && cx);
+        Acc v;
+        TB_CUDA(cudaMemcpyAsync(&v, out.ptr, sizeof(Acc), cudaMemcpyDeviceToHost, st));
+        TB_CUDA(cudaStreamSynchronize(st));
+        sum = to_zd(v);
     });
     return sum;
 }
@@ -325,6 +455,32 @@ void dpd_reduce_dev_t(int type, int op, const DpdLayout& A, const void* a, const
     // go to the first block reaching the extreme value
     std::vector<unsigned> all(A.ndim), irr(A.ndim, 0);
     for (unsigned d = 0; d < A.ndim; d++) all[d] = d;
+    if ((op == REDUCE_SUM || op == REDUCE_SUM_ABS || op == REDUCE_NORM_2) && !repeats(iA))
+    {
+        // sums: every stored block in one launch, in double precision
+        std::vector<PieceSpec> pieces;
+        std::vector<i64> la, sa;
+        for_each_combo(all, A.irrep, A.nirrep, irr, [&]
+        {
+            i64 off = 0;
+            if (block_at(A, irr, la, sa, off)) pieces.push_back(piece_of(la, sa, sa, off, off));
+        });
+        cudaStream_t st = current_stream();
+        with_element(type, [&](auto t)
+        {
+            typedef decltype(t) T;
+            typedef typename SumOf<T>::type Acc;
+            dbuf out(sizeof(Acc), st);
+            l1_sum_pieces<T, Acc>(op, static_cast<const T*>(a), pieces, out.as<Acc>(), st);
+            Acc v;
+            TB_CUDA(cudaMemcpyAsync(&v, out.ptr, sizeof(Acc), cudaMemcpyDeviceToHost, st));
+            TB_CUDA(cudaStreamSynchronize(st));
+            acc = to_zd(v);
+        });
+        result = op == REDUCE_NORM_2 ? zd(std::sqrt(acc.real())) : acc;
+        idx = -1;
+        return;
+    }
     for_each_combo(all, A.irrep, A.nirrep, irr, [&]
     {
         BlockView ab(type, A, a, irr, 1.0);

@@ -235,28 +235,25 @@ k_add_rows(const T* __restrict__ A, T* __restrict__ B, const Strided2 s, T alpha
     }
 }
 
-// transpose: dim p is A's unit dim, dim q is B's unit dim, the rest are outer.
-// Square tile through shared memory (64 wide, 32 for 16-byte elements so the
-// tile stays below 48 KB); reads coalesced along p, writes along q. VW = 2
-// moves pairs of elements (16 bytes for 8-byte types) on both sides when the
-// host has checked that both unit strides are 1, both extents and every other
-// stride are even and both bases are aligned to a pair, so every pair is
-// contiguous and aligned.
-template <typename T>
-constexpr int tile_of() { return sizeof(T) >= 16 ? 32 : 64; }
+// transpose in pairs: dim p is A's unit dim, dim q is B's unit dim, the rest
+// are outer. 64 x 64 tile through shared memory, read along p and written along
+// q in pairs of elements (16 bytes for 8-byte types): the host has checked that
+// both unit strides are 1, both extents and every other stride are even and both
+// bases are aligned to a pair, so every pair is contiguous and aligned, and that
+// the extents fill the tiles (level1_tiles.cuh takes the rest).
+constexpr int TP_TILE = 64;
 
 template <int BYTES> struct RawVec;
 template <> struct RawVec<8> { typedef uint2 type; };
 template <> struct RawVec<16> { typedef uint4 type; };
 
-template <typename T, bool BETA0, int VW>
+template <typename T, bool BETA0>
 __global__ void __launch_bounds__(L1_THREADS, 3)
 k_transpose(const T* __restrict__ A, T* __restrict__ B, const Strided2 s, int p, int q,
             i64 tiles_p, i64 tiles_q, i64 outer, T alpha, T beta, bool conj_a, bool conj_b)
 {
-    constexpr int TT = tile_of<T>();
-    typedef typename RawVec<(VW == 1 || sizeof(T)*VW < 8) ? 8 : sizeof(T)*VW>::type Raw;
-    static_assert(VW == 1 || sizeof(Raw) == sizeof(T)*VW, "pair width");
+    constexpr int TT = TP_TILE, VW = 2;
+    typedef typename RawVec<sizeof(T)*VW>::type Raw;
     __shared__ T tile[TT][TT + 1];
     const i64 np = s.len[p], nq = s.len[q];
     // tile indices in 32 bits (the host checks the tile count), so each tile
@@ -285,8 +282,7 @@ k_transpose(const T* __restrict__ A, T* __restrict__ B, const Strided2 s, int p,
         // of a thread's loads are issued into registers before the first
         // shared-memory store, so they are in flight together.
         constexpr int NJ = TT/8, NH = TT/(32*VW);
-        typedef typename std::conditional<VW == 1, T, Raw>::type Item;
-        Item in[NJ][NH];
+        Raw in[NJ][NH];
         #pragma unroll
         for (int j = 0; j < NJ; j++)
         {
@@ -295,7 +291,7 @@ k_transpose(const T* __restrict__ A, T* __restrict__ B, const Strided2 s, int p,
             {
                 const i64 pi = p0 + (tx + 32*h)*VW, qi = q0 + ty + 8*j;
                 if (pi < np && qi < nq)
-                    in[j][h] = *reinterpret_cast<const Item*>(A + oa + pi*s.sa[p] + qi*s.sa[q]);
+                    in[j][h] = *reinterpret_cast<const Raw*>(A + oa + pi*s.sa[p] + qi*s.sa[q]);
             }
         }
         #pragma unroll
@@ -328,12 +324,6 @@ k_transpose(const T* __restrict__ A, T* __restrict__ B, const Strided2 s, int p,
                 if (pi < np && qi < nq)
                 {
                     T* dst = B + ob + pi*s.sb[p] + qi*s.sb[q];
-                    if (VW == 1)
-                    {
-                        const T v = alpha*cj(tile[ql][pl], conj_a);
-                        *dst = BETA0 ? v : v + beta*cj(*dst, conj_b);
-                    }
-                    else
                     {
                         Raw r;
                         if (!BETA0) r = *reinterpret_cast<const Raw*>(dst);
@@ -530,16 +520,19 @@ template <typename T>
 __global__ void k_reduce_final(int op, const T* pv, const i64* plin, const i64* poff, int n,
                                T* out_v, i64* out_idx)
 {
-    if (threadIdx.x != 0) return;
     const bool is_sum = op == REDUCE_SUM || op == REDUCE_SUM_ABS || op == REDUCE_NORM_2;
     if (is_sum)
     {
+        // the whole warp, in a fixed order (one thread adding 592 partials took 26 us)
         T t = T(0);
-        for (int i = 0; i < n; i++) t += pv[i];
+        for (int i = threadIdx.x; i < n; i += 32) t += pv[i];
+        for (int o = 16; o > 0; o >>= 1) t += shfl_down(t, o);
+        if (threadIdx.x != 0) return;
         if (op == REDUCE_NORM_2) t = sqrt_elem(t);
         *out_v = t; *out_idx = -1;
         return;
     }
+    if (threadIdx.x != 0) return;
     Cand<T> b = {pv[0], plin[0], poff[0]};
     for (int i = 1; i < n; i++)
     {
@@ -560,6 +553,8 @@ __global__ void k_reduce_final(int op, const T* pv, const i64* plin, const i64* 
     }
     *out_v = b.v; *out_idx = b.off;
 }
+
+#include "level1_tiles.cuh"
 
 } // namespace
 
@@ -607,6 +602,147 @@ void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st)
 template void l1_convert<float, double>(const float*, double*, const Strided&, cudaStream_t);
 template void l1_convert<double, float>(const double*, float*, const Strided&, cudaStream_t);
 
+// rows of same-order adds that a warp walks on its own
+constexpr i64 kLongRow = 128;
+
+// the piece of one index space: p A's fastest dimension, q B's (absent where
+// it is p or trivial); false for an empty one
+static bool make_piece(const PieceSpec& sp, Piece& c)
+{
+    const Strided2& ab = sp.ab;
+    c = Piece{};
+    c.offa = sp.offa; c.offb = sp.offb;
+    c.np = c.nq = 1;
+    int pa = -1, pb = -1;
+    i64 outer = 1;
+    for (int d = 0; d < ab.ndim; d++)
+    {
+        if (ab.len[d] == 0) return false;
+        if (ab.len[d] == 1) continue;
+        if (pa < 0 || std::llabs(ab.sa[d]) < std::llabs(ab.sa[pa])) pa = d;
+        if (pb < 0 || std::llabs(ab.sb[d]) < std::llabs(ab.sb[pb])) pb = d;
+    }
+    if (pa >= 0) { c.np = ab.len[pa]; c.sap = ab.sa[pa]; c.sbp = ab.sb[pa]; }
+    if (pb != pa) { c.nq = ab.len[pb]; c.saq = ab.sa[pb]; c.sbq = ab.sb[pb]; c.turn = 1; }
+    for (int d = 0; d < ab.ndim; d++)
+    {
+        if (d == pa || d == pb || ab.len[d] == 1) continue;
+        c.len[c.nd] = ab.len[d]; c.sa[c.nd] = ab.sa[d]; c.sb[c.nd] = ab.sb[d];
+        c.nd++;
+        outer *= ab.len[d];
+    }
+    TB_CHECK(outer < ((i64)1 << 32), TB_ERR_SIZE, "too many outer indices");
+    c.outer = (unsigned)outer;
+    return true;
+}
+
+// op as k_pieces'; partial: kPieceBlocks sums for op 2 and 3
+constexpr int kPieceBlocks = 148*3;      // CTAs of the sums, whose partials have this many places
+
+// one resident wave (pc_blocks is what the kernel is compiled for)
+template <int OP>
+static unsigned pieces_grid(i64 tiles)
+{
+    return (unsigned)std::min<i64>(tiles, (i64)device_sm_count()*pc_blocks<OP>());
+}
+
+template <typename T>
+static void pieces_launch(int op, const T* A, T* B, const std::vector<PieceSpec>& specs, T alpha, T beta, bool conj_a,
+                          bool conj_b, int red_op, typename PcAcc<T>::type* partial, cudaStream_t st)
+{
+    std::vector<Piece> pieces;
+    i64 tiles = 0, elements = 0;
+    for (const PieceSpec& sp : specs) elements += total_of(sp.ab);
+    const i64 size = pc_size<T>(elements);
+    for (const PieceSpec& sp : specs)
+    {
+        Piece c;
+        if (!make_piece(sp, c)) continue;
+        if (op == 3) { c.turn = 0; }
+        const i64 n = pc_tiles<T>(c, size);
+        c.first = (unsigned)tiles;
+        tiles += n;
+        TB_CHECK(tiles < ((i64)1 << 32), TB_ERR_SIZE, "too many tiles");
+        pieces.push_back(c);
+    }
+    if (pieces.empty() && op < 2) return;
+    const Piece one = pieces.empty() ? Piece{} : pieces[0];
+    dbuf dev;
+    const Piece* many = nullptr;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (pieces.size() > 1 && op < 2 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusActive)
+    {
+        // a replay would read the table's source after this call: a launch per piece
+        for (const Piece& c : pieces)
+        {
+            Piece alone = c;
+            alone.first = 0;
+            const i64 n = pc_tiles<T>(alone, size);
+            if (op == 0)
+                k_pieces<T, 0><<<pieces_grid<0>(n), PC_THREADS, 0, st>>>(
+                    A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0, nullptr);
+            else
+                k_pieces<T, 1><<<pieces_grid<1>(n), PC_THREADS, 0, st>>>(
+                    A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0, nullptr);
+        }
+        check_launch("k_pieces");
+        return;
+    }
+    if (pieces.size() > 1)
+    {
+        dev = dbuf(pieces.size()*sizeof(Piece), st);
+        // pageable source: staged by the driver before the call returns
+        TB_CUDA(cudaMemcpyAsync(dev.ptr, pieces.data(), pieces.size()*sizeof(Piece), cudaMemcpyHostToDevice, st));
+        many = dev.as<Piece>();
+    }
+    const int np = (int)pieces.size();
+    const unsigned nt = (unsigned)tiles;
+    if (op == 0)
+        k_pieces<T, 0><<<pieces_grid<0>(tiles), PC_THREADS, 0, st>>>(
+            A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr);
+    else if (op == 1)
+        k_pieces<T, 1><<<pieces_grid<1>(tiles), PC_THREADS, 0, st>>>(
+            A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr);
+    else if (op == 2)
+        k_pieces<T, 2><<<kPieceBlocks, PC_THREADS, 0, st>>>(A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0,
+                                                            partial);
+    else
+        k_pieces<T, 3><<<kPieceBlocks, PC_THREADS, 0, st>>>(A, B, one, many, np, nt, alpha, beta, conj_a, conj_b,
+                                                            red_op, partial);
+    check_launch("k_pieces");
+}
+
+template <typename T>
+void l1_add_pieces(const T* A, T* B, const std::vector<PieceSpec>& pieces, T alpha, T beta, cudaStream_t st,
+                   bool conj_a, bool conj_b)
+{
+    pieces_launch<T>(beta == T(0) ? 0 : 1, A, B, pieces, alpha, beta, conj_a, conj_b, 0, nullptr, st);
+}
+
+template <typename T, typename Acc>
+static void pieces_sum(int op, int red_op, const T* A, const T* B, const std::vector<PieceSpec>& pieces, Acc* d_result,
+                       cudaStream_t st, bool conj_a, bool conj_b)
+{
+    dbuf part(kPieceBlocks*sizeof(Acc), st);
+    pieces_launch<T>(op, A, const_cast<T*>(B), pieces, T(0), T(0), conj_a, conj_b, red_op, part.as<Acc>(), st);
+    k_sum_partials<Acc><<<1, 32, 0, st>>>(part.as<Acc>(), kPieceBlocks, d_result);
+    check_launch("k_sum_partials");
+}
+
+template <typename T, typename Acc>
+void l1_dot_pieces(const T* A, const T* B, const std::vector<PieceSpec>& pieces, Acc* d_result, cudaStream_t st,
+                   bool conj_a, bool conj_b)
+{
+    pieces_sum<T, Acc>(2, 0, A, B, pieces, d_result, st, conj_a, conj_b);
+}
+
+template <typename T, typename Acc>
+void l1_sum_pieces(int red_op, const T* A, const std::vector<PieceSpec>& pieces, Acc* d_result, cudaStream_t st)
+{
+    pieces_sum<T, Acc>(3, red_op, A, A, pieces, d_result, st, false, false);
+}
+
 template <typename T>
 void l1_add(const T* A, T* B, const Strided2& ab, const Strided& ao, const Strided& bo,
             T alpha, T beta, cudaStream_t st, bool conj_a, bool conj_b)
@@ -624,9 +760,18 @@ void l1_add(const T* A, T* B, const Strided2& ab, const Strided& ao, const Strid
             if (std::llabs(ab.sa[d]) < std::llabs(ab.sa[pa])) pa = d;
             if (std::llabs(ab.sb[d]) < std::llabs(ab.sb[pb])) pb = d;
         }
-        if (pa == pb || ab.len[pa] == 1 || ab.len[pb] == 1)
+        const bool rows = pa == pb || ab.len[pa] == 1 || ab.len[pb] == 1;
+        // rows along a common fastest dim that are long and aligned move in 16-byte
+        // vectors, the others in tiles (which are numbered in 32 bits). 16.8M floats
+        // in rows of 128 and more, vectors and tiles: 34 and 44 us, with beta 38 and
+        // 53 (rows of 64: 68 and 44); doubles with beta 68 and 71 (unaligned rows 92
+        // and 72), without 56 and 51; complex doubles 187 and 128, 106 and 101
+        bool vectors = (sizeof(T) < 8 || (sizeof(T) == 8 && !b0)) && ab.len[pa] >= kLongRow && ab.sa[pa] == 1 &&
+                       ab.sb[pa] == 1 && (((uintptr_t)A | (uintptr_t)B) & 15) == 0;
+        for (int d = 0; d < ab.ndim && vectors; d++)
+            vectors = d == pa || (ab.sa[d]*(i64)sizeof(T) % 16 == 0 && ab.sb[d]*(i64)sizeof(T) % 16 == 0);
+        if (rows && (vectors || nab/ab.len[pa] >= ((i64)1 << 32)))
         {
-            // rows along the common fastest dim
             Strided2 s = ab;
             std::swap(s.len[0], s.len[pa]); std::swap(s.sa[0], s.sa[pa]); std::swap(s.sb[0], s.sb[pa]);
             i64 n0 = s.len[0];
@@ -638,41 +783,43 @@ void l1_add(const T* A, T* B, const Strided2& ab, const Strided& ao, const Strid
             check_launch("k_add_rows");
             return;
         }
-        constexpr int TT = tile_of<T>();
-        i64 tp = (ab.len[pa] + TT - 1)/TT, tq = (ab.len[pb] + TT - 1)/TT;
-        i64 outer = nab/(ab.len[pa]*ab.len[pb]);
-        i64 ntiles = tp*tq*outer;
-        TB_CHECK(ntiles < ((i64)1 << 32), TB_ERR_SIZE, "transpose: too many tiles");
-        // pairs: every pair (2i, 2i+1) along p in A and along q in B is
-        // contiguous and aligned to twice the element size
-        bool pairs = sizeof(T) <= 8 && ab.sa[pa] == 1 && ab.sb[pb] == 1 && ab.len[pa] % 2 == 0 &&
-                     ab.len[pb] % 2 == 0 && ((uintptr_t)A % (2*sizeof(T))) == 0 &&
-                     ((uintptr_t)B % (2*sizeof(T))) == 0;
-        for (int d = 0; d < ab.ndim && pairs; d++)
-        {
-            if (d != pa && ab.sa[d] % 2 != 0) pairs = false;
-            if (d != pb && ab.sb[d] % 2 != 0) pairs = false;
-        }
-        TimedLaunch t("k_transpose", st);
         if constexpr (sizeof(T) <= 8)
         {
+            // pairs: every pair (2i, 2i+1) along p in A and along q in B is
+            // contiguous and aligned to twice the element size; 64 x 64 tiles that are
+            // nearly full. FP64, 16.8M elements, here and in fitted tiles: extents 48
+            // 56 and 67 us, 64 48 and 52, 112 56 and 65, 160 56 and 57; but 32 92 and
+            // 51, 80 93 and 59, 100 67 and 61
+            auto full = [](i64 n)
+            {
+                return n <= TP_TILE ? 4*n >= 3*TP_TILE : 6*n >= 5*((n + TP_TILE - 1)/TP_TILE*TP_TILE);
+            };
+            bool pairs = !rows && ab.sa[pa] == 1 && ab.sb[pb] == 1 && ab.len[pa] % 2 == 0 &&
+                         ab.len[pb] % 2 == 0 && ((uintptr_t)A % (2*sizeof(T))) == 0 &&
+                         ((uintptr_t)B % (2*sizeof(T))) == 0 && full(ab.len[pa]) && full(ab.len[pb]);
+            for (int d = 0; d < ab.ndim && pairs; d++)
+            {
+                if (d != pa && ab.sa[d] % 2 != 0) pairs = false;
+                if (d != pb && ab.sb[d] % 2 != 0) pairs = false;
+            }
             if (pairs)
             {
-                const int grid = resident_grid(k_transpose<T, true, 2>, ntiles, L1_THREADS);
-                if (b0) k_transpose<T, true, 2><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer,
-                                                                             alpha, beta, conj_a, conj_b);
-                else k_transpose<T, false, 2><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer,
-                                                                            alpha, beta, conj_a, conj_b);
+                const i64 tp = (ab.len[pa] + TP_TILE - 1)/TP_TILE, tq = (ab.len[pb] + TP_TILE - 1)/TP_TILE;
+                const i64 outer = nab/(ab.len[pa]*ab.len[pb]);
+                const i64 ntiles = tp*tq*outer;
+                TB_CHECK(ntiles < ((i64)1 << 32), TB_ERR_SIZE, "transpose: too many tiles");
+                TimedLaunch t("k_transpose", st);
+                const int grid = resident_grid(k_transpose<T, true>, ntiles, L1_THREADS);
+                if (b0) k_transpose<T, true><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer,
+                                                                          alpha, beta, conj_a, conj_b);
+                else k_transpose<T, false><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer,
+                                                                         alpha, beta, conj_a, conj_b);
                 check_launch("k_transpose");
                 return;
             }
         }
-        const int grid = resident_grid(k_transpose<T, true, 1>, ntiles, L1_THREADS);
-        if (b0) k_transpose<T, true, 1><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer, alpha, beta,
-                                                                     conj_a, conj_b);
-        else k_transpose<T, false, 1><<<grid, L1_THREADS, 0, st>>>(A, B, ab, pa, pb, tp, tq, outer, alpha, beta,
-                                                                    conj_a, conj_b);
-        check_launch("k_transpose");
+        TimedLaunch t(rows ? "k_add_rows" : "k_transpose", st);
+        pieces_launch<T>(b0 ? 0 : 1, A, B, {{ab, 0, 0}}, alpha, beta, conj_a, conj_b, 0, nullptr, st);
         return;
     }
 
@@ -709,6 +856,11 @@ void l1_reduce(int op, const T* A, const Strided& s, T* d_value, i64* d_idx, cud
 }
 
 #define TB_L1_INST(T) \
+    template void l1_add_pieces<T>(const T*, T*, const std::vector<PieceSpec>&, T, T, cudaStream_t, bool, bool); \
+    template void l1_dot_pieces<T, PcAcc<T>::type>(const T*, const T*, const std::vector<PieceSpec>&, \
+                                                   PcAcc<T>::type*, cudaStream_t, bool, bool); \
+    template void l1_sum_pieces<T, PcAcc<T>::type>(int, const T*, const std::vector<PieceSpec>&, PcAcc<T>::type*, \
+                                                   cudaStream_t); \
     template void l1_set<T>(T*, const Strided&, T, cudaStream_t); \
     template void l1_scale<T>(T*, const Strided&, T, cudaStream_t, bool); \
     template void l1_shift<T>(T*, const Strided&, T, T, cudaStream_t, bool); \

@@ -49,6 +49,21 @@ void l1_dot(const T* A, const T* B, const Strided2& ab, T* d_result, cudaStream_
 template <typename S, typename D>
 void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st);
 
+// The same over many pieces in one launch (the stored blocks of a block-sparse
+// tensor): piece i is the index space ab[i] at offsets offa[i], offb[i]
+// (elements). Pieces of B must not overlap. The sums are left in device memory
+// in at least double precision; red_op is SUM, SUM_ABS or NORM_2 (squares,
+// no root).
+struct PieceSpec { Strided2 ab; i64 offa, offb; };
+template <typename T>
+void l1_add_pieces(const T* A, T* B, const std::vector<PieceSpec>& pieces, T alpha, T beta, cudaStream_t st,
+                   bool conj_a, bool conj_b);
+template <typename T, typename Acc>
+void l1_dot_pieces(const T* A, const T* B, const std::vector<PieceSpec>& pieces, Acc* d_result, cudaStream_t st,
+                   bool conj_a, bool conj_b);
+template <typename T, typename Acc>
+void l1_sum_pieces(int red_op, const T* A, const std::vector<PieceSpec>& pieces, Acc* d_result, cudaStream_t st);
+
 // reduction of A with op (reduce_t); writes value and offset to device memory
 template <typename T>
 void l1_reduce(int op, const T* A, const Strided& s, T* d_value, i64* d_idx, cudaStream_t st);
