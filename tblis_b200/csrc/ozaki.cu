@@ -644,10 +644,12 @@ struct CrtConsts
     int nm;                                  // moduli in use (the first nm)
     float m[CRT_MAX], inv[CRT_MAX];          // m_q and fl(1/m_q)
     float c16[CRT_MAX];                      // 2^16 mod m_q, in [0, m_q)
-    float g[CRT_MAX][CRT_MAX];               // g[q][j] = (m_0 ... m_(j-1)) mod m_q (centred)
-    float ginv[CRT_MAX];                     // (m_0 ... m_(q-1))^-1 mod m_q (centred)
-    double md[CRT_MAX];                      // m_q
+    // ((M/m_q)^-1 mod m_q)/m_q as hi + lo + tail: multiples of 2^-40 and 2^-80
+    // below 1 and 2^-40, and the rest
+    double hi[CRT_MAX], lo[CRT_MAX], tail[CRT_MAX];
+    double Mh, Ml;                           // M = m_0 ... m_(nm-1), rounded to double, and the rest
     double invd[CRT_MAX];                    // fl64(1/m_q)
+    uint32_t comp[CRT_MAX];                  // 256 - m_q (q > 0)
 };
 
 constexpr float F_BIAS = 8388608.0f;         // 2^23: (0x4B000000 | u) as float is 2^23 + u
@@ -711,7 +713,9 @@ struct PlaneGeom
 };
 
 constexpr int SL_LD = SL_T + 1;            // padded smem row (doubles)
-constexpr int SL_BLOCKS_PER_SM = 2;       // 128 registers a thread: more of the 16 elements' FP64 chains in flight
+// 128 registers a thread: more of the 16 elements' FP64 chains in flight (residues
+// with 3 blocks: 2.87 ms for 13 planes of 25600 x 25600 where 2 take 2.81)
+constexpr int SL_BLOCKS_PER_SM = 2;
 constexpr size_t SL_SMEM = 2*SL_T*SL_LD*sizeof(double);
 
 // writes the S tiled planes (PlaneGeom) of 64x64 tiles of the operand:
@@ -816,19 +820,28 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
             if constexpr (CRT)
             {
                 // e_rows holds the row's shift s. y = 1.5*2^52 + a with
-                // a = rint(x*2^s) (one rounding, |a| <= 2^50); the low byte of
-                // y is a mod 256; for odd m, y - m*rint(a/m) = 1.5*2^52 + r
-                // exactly, |r| <= (m-1)/2, and its low word is r. Three FP64
-                // operations per modulus; 16 k bytes per plane row.
+                // a = rint(x*2^s) (one rounding, |a| <= 2^50), so y's low byte is
+                // a mod 256. For odd m, z = 1.5*2^52 + rint(a/m) holds the quotient
+                // mod 2^32 in its low word, and the residue a - m*rint(a/m),
+                // |.| <= (m-1)/2, has the byte a + (256 - m)*rint(a/m) mod 256: with
+                // bytes 0 and 2 of a word holding two elements, one integer
+                // multiply-add serves both (256 + 63*255 stays below 2^16). One FP64
+                // operation per modulus and element, where subtracting m*rint(a/m)
+                // in FP64 took three and bound the pass: 2.9 ms for the ladder's A
+                // against 2.1 ms that its 13.8 GB take.
                 constexpr double SH = 6755399441055744.0;
                 const int sh1 = e >> 1, sh2 = e - sh1;
                 const double sc1 = pow2i(sh1), sc2 = pow2i(sh2);
-                double y[16], av[16];
+                double av[16];
+                uint32_t ylo[8];                 // low bytes of two elements each
                 #pragma unroll
-                for (int u = 0; u < 16; u++)
+                for (int u = 0; u < 16; u += 2)
                 {
-                    y[u] = __fma_rn(__dmul_rn(src[u], sc1), sc2, SH);
-                    av[u] = __dsub_rn(y[u], SH);
+                    const double y0 = __fma_rn(__dmul_rn(src[u], sc1), sc2, SH);
+                    const double y1 = __fma_rn(__dmul_rn(src[u + 1], sc1), sc2, SH);
+                    av[u] = __dsub_rn(y0, SH);
+                    av[u + 1] = __dsub_rn(y1, SH);
+                    ylo[u/2] = __byte_perm((uint32_t)__double2loint(y0), (uint32_t)__double2loint(y1), 0x0400) & 0x00ff00ffu;
                 }
                 const i64 plane_stride = tile_bytes;
                 unsigned char* dst = block(kk);
@@ -839,20 +852,20 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
                     #pragma unroll
                     for (int g = 0; g < 4; g++)
                     {
-                        uint32_t b[4];
+                        uint32_t r[2];
                         #pragma unroll
-                        for (int u = 0; u < 4; u++)
+                        for (int h = 0; h < 2; h++)
                         {
-                            const int i = g*4 + u;
-                            if (q == 0) b[u] = (uint32_t)__double2loint(y[i]);
+                            const int i = g*4 + h*2;
+                            if (q == 0) r[h] = ylo[i/2];
                             else
                             {
-                                const double qm = __dsub_rn(__fma_rn(av[i], cc.invd[q], SH), SH);
-                                b[u] = (uint32_t)__double2loint(__fma_rn(-qm, cc.md[q], y[i]));
+                                const uint32_t z0 = (uint32_t)__double2loint(__fma_rn(av[i], cc.invd[q], SH));
+                                const uint32_t z1 = (uint32_t)__double2loint(__fma_rn(av[i + 1], cc.invd[q], SH));
+                                r[h] = (__byte_perm(z0, z1, 0x0400) & 0x00ff00ffu)*cc.comp[q] + ylo[i/2];
                             }
                         }
-                        // byte 0 of each word, four to a word
-                        w[g] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+                        w[g] = __byte_perm(r[0], r[1], 0x6420);
                     }
                     *reinterpret_cast<uint4*>(dst + q*plane_stride) = make_uint4(w[0], w[1], w[2], w[3]);
                 }
@@ -1278,11 +1291,18 @@ struct CrtCombineArgs
 
 // One block of 256 threads per (output tile, batch index, quarter of the
 // tile's columns): lane t of a warp takes rows 4t..4t+3 and warp w the
-// columns w, w+8, ... of the quarter; for each element
-// it sums the chunk residues, recovers the balanced mixed-radix digits v_q of
-// the integer product (Garner's algorithm, exact in FP32), evaluates
-// sum v_q m_0...m_(q-1) by Horner in FP64, scales by 2^-(sA+sB) and applies
-// alpha and beta through C's scatter vectors (beta == 0: C is not read).
+// columns w, w+8, ... of the quarter. For each element it sums the chunk residues
+// and recovers the integer x they stand for: x/M is the sum over the moduli of
+// r_q times ((M/m_q)^-1 mod m_q)/m_q, less the nearest integer (the Chinese
+// remainder theorem; as in the published Ozaki scheme II, the fractions are split
+// so that the sums are exact). With 40-bit pieces the first two of the three sums
+// are exact in FP64 (16 terms below 2^48 units) and the third is below 2^-68, so
+// x/M is known to 2^-107: to 13 moduli (M below 2^104) x is the exact integer up to
+// 2^51 and one rounding of it above; with more, |x| stays below 2^101 and is known
+// to 2^20. Then 2^-(sA+sB), alpha and beta through C's scatter
+// vectors (beta == 0: C is not read). Bound by FP64 issue, about 5 operations a
+// modulus; Garner's mixed radix digits in FP32 before took NM^2/2 more and 0.73
+// ms for the ladder's 59 M elements, against 0.19 ms for their bytes.
 template <int NM>
 __global__ void __launch_bounds__(256)
 oz_crt_combine(const CrtCombineArgs p)
@@ -1327,31 +1347,36 @@ oz_crt_combine(const CrtCombineArgs p)
         #pragma unroll
         for (int q = 0; q < NM; q++) wc[q] = wn[q];
         if (col + 8 < c1 && n + 8 < p.N) load(col + 8);
-        float v[RW][NM];
+        constexpr double TWO52 = 4503599627370496.0;
+        double sh[RW], sl[RW], stl[RW];
+        #pragma unroll
+        for (int r = 0; r < RW; r++) sh[r] = sl[r] = stl[r] = 0.0;
         #pragma unroll
         for (int q = 0; q < NM; q++)
         {
             uint32_t rs[RW];
             #pragma unroll
             for (int r = 0; r < RW; r++) rs[r] = (wc[q] >> (8*r)) & 0xFFu;
-            for (int ch = 1; ch < p.chunks; ch++)
+            if (p.chunks > 1)
             {
-                const uint32_t w = *reinterpret_cast<const uint32_t*>(base + ch*p.chunk_bytes +
-                                                                      q*(i64)CRT_OUT_TILE + col*OZ_BM);
+                for (int ch = 1; ch < p.chunks; ch++)
+                {
+                    const uint32_t w = *reinterpret_cast<const uint32_t*>(base + ch*p.chunk_bytes +
+                                                                          q*(i64)CRT_OUT_TILE + col*OZ_BM);
+                    #pragma unroll
+                    for (int r = 0; r < RW; r++) rs[r] += (w >> (8*r)) & 0xFFu;
+                }
                 #pragma unroll
-                for (int r = 0; r < RW; r++) rs[r] += (w >> (8*r)) & 0xFFu;
+                for (int r = 0; r < RW; r++) rs[r] %= (uint32_t)crt_modulus(q);
             }
-            const float mq = p.cc.m[q], inv = p.cc.inv[q], gi = p.cc.ginv[q];
+            const double h = p.cc.hi[q], lo = p.cc.lo[q], tl = p.cc.tail[q];
             #pragma unroll
             for (int r = 0; r < RW; r++)
             {
-                // r_q minus the digits found so far at their weights, times the
-                // inverse weight, modulo m_q, balanced: |.| < 2^18 and 2^14, exact
-                float t = __fsub_rn(__int_as_float(0x4B000000 | (int)rs[r]), F_BIAS);
-                #pragma unroll
-                for (int i = 0; i < q; i++) t = __fmaf_rn(-v[r][i], p.cc.g[q][i], t);
-                t = crt_reduce(t, mq, inv);
-                v[r][q] = crt_reduce(__fmul_rn(t, gi), mq, inv);
+                const double d = __hiloint2double(0x43300000, (int)rs[r]) - TWO52;
+                sh[r] = fma(d, h, sh[r]);
+                sl[r] = fma(d, lo, sl[r]);
+                stl[r] = fma(d, tl, stl[r]);
             }
         }
         const int sb = p.sB[(i64)l*p.N + n];
@@ -1361,9 +1386,14 @@ oz_crt_combine(const CrtCombineArgs p)
         for (int r = 0; r < RW; r++)
         {
             if (m0 + r >= p.M) break;
-            double x = (double)v[r][NM - 1];
-            #pragma unroll
-            for (int q = NM - 2; q >= 0; q--) x = fma(x, p.cc.md[q], (double)v[r][q]);
+            // x/M = f + fe + stl, f + fe = frac(sh) + sl exactly; then times M
+            const double fh = __dsub_rn(sh[r], rint(sh[r]));
+            const double f = __dadd_rn(fh, sl[r]), bb = __dsub_rn(f, fh);
+            const double fe = __dadd_rn(__dsub_rn(fh, __dsub_rn(f, bb)), __dsub_rn(sl[r], bb));
+            const double ph = __dmul_rn(p.cc.Mh, f);
+            const double pl = fma(p.cc.Mh, fe + stl[r], fma(p.cc.Ml, f, fma(p.cc.Mh, f, -ph)));
+            double x = ph + pl;
+            if (NM <= 13 && fabs(x) < 2251799813685248.0) x = rint(x);
             // 2^-(sA+sB) as two normal powers of two where the shifts allow
             const double val = p.alpha*((fast && sb > -500 && sb < 500) ? x*rsc[r]*csc : ldexp(x, -(sa[r] + sb)));
             double* dst = C + cm[r] + cn;
@@ -1453,6 +1483,77 @@ void gemm_dispatch(int kind, int S, const OzGemmArgs& a, cudaStream_t st)
     else launch_gemm<1, OZ_TF32>(a, st);
 }
 
+// The error models' sums over one operand's rows, taken on the device: the host
+// needs six numbers, and fetching the rows and summing them there left the GPU
+// idle for 1.7 ms of a 19.4 ms ladder contraction.
+struct RowSums
+{
+    double ss;               // sum of the rows' sums of squares
+    double num1, num2;       // sum of 4^(e - emax) over the rows: e of the row maxima, of the row norms
+    int emax1, emax2;        // largest such exponent (-100000: none)
+};
+
+constexpr int RS_THREADS = 1024;
+
+// block 0: A's rows, block 1: B's; fixed order of summation
+__global__ void __launch_bounds__(RS_THREADS)
+oz_row_sums(const int* eA, const double* sA, i64 nA, const int* eB, const double* sB, i64 nB, RowSums* out)
+{
+    const int* e = blockIdx.x ? eB : eA;
+    const double* s = blockIdx.x ? sB : sA;
+    const i64 n = blockIdx.x ? nB : nA;
+    __shared__ double sd[32], sd2[32];
+    __shared__ int si[32], si2[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // exponent of a row's norm, as oz_crt_shifts takes it
+    auto norm_exp = [](double ss)
+    {
+        const double v = sqrt(ss);
+        int x = -100000;
+        if (v > 0.0 && v <= 1.7e308) frexp(v*(1.0 + 0x1p-20), &x);
+        return x;
+    };
+    double sum = 0.0;
+    int m1 = -100000, m2 = -100000;
+    for (i64 i = threadIdx.x; i < n; i += RS_THREADS)
+    {
+        sum += s[i];
+        m1 = max(m1, e[i]);
+        m2 = max(m2, norm_exp(s[i]));
+    }
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        m1 = max(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+        m2 = max(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+    }
+    if (lane == 0) { sd[warp] = sum; si[warp] = m1; si2[warp] = m2; }
+    __syncthreads();
+    sum = 0.0;
+    for (int w = 0; w < RS_THREADS/32; w++) { sum += sd[w]; m1 = max(m1, si[w]); m2 = max(m2, si2[w]); }
+    __syncthreads();
+    double n1 = 0.0, n2 = 0.0;
+    for (i64 i = threadIdx.x; i < n; i += RS_THREADS)
+    {
+        n1 += ldexp(1.0, 2*(e[i] - m1));
+        const int x = norm_exp(s[i]);
+        if (x > -100000) n2 += ldexp(1.0, 2*(x - m2));
+    }
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        n1 += __shfl_xor_sync(0xffffffffu, n1, o);
+        n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    }
+    if (lane == 0) { sd[warp] = n1; sd2[warp] = n2; }
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        n1 = n2 = 0.0;
+        for (int w = 0; w < RS_THREADS/32; w++) { n1 += sd[w]; n2 += sd2[w]; }
+        out[blockIdx.x] = RowSums{sum, n1, n2, m1, m2};
+    }
+}
+
 // a-priori normwise error estimate for S slices (rounding of both operands
 // to S digits plus the dropped cross terms), from per-row maxima and norms:
 // rounding row i to S digits leaves an error of about 2^(e_i - 7S) per
@@ -1462,25 +1563,16 @@ struct ErrorModel
 {
     double ra2 = 0, rb2 = 0;      // squared relative error at S = 0: mantissa ...
     int ea = 0, eb = 0;           // ... and binary exponent
-    static void build(const std::vector<int>& e, const std::vector<double>& ss, i64 K, double& m, int& ex)
+    static void build(const RowSums& r, i64 K, double& m, int& ex)
     {
-        int emax = -100000;
-        for (int v : e) emax = std::max(emax, v);
-        double num = 0.0, den = 0.0;
-        for (size_t i = 0; i < e.size(); i++)
-        {
-            num += std::ldexp(1.0, 2*(e[i] - emax));
-            den += ss[i];
-        }
-        if (den <= 0.0 || num == 0.0) { m = 0.0; ex = 0; return; }
-        m = (double)K/3.0*num/den;
-        ex = 2*emax;
+        if (r.ss <= 0.0 || r.num1 == 0.0) { m = 0.0; ex = 0; return; }
+        m = (double)K/3.0*r.num1/r.ss;
+        ex = 2*r.emax1;
     }
-    ErrorModel(const std::vector<int>& eA, const std::vector<double>& ssA,
-               const std::vector<int>& eB, const std::vector<double>& ssB, i64 K)
+    ErrorModel(const RowSums& A, const RowSums& B, i64 K)
     {
-        build(eA, ssA, K, ra2, ea);
-        build(eB, ssB, K, rb2, eb);
+        build(A, K, ra2, ea);
+        build(B, K, rb2, eb);
     }
     // residual bound of S digits relative to 2^e: base 254 (INT8):
     // 1/(2*127*254^(S-1)); base 128 (BF16): 2^-7S
@@ -1505,15 +1597,6 @@ double diagonal_weight(int kind, int d)
 }
 
 // ---- scheme II host side ------------------------------------------------------
-
-// (2 m + 1)/2 rounded: x mod m in [-(m-1)/2, (m-1)/2] ([-128, 127] for 256)
-i64 centred(i64 x, i64 m)
-{
-    x %= m;
-    if (x < 0) x += m;
-    if (2*x >= m) x -= m;
-    return x;
-}
 
 i64 powmod(i64 b, i64 e, i64 m)
 {
@@ -1577,17 +1660,26 @@ CrtConsts crt_consts(int nm)
         const i64 m = crt_modulus(q);
         c.m[q] = (float)m;
         c.inv[q] = 1.0f/(float)m;
-        c.md[q] = (double)m;
         c.invd[q] = 1.0/(double)m;
+        c.comp[q] = (uint32_t)(256 - m);
         c.c16[q] = (float)powmod(2, 16, m);
-        i64 P = 1 % m;                               // m_0 ... m_(j-1) mod m_q
-        for (int j = 0; j < q; j++)
-        {
-            c.g[q][j] = (float)centred(P, m);
-            P = P*crt_modulus(j) % m;
-        }
-        c.ginv[q] = q == 0 ? 1.0f : (float)centred(invmod(P, m), m);
+        i64 P = 1 % m;                               // M/m_q mod m_q
+        for (int j = 0; j < nm; j++)
+            if (j != q) P = P*crt_modulus(j) % m;
+        i64 t = invmod(P, m);                        // t/m_q in base 2^-40
+        const i64 d1 = (t << 40)/m;
+        t = (t << 40) % m;
+        const i64 d2 = (t << 40)/m;
+        t = (t << 40) % m;
+        c.hi[q] = std::ldexp((double)d1, -40);
+        c.lo[q] = std::ldexp((double)d2, -80);
+        c.tail[q] = std::ldexp((double)t/(double)m, -80);
     }
+    unsigned __int128 M = 1;                         // below 2^126
+    for (int q = 0; q < nm; q++) M *= (unsigned __int128)crt_modulus(q);
+    c.Mh = (double)M;
+    const unsigned __int128 back = (unsigned __int128)c.Mh;
+    c.Ml = M >= back ? (double)(M - back) : -(double)(back - M);
     return c;
 }
 
@@ -1613,29 +1705,15 @@ struct CrtErrorModel
 {
     double ra = 0, rb = 0;   // sqrt(K/12 sum 4^(e_i - emax)/sum ss) ...
     int ea = 0, eb = 0;      // ... and emax
-    static void build(const std::vector<double>& ss, i64 K, double& r, int& emax)
+    static void build(const RowSums& s, i64 K, double& r, int& emax)
     {
-        std::vector<int> e(ss.size());
-        emax = -100000;
-        double den = 0.0;
-        for (size_t i = 0; i < ss.size(); i++)
-        {
-            const double v = std::sqrt(ss[i]);
-            int x = -100000;
-            if (v > 0.0 && v <= 1.7e308) std::frexp(v*(1.0 + 0x1p-20), &x);
-            e[i] = x;
-            emax = std::max(emax, x);
-            den += ss[i];
-        }
-        double num = 0.0;
-        for (int x : e)
-            if (x > -100000) num += std::ldexp(1.0, 2*(x - emax));
-        r = den > 0.0 && num > 0.0 ? std::sqrt((double)K/12.0*num/den) : 0.0;
+        emax = s.emax2;
+        r = s.ss > 0.0 && s.num2 > 0.0 ? std::sqrt((double)K/12.0*s.num2/s.ss) : 0.0;
     }
-    CrtErrorModel(const std::vector<double>& ssA, const std::vector<double>& ssB, i64 K)
+    CrtErrorModel(const RowSums& A, const RowSums& B, i64 K)
     {
-        build(ssA, K, ra, ea);
-        build(ssB, K, rb, eb);
+        build(A, K, ra, ea);
+        build(B, K, rb, eb);
     }
     double operator()(int nm) const
     {
@@ -1822,6 +1900,11 @@ void ozaki_begin(OzakiJob& j, cudaStream_t st)
                     j.tab->b_n_step, j.tab->b_k_step};
     stats(oa, j.eA.as<int>(), j.sA.as<double>(), st);
     stats(ob, j.eB.as<int>(), j.sB.as<double>(), st);
+    if (j.single) return;
+    j.sums = dbuf(2*sizeof(RowSums), st);
+    oz_row_sums<<<2, RS_THREADS, 0, st>>>(j.eA.as<int>(), j.sA.as<double>(), v.l*v.m, j.eB.as<int>(), j.sB.as<double>(),
+                                          v.l*v.n, j.sums.as<RowSums>());
+    check_launch("oz_row_sums");
 }
 
 void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
@@ -1840,33 +1923,23 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
     else
     {
         // the error model (and, without an explicit count, the slice count)
-        std::vector<int> heA(v.l*v.m), heB(v.l*v.n);
-        std::vector<double> hsA(v.l*v.m), hsB(v.l*v.n);
-        if (stats_ready)
-        {
-            // the statistics are complete: copy them without queueing behind
-            // the caller's stream
-            TB_CUDA(cudaMemcpy(heA.data(), j.eA.ptr, heA.size()*sizeof(int), cudaMemcpyDeviceToHost));
-            TB_CUDA(cudaMemcpy(heB.data(), j.eB.ptr, heB.size()*sizeof(int), cudaMemcpyDeviceToHost));
-            TB_CUDA(cudaMemcpy(hsA.data(), j.sA.ptr, hsA.size()*sizeof(double), cudaMemcpyDeviceToHost));
-            TB_CUDA(cudaMemcpy(hsB.data(), j.sB.ptr, hsB.size()*sizeof(double), cudaMemcpyDeviceToHost));
-        }
+        RowSums rs[2];
+        // (statistics that are complete: fetched without queueing behind the
+        // caller's stream)
+        if (stats_ready) TB_CUDA(cudaMemcpy(rs, j.sums.ptr, sizeof(rs), cudaMemcpyDeviceToHost));
         else
         {
-            TB_CUDA(cudaMemcpyAsync(heA.data(), j.eA.ptr, heA.size()*sizeof(int), cudaMemcpyDeviceToHost, st));
-            TB_CUDA(cudaMemcpyAsync(heB.data(), j.eB.ptr, heB.size()*sizeof(int), cudaMemcpyDeviceToHost, st));
-            TB_CUDA(cudaMemcpyAsync(hsA.data(), j.sA.ptr, hsA.size()*sizeof(double), cudaMemcpyDeviceToHost, st));
-            TB_CUDA(cudaMemcpyAsync(hsB.data(), j.sB.ptr, hsB.size()*sizeof(double), cudaMemcpyDeviceToHost, st));
+            TB_CUDA(cudaMemcpyAsync(rs, j.sums.ptr, sizeof(rs), cudaMemcpyDeviceToHost, st));
             TB_CUDA(cudaStreamSynchronize(st));
         }
-        const ErrorModel est(heA, hsA, heB, hsB, v.k);
+        const ErrorModel est(rs[0], rs[1], v.k);
         // scheme II (moduli) is an INT8 option: its count from the
         // tolerance, or the caller's when it forces the scheme
         int nm = 0;
         double nm_err = 0;
         if (kind == OZ_I8 && j.scheme != 1)
         {
-            const CrtErrorModel est2(hsA, hsB, v.k);
+            const CrtErrorModel est2(rs[0], rs[1], v.k);
             if (j.scheme == 2 && S > 0) nm = S;
             else
                 for (int q = 2; q <= CRT_MAX; q++)

@@ -41,6 +41,7 @@ struct OzakiJob
     int scheme = 0;
     std::shared_ptr<GemmTables> tab;
     dbuf eA, eB, sA, sB;             // row exponents and sums of squares
+    dbuf sums;                       // their sums over the rows of A and of B
     OzakiResult res;
 };
 // queues the row statistics of A and B on st
