@@ -561,14 +561,16 @@ void gemm_f64_variant_tile(int variant, int& bm, int& bn)
     bm = v.bm; bn = v.bn;
 }
 
-int gemm_f64_grouped_num_variants() { return kNumVariants + 1; }
+int gemm_f64_grouped_num_variants() { return kNumVariants + 2; }
 bool gemm_f64_is_ws_variant(int variant) { return variant == kNumVariants + 1; }
+bool gemm_f64_is_dense_variant(int variant) { return variant == kNumVariants + 2; }
 
 void gemm_f64_grouped_launch(const GroupDesc* d_groups, const i64* d_tile_begin, int ngroups,
                              i64 total_tiles, int variant, cudaStream_t stream, unsigned long long* d_counter)
 {
     if (ngroups <= 0 || total_tiles <= 0) return;
-    TB_CHECK(!gemm_f64_is_ws_variant(variant), TB_ERR_ARG, "the packed variant runs through its grouped plan");
+    TB_CHECK(!gemm_f64_is_ws_variant(variant) && !gemm_f64_is_dense_variant(variant), TB_ERR_ARG,
+             "the packed and dense variants run through their grouped plan");
     const Variant& v = kVariants[std::max(1, std::min(variant, kNumVariants)) - 1];
     if (d_counter) TB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long), stream));
     v.grouped(d_groups, d_tile_begin, ngroups, total_tiles, d_counter, stream);

@@ -65,7 +65,27 @@ struct GroupDesc
     int shape;
     int nst;
     i64 pa, pb;
+    // dense grouped path: gather of A and B: 0 single elements, 1 pairs; in a plan
+    // whose groups differ in direction 0 and 1 along k, 2 single elements along the
+    // rows
+    int how_a, how_b;
 };
+
+// The dense grouped path (gemm_f64_dense.cu): a plan lists the 128 x 128 tiles
+// of its groups (those with k steps), and gemm_f64_group_dense_plan deals their k
+// steps to CTAs in runs of equal modelled cost: CTA c starts at start[c] and ends
+// at start[c + 1]; cuts lists the tiles that several CTAs share.
+struct GroupTile { int g, tm, tn; };
+struct GroupStart { int tile, step; };
+struct GroupCut { int tile, cta, count, slot; };     // runs of CTAs [cta, cta + count), the first in `slot`
+struct GroupExtents { i64 M, N; int nst; };
+void gemm_f64_group_dense_tile(int& bm, int& bn);
+size_t gemm_f64_group_dense_bytes(int ctas);         // workspace for the partial sums
+void gemm_f64_group_dense_plan(const std::vector<GroupTile>& tiles, const std::vector<GroupExtents>& groups, int sms,
+                               std::vector<GroupStart>& start, std::vector<GroupCut>& cuts);
+void gemm_f64_group_dense_launch(const GroupDesc* d_groups, const GroupTile* d_tiles, const GroupStart* d_start, int ctas,
+                                 const GroupCut* d_cuts, int ncuts, double* partial, int modes, cudaStream_t s);
+// (modes: 2*amode + bmode shared by all groups, or 4)
 
 // one piece of a panel to pack: k steps [s0, s0 + ns) of rows
 // [panel*BM, ...) of group g's A (side 0), or of columns [panel*BN, ...) of
@@ -77,11 +97,13 @@ struct PackItem
 
 int gemm_f64_num_variants();
 void gemm_f64_variant_tile(int variant, int& bm, int& bn);
-// variants of a grouped launch: the tile family above, then the packed path
+// variants of a grouped launch: the tile family above, the packed path
 // (variant gemm_f64_num_variants() + 1, tiles of each group's own shape; run
 // by the grouped plan, not by gemm_f64_grouped_launch)
 int gemm_f64_grouped_num_variants();
 bool gemm_f64_is_ws_variant(int variant);
+// the dense grouped path, the last variant
+bool gemm_f64_is_dense_variant(int variant);
 
 // The packed grouped path (gemm_f64_ws.cu): gemm_f64_ws_pack gathers the A
 // row panels and B column panels of every group into contiguous, swizzled

@@ -283,15 +283,18 @@ struct Gather
         }
         else
         {
-            // the rows this warp copies: PER consecutive ones at each of J steps
+            // the rows this warp copies, PER consecutive ones at each of J steps, in
+            // its own quarter of sro: which rows they are depends on W, and another
+            // warp may still be at a run that was gathered with the other W
             constexpr int PER = 32/LANES;
+            static_assert(PER*J == R/DN_PRODUCERS, "a warp's share of the rows");
             int odd = 0;
             __syncwarp();
             for (int x = t % 32; x < PER*J; x += 32)
             {
                 const int r = (t/32)*PER + x % PER + x/PER*STEP;
                 const i64 o = r < rem ? __ldg(rvec + r) : 0;
-                sro[r] = o;
+                sro[(t/32)*(PER*J) + x] = o;
                 odd |= (int)(o & 1);
             }
             even = __all_sync(0xffffffffu, odd == 0) != 0;
@@ -384,6 +387,8 @@ struct Gather
         }
         else
         {
+            constexpr int PER = 32/LANES;
+            const i64* ros = sro + (t/32)*(PER*J) + (t % 32)/LANES;    // row t/LANES + j*STEP: ros[j*PER]
             const int kl = W*(t % LANES);
             const i64 o0 = __shfl_sync(0xffffffffu, mine, base + kl);
             const i64 o1 = W == 2 ? __shfl_sync(0xffffffffu, mine, base + kl + W - 1) : 0;
@@ -395,11 +400,11 @@ struct Gather
                 if (rem < R)
                 {
                     #pragma unroll 4
-                    for (int r = t/LANES; r < rem; r += STEP)
+                    for (int j = 0; t/LANES + j*STEP < rem; j++)
                     {
-                        double* dst = Xs + tile_pos<R, MODE>(r, kl);
-                        if (W == 2) cp_pair16(dst, Xk + sro[r]);
-                        else cp_elem(dst, Xk + sro[r]);
+                        double* dst = Xs + tile_pos<R, MODE>(t/LANES + j*STEP, kl);
+                        if (W == 2) cp_pair16(dst, Xk + ros[j*PER]);
+                        else cp_elem(dst, Xk + ros[j*PER]);
                     }
                     return;
                 }
@@ -408,8 +413,8 @@ struct Gather
                 {
                     const int r = t/LANES + j*STEP;
                     double* dst = Xs + tile_pos<R, MODE>(r, kl);
-                    if (W == 2) cp_pair16(dst, Xk + sro[r]);
-                    else cp_elem(dst, Xk + sro[r]);
+                    if (W == 2) cp_pair16(dst, Xk + ros[j*PER]);
+                    else cp_elem(dst, Xk + ros[j*PER]);
                 }
                 return;
             }
@@ -419,7 +424,7 @@ struct Gather
             {
                 const int r = t/LANES + j*STEP;
                 if (r >= rem) break;
-                const i64 row = sro[r];
+                const i64 row = ros[j*PER];
                 double* dst = Xs + tile_pos<R, MODE>(r, kl);
                 if (adj && ok1 && ((uintptr_t)(Xk + row) & 15) == 0) cp_pair16(dst, Xk + row);
                 else
@@ -435,6 +440,47 @@ struct Gather
     {
         if (pairs) copy<2>(Xs, u, kvalid);
         else copy<1>(Xs, u, kvalid);
+    }
+};
+
+// The gather of a grouped GEMM, whose direction differs from group to group: one
+// stage layout (MODE 1) for both. how: 0 single elements along k, 1 pairs along k,
+// 2 single elements along the rows.
+template <int R>
+struct GatherG : Gather<R, 1>
+{
+    typedef Gather<R, 1> Base;
+    static constexpr int STEP = DN_PT/R, J = BK/STEP;         // along the rows: k per pass, copies per thread
+    static_assert(DN_PT % R == 0 && J*STEP == BK, "gather geometry");
+
+    __device__ __forceinline__ void start(const double* X_, const i64* rvec, const i64* kvec_, i64 r0, int rem_, int how)
+    {
+        if (how < 2) { Base::start(X_, rvec, kvec_, r0, rem_, how == 1); return; }
+        this->X = X_; this->kvec = kvec_;
+        this->rem = rem_;
+        const int r = threadIdx.x % R;
+        this->ro[0] = r < rem_ ? __ldg(rvec + r0 + r) : 0;
+    }
+
+    __device__ __forceinline__ void stage(double* Xs, int u, int kvalid, int how) const
+    {
+        if (how < 2) { Base::stage(Xs, u, kvalid, how == 1); return; }
+        const i64 mine = u & 2 ? this->ko[1] : this->ko[0];
+        const int t = threadIdx.x % DN_PT, base = (u & 1)*BK, r = t % R, k0 = t/R;
+        i64 k[J];
+        #pragma unroll
+        for (int j = 0; j < J; j++) k[j] = __shfl_sync(0xffffffffu, mine, base + k0 + j*STEP);
+        if (r >= this->rem) return;
+        const double* Xr = this->X + this->ro[0];
+        if (kvalid == BK)
+        {
+            #pragma unroll
+            for (int j = 0; j < J; j++) cp_elem(Xs + tile_pos<R, 1>(r, k0 + j*STEP), Xr + k[j]);
+            return;
+        }
+        #pragma unroll
+        for (int j = 0; j < J; j++)
+            cp_elem(Xs + tile_pos<R, 1>(r, k0 + j*STEP), Xr + k[j], k0 + j*STEP < kvalid);
     }
 };
 
@@ -519,6 +565,11 @@ struct GatherZ
     }
 };
 
+// MODE 2: the direction is chosen at run time
+template <int R, int MODE, bool CPLX> struct GatherOf { typedef Gather<R, MODE> type; };
+template <int R> struct GatherOf<R, 2, false> { typedef GatherG<R> type; };
+template <int R, int MODE> struct GatherOf<R, MODE, true> { typedef GatherZ<R> type; };
+
 // ---- kernel ---------------------------------------------------------------------------
 
 // Row-warp and column-warp of a consumer warp. Warps cw and cw + 4 share an SM
@@ -563,6 +614,104 @@ __device__ __forceinline__ void update_z(const GemmF64Args& p, double* dst, doub
     *reinterpret_cast<double2*>(dst) = make_double2(vr, vi);
 }
 
+// the operands of one K segment of a tile; how_a / how_b as the gathers take them
+struct Operands
+{
+    const double *A, *B;
+    const i64 *a_m, *a_k, *b_n, *b_k;
+    i64 K;
+    int how_a, how_b;
+};
+
+// where a tile's results go
+struct Target
+{
+    double* C;
+    const i64 *c_m, *c_n;
+    double alpha, beta;
+};
+
+// one contraction (possibly with a batch index)
+template <int BM, int BN, bool CPLX>
+struct DenseWork
+{
+    typedef TileAt Tile;
+    const GemmF64Args& p;
+    __device__ __forceinline__ const GemmF64Args& args() const { return p; }
+    __device__ __forceinline__ bool run(unsigned r, Run& out) const { return run_at(p, blockIdx.x, r, out); }
+    __device__ __forceinline__ Tile tile(const Run& run) const { return tile_at<BM, BN>(p, run.tile); }
+    __device__ __forceinline__ int segments(const Tile&) const { return 1; }
+    __device__ __forceinline__ Operands operands(const Tile& t, int) const
+    {
+        constexpr int ES = CPLX ? 2 : 1;
+        return Operands{p.A + ES*p.a_l[t.l], p.B + ES*p.b_l[t.l], p.a_m, p.a_k, p.b_n, p.b_k, p.K,
+                        CPLX ? p.amode == 0 : p.pair_a != 0, CPLX ? p.bmode == 0 : p.pair_b != 0};
+    }
+    __device__ __forceinline__ Target target(const Tile& t) const
+    {
+        return Target{p.C + (CPLX ? 2 : 1)*p.c_l[t.l], p.c_m, p.c_n, p.alpha, p.beta};
+    }
+    __device__ __forceinline__ double* partial() const { return p.partial; }
+};
+
+// The GEMMs of a grouped plan: tiles listed by the plan (group by group), the k
+// steps of all of them dealt to the CTAs in runs of equal modelled cost, which the
+// plan has worked out too: CTA c takes k steps [start[c], start[c + 1]).
+template <int BM, int BN>
+struct GroupWork
+{
+    struct Tile
+    {
+        i64 m0, n0;
+        int mrem, nrem;
+        const GroupDesc* g;
+    };
+    const GroupDesc* groups;
+    const GroupTile* tiles;
+    const GroupStart* start;
+    double* w;
+    __device__ __forceinline__ GemmF64Args args() const { return GemmF64Args(); }     // complex groups do not occur
+    __device__ __forceinline__ bool run(unsigned r, Run& out) const
+    {
+        const GroupStart a = start[blockIdx.x], b = start[blockIdx.x + 1];
+        const int t = a.tile + (int)r;
+        if (t > b.tile || (t == b.tile && b.step == 0)) return false;
+        const int nst = groups[tiles[t].g].nst;
+        out.tile = (unsigned)t;
+        out.s0 = r == 0 ? a.step : 0;
+        out.s1 = t == b.tile ? b.step : nst;
+        out.slot = out.s1 - out.s0 == nst ? -1 : r == 0 ? 0 : 1;
+        return out.s0 < out.s1;
+    }
+    __device__ __forceinline__ Tile tile(const Run& run) const
+    {
+        const GroupTile x = tiles[run.tile];
+        Tile t;
+        t.g = groups + x.g;
+        t.m0 = (i64)x.tm*BM;
+        t.n0 = (i64)x.tn*BN;
+        t.mrem = (int)min((i64)BM, t.g->M - t.m0);
+        t.nrem = (int)min((i64)BN, t.g->N - t.n0);
+        return t;
+    }
+    __device__ __forceinline__ int segments(const Tile& t) const { return t.g->nseg > 0 ? t.g->nseg : 1; }
+    __device__ __forceinline__ Operands operands(const Tile& t, int sg) const
+    {
+        const GroupDesc& g = *t.g;
+        if (g.nseg > 0)
+        {
+            const SegDesc& s = g.segs[sg];
+            return Operands{g.A, g.B, s.a_m, s.a_k, s.b_n, s.b_k, s.K, g.how_a, g.how_b};
+        }
+        return Operands{g.A, g.B, g.a_m, g.a_k, g.b_n, g.b_k, g.K, g.how_a, g.how_b};
+    }
+    __device__ __forceinline__ Target target(const Tile& t) const
+    {
+        return Target{t.g->C, t.g->c_m, t.g->c_n, t.g->alpha, t.g->beta};
+    }
+    __device__ __forceinline__ double* partial() const { return w; }
+};
+
 // calls f with the fragment counts as constants: an MMA under a run-time
 // condition is predicated, and the pipe takes as long for one that is off
 template <int MF, int NF, typename F>
@@ -591,9 +740,11 @@ __device__ __forceinline__ bool dn_fragments(int ni, int nj, F&& f)
 // part p ^ q and a sign. N, K and the scatter vectors stay in complex units in
 // the arguments; M x 2N tiles of 16 real k (8 complex) are what the tile loop
 // sees.
-template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS, int AMODE, int BMODE, bool CPLX>
-__global__ void __launch_bounds__(dn_threads(TEAMS), 1)
-gemm_f64_dense_kernel(const GemmF64Args p)
+//
+// Work: the source of runs, tiles and operands (DenseWork, GroupWork).
+template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS, int AMODE, int BMODE, bool CPLX,
+          typename Work>
+__device__ __forceinline__ void dn_body(const Work& work)
 {
     static_assert(WGM*WGN == DN_CONSUMERS, "consumer warps");
     static_assert(STAGES % TEAMS == 0 && LAG*TEAMS < STAGES, "ring");
@@ -626,8 +777,6 @@ gemm_f64_dense_kernel(const GemmF64Args p)
         // two teams take the stages in turn
         const int team = warp/DN_PRODUCERS;
         int turn = 0;
-        // complex: the gather directions
-        const bool pair_a = CPLX ? p.amode == 0 : p.pair_a != 0, pair_b = CPLX ? p.bmode == 0 : p.pair_b != 0;
         bool ok = true;
         bool wrapped = false;                         // the first round of stages starts empty
         // A warp publishes a stage LAG stages after it issued it, when its copies
@@ -637,18 +786,25 @@ gemm_f64_dense_kernel(const GemmF64Args p)
         // per stage; a longer one only delays a run's first stage.
         int lag = 0;
         uint32_t pub = team;                          // the team's next stage to publish
-        for (unsigned r = 0; ok && run_at(p, blockIdx.x, r, run); r++)
+        for (unsigned r = 0; ok && work.run(r, run); r++)
         {
-            const TileAt t = tile_at<BM, BN>(p, run.tile);
+            const typename Work::Tile t = work.tile(run);
             constexpr int KS = CPLX ? BK/2 : BK;               // k of the scatter vectors per stage
-            typename std::conditional<CPLX, GatherZ<BM>, Gather<BM, AMODE>>::type ga;
-            typename std::conditional<CPLX, GatherZ<BN/2>, Gather<BN, BMODE>>::type gb;
+            constexpr int ES = CPLX ? 2 : 1;                   // doubles per element
+            int base = 0;                                      // first k step of the segment
+            for (int sg = 0; ok && sg < work.segments(t); sg++)
+            {
+            const Operands o = work.operands(t, sg);
+            const int steps = (int)((o.K + KS - 1)/KS), lo = max(run.s0, base), hi = min(run.s1, base + steps);
+            if (lo < hi)
+            {
+            typename GatherOf<BM, AMODE, CPLX>::type ga;
+            typename GatherOf<CPLX ? BN/2 : BN, BMODE, CPLX>::type gb;
             ga.sro = sro + team*(BM + BN);
             gb.sro = ga.sro + BM;
-            constexpr int ES = CPLX ? 2 : 1;                   // doubles per element
-            const i64 k_begin = (i64)run.s0*KS, k_end = min(p.K, (i64)run.s1*KS);
-            ga.start(p.A + ES*p.a_l[t.l], p.a_m, p.a_k, t.m0, t.mrem, pair_a);
-            gb.start(p.B + ES*p.b_l[t.l], p.b_n, p.b_k, t.n0/ES, t.nrem/ES, pair_b);
+            const i64 k_begin = (i64)(lo - base)*KS, k_end = min(o.K, (i64)(hi - base)*KS);
+            ga.start(o.A, o.a_m, o.a_k, t.m0, t.mrem, o.how_a);
+            gb.start(o.B, o.b_n, o.b_k, t.n0/ES, t.nrem/ES, o.how_b);
             ga.fetch(k_begin, k_end);
             gb.fetch(k_begin, k_end);
             int u = 0;
@@ -670,8 +826,8 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                     }
                     const int kvalid = (int)min((i64)KS, k_end - k0);
                     double* As = smem + st*STAGE;
-                    ga.stage(As, u, kvalid, pair_a);
-                    gb.stage(As + BK*BM, u, kvalid, pair_b);
+                    ga.stage(As, u, kvalid, o.how_a);
+                    gb.stage(As + BK*BM, u, kvalid, o.how_b);
                     cp_async_commit();
                     if (lag < LAG) lag++;
                     else
@@ -685,6 +841,9 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                 if (TEAMS > 1) turn ^= 1;
                 u = (u + 1) & 3;
                 if (++st == STAGES) { st = 0; phase ^= 1; wrapped = true; }
+            }
+            }
+            base += steps;
             }
         }
         // the last stages (also after a wait that gave up: the copies land before
@@ -709,12 +868,13 @@ gemm_f64_dense_kernel(const GemmF64Args p)
     if (CPLX)
     {
         const bool col_im = fr & 1, k_im = fc & 1;
+        const GemmF64Args& p = work.args();
         const bool neg = k_im ? (col_im ? p.conj_a != 0 : (p.conj_a != 0) == (p.conj_b != 0)) : col_im && p.conj_b;
         sign = neg ? 0x80000000u : 0u;
     }
-    for (unsigned r = 0; run_at(p, blockIdx.x, r, run); r++)
+    for (unsigned r = 0; work.run(r, run); r++)
     {
-        TileAt t = tile_at<BM, BN>(p, run.tile);
+        typename Work::Tile t = work.tile(run);
         // fragments of this warp inside the GEMM: 16-row fragment i*WGM + wm, 8-column fragment j*WGN + wn
         const int ni = min(MF, max(0, ((t.mrem + 15)/16 - wm + WGM - 1)/WGM));
         const int nj = min(NF, max(0, ((t.nrem + 7)/8 - wn + WGN - 1)/WGN));
@@ -748,13 +908,13 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                                 if (CPLX)
                                     bf[j][q] = flip(Bs[tile_pos<BN/2, 1>((j*WGN + wn)*4 + (fr >> 1),
                                                                          (kk + fc + 4*q) ^ (fr & 1))], sign);
-                                else bf[j][q] = Bs[tile_pos<BN, BMODE>((j*WGN + wn)*8 + fr, kk + fc + 4*q)];
+                                else bf[j][q] = Bs[tile_pos<BN, BMODE != 0>((j*WGN + wn)*8 + fr, kk + fc + 4*q)];
                             }
                         #pragma unroll
                         for (int i = 0; i < NI; i++)
                             #pragma unroll
                             for (int q = 0; q < 4; q++)
-                                af[i][q] = As[tile_pos<BM, AMODE>((i*WGM + wm)*16 + fr + 8*(q & 1),
+                                af[i][q] = As[tile_pos<BM, AMODE != 0>((i*WGM + wm)*16 + fr + 8*(q & 1),
                                                                   kk + fc + 4*(q >> 1))];
                         if (kk + 8 == BK)
                         {
@@ -777,12 +937,12 @@ gemm_f64_dense_kernel(const GemmF64Args p)
 
         // the run and its tile again (not kept over the loop above)
         asm volatile("" : "+r"(r));
-        run_at(p, blockIdx.x, r, run);
-        t = tile_at<BM, BN>(p, run.tile);
+        work.run(r, run);
+        t = work.tile(run);
         if (run.slot >= 0)
         {
             // this run's sums, thread by thread, for gemm_f64_fixup
-            double* w = p.partial + ((i64)blockIdx.x*2 + run.slot)*(BM*BN) + (threadIdx.x - TEAMS*DN_PT);
+            double* w = work.partial() + ((i64)blockIdx.x*2 + run.slot)*(BM*BN) + (threadIdx.x - TEAMS*DN_PT);
             #pragma unroll
             for (int i = 0; i < MF; i++)
                 #pragma unroll
@@ -794,8 +954,9 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                     }
             continue;
         }
-        double* C = p.C + (CPLX ? 2 : 1)*p.c_l[t.l];
-        const double alpha = p.alpha, beta = p.beta;
+        const Target c = work.target(t);
+        double* C = c.C;
+        const double alpha = c.alpha, beta = c.beta;
         #pragma unroll
         for (int j = 0; j < NF; j++)
         {
@@ -803,7 +964,7 @@ gemm_f64_dense_kernel(const GemmF64Args p)
             if (n >= t.nrem) continue;
             if (CPLX)
             {
-                double* C0 = C + 2*__ldg(p.c_n + (t.n0 + n)/2);
+                double* C0 = C + 2*__ldg(c.c_n + (t.n0 + n)/2);
                 #pragma unroll
                 for (int i = 0; i < MF; i++)
                     #pragma unroll
@@ -811,13 +972,13 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                     {
                         const int m = (i*WGM + wm)*16 + 8*hh + fr;
                         if (m < t.mrem)
-                            update_z(p, C0 + 2*__ldg(p.c_m + t.m0 + m), acc[i][j][2*hh], acc[i][j][2*hh + 1]);
+                            update_z(work.args(), C0 + 2*__ldg(c.c_m + t.m0 + m), acc[i][j][2*hh], acc[i][j][2*hh + 1]);
                     }
                 continue;
             }
             const bool two = n + 1 < t.nrem;
-            double* C0 = C + __ldg(p.c_n + t.n0 + n);
-            double* C1 = C + (two ? __ldg(p.c_n + t.n0 + n + 1) : 0);
+            double* C0 = C + __ldg(c.c_n + t.n0 + n);
+            double* C1 = C + (two ? __ldg(c.c_n + t.n0 + n + 1) : 0);
             #pragma unroll
             for (int i = 0; i < MF; i++)
                 #pragma unroll
@@ -825,12 +986,61 @@ gemm_f64_dense_kernel(const GemmF64Args p)
                 {
                     const int m = (i*WGM + wm)*16 + 8*hh + fr;
                     if (m >= t.mrem) continue;
-                    const i64 ro = __ldg(p.c_m + t.m0 + m);
+                    const i64 ro = __ldg(c.c_m + t.m0 + m);
                     const double v0 = alpha*acc[i][j][2*hh], v1 = alpha*acc[i][j][2*hh + 1];
                     C0[ro] = beta == 0.0 ? v0 : v0 + beta*C0[ro];
                     if (two) C1[ro] = beta == 0.0 ? v1 : v1 + beta*C1[ro];
                 }
         }
+    }
+}
+
+template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS, int AMODE, int BMODE, bool CPLX>
+__global__ void __launch_bounds__(dn_threads(TEAMS), 1)
+gemm_f64_dense_kernel(const GemmF64Args p)
+{
+    const DenseWork<WGM*MF*16, WGN*NF*8, CPLX> work{p};
+    dn_body<WGM, WGN, MF, NF, STAGES, LAG, TEAMS, AMODE, BMODE, CPLX>(work);
+}
+
+// the GEMMs of a grouped plan, 128 x 128 tiles (GroupWork). AMODE, BMODE: the
+// gather directions where all groups share them, else 2 (chosen per group, one
+// stage layout for both, single elements along the rows)
+constexpr int GD_BM = 128, GD_BN = 128;
+template <int AMODE, int BMODE>
+__global__ void __launch_bounds__(dn_threads(1), 1)
+gemm_f64_group_dense_kernel(const GroupDesc* __restrict__ groups, const GroupTile* __restrict__ tiles,
+                            const GroupStart* __restrict__ start, double* __restrict__ partial)
+{
+    const GroupWork<GD_BM, GD_BN> work{groups, tiles, start, partial};
+    dn_body<2, 4, 4, 4, 6, 1, 1, AMODE, BMODE, false>(work);
+}
+
+// sums the runs of a cut tile of a grouped plan in CTA order; block (cut tile,
+// fragment), thread t the elements of consumer thread t
+__global__ void __launch_bounds__(DN_CT)
+gemm_f64_group_fixup(const GroupDesc* __restrict__ groups, const GroupTile* __restrict__ tiles,
+                     const GroupCut* __restrict__ cuts, const double* __restrict__ partial)
+{
+    constexpr int NF = 4, WGM = 2, WGN = 4, SLOT = GD_BM*GD_BN;
+    const GroupCut x = cuts[blockIdx.x];
+    const GroupTile tl = tiles[x.tile];
+    const GroupDesc& g = groups[tl.g];
+    const int lane = threadIdx.x & 31, e = blockIdx.y, j = e % NF, i = e/NF;
+    int wm, wn;
+    warp_at<WGN>(threadIdx.x >> 5, wm, wn);
+    #pragma unroll
+    for (int q = 0; q < 4; q++)
+    {
+        const i64 m = (i64)tl.tm*GD_BM + (i*WGM + wm)*16 + 8*(q >> 1) + (lane >> 2);
+        const i64 n = (i64)tl.tn*GD_BN + (j*WGN + wn)*8 + 2*(lane & 3) + (q & 1);
+        if (m >= g.M || n >= g.N) continue;
+        const i64 at = (i64)(4*e + q)*DN_CT + threadIdx.x;
+        double s = partial[((i64)x.cta*2 + x.slot)*SLOT + at];
+        for (int c = 1; c < x.count; c++) s += partial[(i64)(x.cta + c)*2*SLOT + at];
+        double* dst = g.C + __ldg(g.c_m + m) + __ldg(g.c_n + n);
+        const double v = g.alpha*s;
+        *dst = g.beta == 0.0 ? v : v + g.beta*(*dst);
     }
 }
 
@@ -1084,6 +1294,95 @@ void gemm_f64_dense_launch(const GemmF64Args& a, cudaStream_t stream)
     if (a.tile == 0) Tile128::launch(a, stream);
     else if (a.tile == 1) Tile64::launch(a, stream);
     else TileTall::launch(a, stream);
+}
+
+void gemm_f64_group_dense_tile(int& bm, int& bn) { bm = GD_BM; bn = GD_BN; }
+
+size_t gemm_f64_group_dense_bytes(int ctas) { return (size_t)ctas*2*GD_BM*GD_BN*sizeof(double); }
+
+void gemm_f64_group_dense_plan(const std::vector<GroupTile>& tiles, const std::vector<GroupExtents>& groups, int sms,
+                               std::vector<GroupStart>& start, std::vector<GroupCut>& cuts)
+{
+    constexpr double kRun = 2500;                     // a tile's C update and operand tables
+    std::vector<double> cyc(tiles.size());            // per k step
+    double total = 0;
+    for (size_t t = 0; t < tiles.size(); t++)
+    {
+        const GroupExtents& g = groups[tiles[t].g];
+        const int m = (int)std::min<i64>(GD_BM, g.M - (i64)tiles[t].tm*GD_BM);
+        const int n = (int)std::min<i64>(GD_BN, g.N - (i64)tiles[t].tn*GD_BN);
+        cyc[t] = step_cycles<Tile128>(m, n);
+        total += cyc[t]*g.nst + kRun;
+    }
+    // few CTAs where the work is small: no run below 3000 cycles
+    const int ctas = (int)std::max(1.0, std::min((double)sms, total/3000.0));
+    start.assign(1, GroupStart{0, 0});
+    cuts.clear();
+    double at = 0;                                    // cost before tile t
+    size_t t = 0;
+    for (int c = 1; c < ctas; c++)
+    {
+        const double want = total*c/ctas;
+        while (t < tiles.size() && at + cyc[t]*groups[tiles[t].g].nst + kRun <= want)
+        {
+            at += cyc[t]*groups[tiles[t].g].nst + kRun;
+            t++;
+        }
+        GroupStart s{(int)t, 0};
+        if (t < tiles.size())
+        {
+            // a boundary inside a tile, at a whole step; close to an end it moves there
+            const int nst = groups[tiles[t].g].nst;
+            int step = (int)std::lround((want - at)/cyc[t]);
+            if (step < 2) step = 0;
+            if (step > nst - 2) { s.tile = (int)t + 1; step = 0; }
+            s.step = step;
+        }
+        const GroupStart& last = start.back();
+        if (s.tile < last.tile || (s.tile == last.tile && s.step < last.step)) s = last;
+        start.push_back(s);
+    }
+    start.push_back(GroupStart{(int)tiles.size(), 0});
+    // CTAs without work are dropped, so that a cut tile's runs are consecutive CTAs'
+    std::vector<GroupStart> kept(1, start[0]);
+    for (size_t c = 1; c < start.size(); c++)
+        if (start[c].tile != kept.back().tile || start[c].step != kept.back().step) kept.push_back(start[c]);
+    start.swap(kept);
+    // a tile is cut where a boundary falls inside it: its runs are the last of the
+    // CTA before (slot 0 if that is also that CTA's first) and the first of the others
+    for (size_t c = 1; c + 1 < start.size(); c++)
+    {
+        if (start[c].step == 0) continue;
+        if (!cuts.empty() && cuts.back().tile == start[c].tile) { cuts.back().count++; continue; }
+        cuts.push_back(GroupCut{start[c].tile, (int)c - 1, 2, start[c - 1].tile == start[c].tile ? 0 : 1});
+    }
+}
+
+void gemm_f64_group_dense_launch(const GroupDesc* d_groups, const GroupTile* d_tiles, const GroupStart* d_start, int ctas,
+                                 const GroupCut* d_cuts, int ncuts, double* partial, int modes, cudaStream_t s)
+{
+    if (ctas <= 0) return;
+    constexpr size_t bytes = dn_smem<2, 4, 4, 4, 6, 1>();
+    auto go = [&](auto kern)
+    {
+        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        TimedLaunch t("gemm_f64_group_dense_kernel", s);
+        kern<<<(unsigned)ctas, dn_threads(1), bytes, s>>>(d_groups, d_tiles, d_start, partial);
+        check_launch("gemm_f64_group_dense_kernel");
+    };
+    switch (modes)
+    {
+        case 0: go(gemm_f64_group_dense_kernel<0, 0>); break;
+        case 1: go(gemm_f64_group_dense_kernel<0, 1>); break;
+        case 2: go(gemm_f64_group_dense_kernel<1, 0>); break;
+        case 3: go(gemm_f64_group_dense_kernel<1, 1>); break;
+        default: go(gemm_f64_group_dense_kernel<2, 2>);
+    }
+    if (ncuts > 0)
+    {
+        gemm_f64_group_fixup<<<dim3((unsigned)ncuts, 16), DN_CT, 0, s>>>(d_groups, d_tiles, d_cuts, partial);
+        check_launch("gemm_f64_group_fixup");
+    }
 }
 
 int gemm_f64_dense_error_flag()

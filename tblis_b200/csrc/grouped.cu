@@ -7,6 +7,7 @@
 // scratch buffer; the fastest is cached under the histogram and reused by
 // every plan with the same histogram.
 #include "grouped.hpp"
+#include "mult.hpp"
 
 #include <algorithm>
 #include <atomic>
@@ -172,11 +173,12 @@ void GroupedPlan::finalize(cudaStream_t st)
     {
         const bool ws = gemm_f64_is_ws_variant(v);
         int bm = 0, bn = 0;
-        if (!ws) gemm_f64_variant_tile(v, bm, bn);
+        if (!ws && !gemm_f64_is_dense_variant(v)) gemm_f64_variant_tile(v, bm, bn);
         i64 t = 0;
         for (auto& g : groups)
         {
             if (ws) gemm_f64_ws_tile(g.ws_shape, bm, bn);
+            else if (gemm_f64_is_dense_variant(v)) gemm_f64_group_dense_tile(bm, bn);
             tile_begin[v - 1].push_back(t);
             t += ((g.M + bm - 1)/bm)*((g.N + bn - 1)/bn);
         }
@@ -224,6 +226,56 @@ void GroupedPlan::finalize(cudaStream_t st)
                                cudaMemcpyHostToDevice));
         }
     }
+    // dense path: the tiles of the groups that have k steps, dealt to the CTAs
+    {
+        int bm, bn;
+        gemm_f64_group_dense_tile(bm, bn);
+        std::vector<GroupTile> tiles;
+        std::vector<GroupExtents> ext;
+        for (size_t gi = 0; gi < groups.size(); gi++)
+        {
+            const int m = 2*groups[gi].amode + groups[gi].bmode;
+            gmodes = gi == 0 || m == gmodes ? m : 4;
+            if (gmodes == 4) break;
+        }
+        for (size_t gi = 0; gi < groups.size(); gi++)
+        {
+            GroupTables& g = groups[gi];
+            ext.push_back({g.M, g.N, g.nst});
+            const ivec &am = g.segs.empty() ? g.a_m : g.segs[0].a_m, &ak = g.segs.empty() ? g.a_k : g.segs[0].a_k;
+            const ivec &bk = g.segs.empty() ? g.b_k : g.segs[0].b_k, &bn_ = g.segs.empty() ? g.b_n : g.segs[0].b_n;
+            // pairs of neighbours along the gathered direction, or single elements
+            auto how = [&](int mode, const ivec& rows, const ivec& k)
+            {
+                if (mode == 0 && gmodes == 4) return 2;
+                const ivec &along = mode == 0 ? rows : k, &across = mode == 0 ? k : rows;
+                return (int)pairs_along(along.data(), (i64)along.size(), across.data(), (i64)across.size());
+            };
+            g.how_a = how(g.amode, am, ak);
+            g.how_b = how(g.bmode, bn_, bk);
+            if (g.nst == 0) continue;
+            for (i64 tm = 0; tm*bm < g.M; tm++)
+                for (i64 tn = 0; tn*bn < g.N; tn++) tiles.push_back({(int)gi, (int)tm, (int)tn});
+        }
+        TB_CHECK(tiles.size() < (1ull << 31), TB_ERR_SIZE, "too many tiles");
+        if (!tiles.empty())
+        {
+            std::vector<GroupStart> start;
+            std::vector<GroupCut> cuts;
+            gemm_f64_group_dense_plan(tiles, ext, device_sm_count(), start, cuts);
+            gctas = (int)start.size() - 1;
+            ngcuts = (int)cuts.size();
+            auto up = [](auto*& dst, const auto& v)
+            {
+                if (v.empty()) return;
+                TB_CUDA(cudaMalloc(&dst, v.size()*sizeof(v[0])));
+                TB_CUDA(cudaMemcpy(dst, v.data(), v.size()*sizeof(v[0]), cudaMemcpyHostToDevice));
+            };
+            up(d_gtiles, tiles);
+            up(d_gstart, start);
+            up(d_gcuts, cuts);
+        }
+    }
     TB_CUDA(cudaMalloc(&d_counter, sizeof(unsigned long long)));
     if (!groups.empty())
     {
@@ -236,6 +288,7 @@ void GroupedPlan::finalize(cudaStream_t st)
 }
 
 static void release_pack(GroupedPlan& plan);
+static void release_gpart(GroupedPlan& plan);
 
 GroupedPlan::~GroupedPlan()
 {
@@ -248,7 +301,11 @@ GroupedPlan::~GroupedPlan()
     if (d_counter) cudaFree(d_counter);
     if (h_descs) cudaFreeHost(h_descs);
     if (d_pack_items) cudaFree(d_pack_items);
+    if (d_gtiles) cudaFree(d_gtiles);
+    if (d_gstart) cudaFree(d_gstart);
+    if (d_gcuts) cudaFree(d_gcuts);
     release_pack(*this);
+    release_gpart(*this);
 }
 
 GroupedPlanCache& grouped_plan_cache()
@@ -299,6 +356,10 @@ static void fill_descs(GroupedPlan& plan, GroupDesc* out, const double* const* p
         d.nst = g.nst;
         d.pa = g.pa;
         d.pb = g.pb;
+        // pairs need operands at a 16-byte boundary (the gather checks each pair;
+        // without one, single elements are the faster gather)
+        d.how_a = g.how_a == 1 && ((uintptr_t)d.A & 15) ? 0 : g.how_a;
+        d.how_b = g.how_b == 1 && ((uintptr_t)d.B & 15) ? 0 : g.how_b;
     }
 }
 
@@ -352,6 +413,41 @@ static bool ensure_pack(GroupedPlan& plan)
     return true;
 }
 
+static void release_gpart(GroupedPlan& plan)
+{
+    if (!plan.d_gpart) return;
+    cudaFree(plan.d_gpart);
+    plan.d_gpart = nullptr;
+    g_pack_held -= plan.gpart_held;
+    plan.gpart_held = 0;
+}
+
+// the dense path's workspace (two tiles per CTA, 39 MB), allocated on first
+// use and counted with the packed panels; false when it would pass the cap or
+// the device has no room
+static bool ensure_gpart(GroupedPlan& plan)
+{
+    if (plan.d_gpart || plan.ngcuts == 0) return true;
+    if (plan.gpart_failed) return false;
+    const size_t bytes = gemm_f64_group_dense_bytes(plan.gctas);
+    if (g_pack_held.load() + bytes > pack_cap() || cudaMalloc(&plan.d_gpart, bytes) != cudaSuccess)
+    {
+        cudaGetLastError();
+        plan.d_gpart = nullptr;
+        plan.gpart_failed = true;
+        return false;
+    }
+    plan.gpart_held = bytes;
+    g_pack_held += bytes;
+    return true;
+}
+
+// what variant v needs to run; false: not available for this plan
+static bool ensure_variant(GroupedPlan& plan, int v)
+{
+    return gemm_f64_is_ws_variant(v) ? ensure_pack(plan) : gemm_f64_is_dense_variant(v) ? ensure_gpart(plan) : true;
+}
+
 // one run of variant v of the plan on the descriptors descs
 static void launch_variant(GroupedPlan& plan, const GroupDesc* descs, int v, cudaStream_t st)
 {
@@ -364,6 +460,9 @@ static void launch_variant(GroupedPlan& plan, const GroupDesc* descs, int v, cud
         gemm_f64_ws_launch(descs, variant_tile_begin(plan, v), ng, plan.total_tiles[v - 1], plan.d_pack,
                            plan.d_pack + plan.pack_a, st, plan.d_counter);
     }
+    else if (gemm_f64_is_dense_variant(v))
+        gemm_f64_group_dense_launch(descs, plan.d_gtiles, plan.d_gstart, plan.gctas, plan.d_gcuts, plan.ngcuts,
+                                    plan.d_gpart, plan.gmodes, st);
     else
         gemm_f64_grouped_launch(descs, variant_tile_begin(plan, v), ng, plan.total_tiles[v - 1], v, st,
                                 plan.d_counter);
@@ -378,8 +477,7 @@ static int autotune(GroupedPlan& plan, const double* const* ptrs, const double* 
         if (it != g_tuned.end()) return it->second;
     }
     const char* env = getenv("TBLIS_B200_GEMM_VARIANT");
-    if (env && atoi(env) >= 1 && atoi(env) <= gemm_f64_grouped_num_variants() &&
-        (!gemm_f64_is_ws_variant(atoi(env)) || ensure_pack(plan)))
+    if (env && atoi(env) >= 1 && atoi(env) <= gemm_f64_grouped_num_variants() && ensure_variant(plan, atoi(env)))
         return atoi(env);
 
     // scratch C covering the offsets of every group: candidates write there
@@ -398,7 +496,7 @@ static int autotune(GroupedPlan& plan, const double* const* ptrs, const double* 
     float best_ms = 1e30f;
     for (int v = 1; v <= gemm_f64_grouped_num_variants(); v++)
     {
-        if (gemm_f64_is_ws_variant(v) && !ensure_pack(plan)) continue;
+        if (!ensure_variant(plan, v)) continue;
         launch_variant(plan, dd.as<GroupDesc>(), v, st);     // warm-up
         TB_CUDA(cudaEventRecord(e0, st));
         launch_variant(plan, dd.as<GroupDesc>(), v, st);
@@ -412,6 +510,7 @@ static int autotune(GroupedPlan& plan, const double* const* ptrs, const double* 
     cudaEventDestroy(e1);
     // the timed launches are complete (event synchronised): give the room back
     if (!gemm_f64_is_ws_variant(best)) release_pack(plan);
+    if (!gemm_f64_is_dense_variant(best)) release_gpart(plan);
     std::lock_guard<std::mutex> lk(g_tune_mtx);
     g_tuned[plan.histogram] = best;
     return best;
@@ -425,8 +524,8 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
     {
         plan.variant = autotune(plan, ptrs, alphas, betas, st);
         // a variant tuned on another plan of the same shape histogram: the
-        // packed path needs this plan's buffer too
-        if (gemm_f64_is_ws_variant(plan.variant) && !ensure_pack(plan)) plan.variant = 4;
+        // packed and dense paths need this plan's buffers too
+        if (!ensure_variant(plan, plan.variant)) plan.variant = 4;
     }
     const int v = plan.variant;
 
@@ -487,11 +586,12 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
     }
     if (plan.graph)
     {
-        const bool ws = gemm_f64_is_ws_variant(v);
-        TimedLaunch t(ws ? "gemm_f64_pack_kernel+gemm_f64_ws_kernel" : "gemm_f64_grouped_kernel", st);
+        const bool ws = gemm_f64_is_ws_variant(v), dense = gemm_f64_is_dense_variant(v);
+        TimedLaunch t(ws ? "gemm_f64_pack_kernel+gemm_f64_ws_kernel"
+                         : dense ? "gemm_f64_group_dense_kernel" : "gemm_f64_grouped_kernel", st);
         TB_CUDA(cudaGraphLaunch(plan.graph, st));
         count_launch();
-        if (ws) count_launch();             // the pack kernel and the GEMM kernel
+        if (ws || (dense && plan.ngcuts > 0)) count_launch();     // pack and GEMM; GEMM and fixup
     }
     else
     {

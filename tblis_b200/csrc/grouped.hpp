@@ -30,6 +30,7 @@ struct GroupTables
     int a_slot = 0, b_slot = 1, c_slot = 2;   // indices into the run's pointer array
     i64 a_off = 0, b_off = 0, c_off = 0;      // element offsets added to those pointers
     int sidx = 0;                             // index into the run's alpha/beta arrays
+    int how_a = 0, how_b = 0;                 // gather directions of the dense path (finalize)
     int ws_shape = 0;                         // tile shape of the packed path (finalize)
     int nst = 0;                              // k steps over all segments (finalize)
     i64 pa = 0, pb = 0;                       // offsets of the packed A / B panels (finalize)
@@ -70,6 +71,16 @@ struct GroupedPlan
     double* d_pack = nullptr;
     size_t pack_held = 0;                     // bytes of d_pack counted against the cap
     bool pack_failed = false;
+    // dense path: its tiles, their division over CTAs, and the partial sums'
+    // workspace (allocated on first use)
+    GroupTile* d_gtiles = nullptr;
+    GroupStart* d_gstart = nullptr;
+    GroupCut* d_gcuts = nullptr;
+    int gctas = 0, ngcuts = 0;
+    int gmodes = 4;                           // gather directions shared by all groups (2*amode + bmode), or 4
+    double* d_gpart = nullptr;
+    size_t gpart_held = 0;
+    bool gpart_failed = false;
     std::string histogram;
     std::vector<std::shared_ptr<GroupedPlan>> parts;   // plans whose groups this one merges (kept alive)
 

@@ -429,6 +429,14 @@ static void pair_stats(const i64* t, i64 n, double& adj, double& even)
     even = n > 0 ? (double)e/(double)n : 0.0;
 }
 
+bool pairs_along(const i64* along, i64 n, const i64* across, i64 m)
+{
+    double adj, even, adj2, even2;
+    pair_stats(along, n, adj, even);
+    pair_stats(across, m, adj2, even2);
+    return adj >= 0.9 && even2 >= 0.9;
+}
+
 void gemm_pair_modes(const GemmView& v, const i64* a_m, const i64* a_k, const i64* b_n, const i64* b_k,
                      const i64* a_l, const i64* b_l, bool a_pairs[2], bool b_pairs[2])
 {

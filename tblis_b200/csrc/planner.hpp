@@ -80,6 +80,10 @@ struct GemmTables
     ~GemmTables();
 };
 
+// whether nearly all pairs of neighbours of `along` are adjacent in memory at an
+// even offset, and nearly all offsets of `across` even
+bool pairs_along(const i64* along, i64 n, const i64* across, i64 m);
+
 // Decides, from a view's host scatter vectors, whether the FP64 kernel may
 // gather A and B in 16-byte pairs in each gather mode (GemmTables::a_pairs).
 void gemm_pair_modes(const GemmView& v, const i64* a_m, const i64* a_k, const i64* b_n, const i64* b_k,
