@@ -26,6 +26,9 @@ struct GemmF64Args
     // elements, every element 16-byte aligned)
     int cplx, conj_a, conj_b, conj_c;
     double alpha_im, beta_im;
+    // dense kernel: run only if the word at gate is above gate_above (null: always)
+    const unsigned* gate;
+    unsigned gate_above;
     int pair_a, pair_b;      // gather the operand's contiguous dimension in pairs (16-byte copies)
     // set by gemm_f64_dense_plan: k steps of a tile, tiles done whole, tiles
     // whose k steps are cut into equal runs over sk_ctas CTAs, CTAs, workspace

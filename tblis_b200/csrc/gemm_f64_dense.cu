@@ -999,6 +999,7 @@ template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS, int 
 __global__ void __launch_bounds__(dn_threads(TEAMS), 1)
 gemm_f64_dense_kernel(const GemmF64Args p)
 {
+    if (p.gate && *p.gate <= p.gate_above) return;
     const DenseWork<WGM*MF*16, WGN*NF*8, CPLX> work{p};
     dn_body<WGM, WGN, MF, NF, STAGES, LAG, TEAMS, AMODE, BMODE, CPLX>(work);
 }
@@ -1054,6 +1055,7 @@ __global__ void __launch_bounds__(DN_CT*GROUPS)
 gemm_f64_fixup(const GemmF64Args p)
 {
     constexpr int BM = WGM*MF*16, BN = WGN*NF*8;
+    if (p.gate && *p.gate <= p.gate_above) return;
     __shared__ double sums[GROUPS][2][DN_CT];
     const int tc = threadIdx.x % DN_CT, grp = threadIdx.x/DN_CT;
     const int lane = tc & 31;

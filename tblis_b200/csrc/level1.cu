@@ -117,8 +117,10 @@ __global__ void __launch_bounds__(L1_THREADS) k_unary(T* A, const Strided s, T v
 // ---- element-type conversion at equal offsets -------------------------------------
 
 template <typename S, typename D>
-__global__ void __launch_bounds__(L1_THREADS) k_convert(const S* __restrict__ src, D* __restrict__ dst, const Strided s)
+__global__ void __launch_bounds__(L1_THREADS) k_convert(const S* __restrict__ src, D* __restrict__ dst, const Strided s,
+                                                        const unsigned* gate, unsigned gate_above)
 {
+    if (gate && *gate <= gate_above) return;
     const i64 n0 = s.ndim ? s.len[0] : 1;
     const i64 st0 = s.ndim ? s.stride[0] : 0;
     i64 rows = 1;
@@ -134,6 +136,28 @@ __global__ void __launch_bounds__(L1_THREADS) k_convert(const S* __restrict__ sr
         const i64 ro = row_offset(s.len, s.stride, s.ndim, r);
         const i64 i0 = c*SEG, i1 = min(n0, i0 + SEG);
         for (i64 i = i0 + lane; i < i1; i += 32) dst[ro + i*st0] = (D)src[ro + i*st0];
+    }
+}
+
+// dst = (float)(src + beta*dst) at equal offsets
+__global__ void __launch_bounds__(L1_THREADS) k_convert_add(const double* __restrict__ src, float* __restrict__ dst,
+                                                            const Strided s, double beta)
+{
+    const i64 n0 = s.ndim ? s.len[0] : 1;
+    const i64 st0 = s.ndim ? s.stride[0] : 0;
+    i64 rows = 1;
+    for (int d = 1; d < s.ndim; d++) rows *= s.len[d];
+    const i64 nchunk = (n0 + SEG - 1)/SEG;
+    const i64 nseg = rows*nchunk;
+    const int lane = threadIdx.x & 31;
+    const i64 warp0 = (blockIdx.x*(i64)blockDim.x + threadIdx.x) >> 5;
+    const i64 nwarps = ((i64)gridDim.x*blockDim.x) >> 5;
+    for (i64 sg = warp0; sg < nseg; sg += nwarps)
+    {
+        const i64 r = rows == 1 ? 0 : sg / nchunk, c = sg - r*nchunk;
+        const i64 ro = row_offset(s.len, s.stride, s.ndim, r);
+        const i64 i0 = c*SEG, i1 = min(n0, i0 + SEG);
+        for (i64 i = i0 + lane; i < i1; i += 32) dst[ro + i*st0] = (float)(src[ro + i*st0] + beta*(double)dst[ro + i*st0]);
     }
 }
 
@@ -588,19 +612,29 @@ template <typename T> void l1_shift(T* A, const Strided& s, T shift, T alpha, cu
 }
 
 template <typename S, typename D>
-void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st)
+void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st, const unsigned* gate, unsigned gate_above)
 {
     i64 total = total_of(s);
     if (total == 0) return;
     i64 n0 = s.ndim ? s.len[0] : 1;
     i64 segs = (total/n0)*((n0 + SEG - 1)/SEG);
     int grid = l1_grid(segs, L1_THREADS/32);
-    k_convert<S, D><<<grid, L1_THREADS, 0, st>>>(src, dst, s);
+    k_convert<S, D><<<grid, L1_THREADS, 0, st>>>(src, dst, s, gate, gate_above);
     check_launch("k_convert");
 }
 
-template void l1_convert<float, double>(const float*, double*, const Strided&, cudaStream_t);
-template void l1_convert<double, float>(const double*, float*, const Strided&, cudaStream_t);
+void l1_convert_add(const double* src, float* dst, const Strided& s, double beta, cudaStream_t st)
+{
+    i64 total = total_of(s);
+    if (total == 0) return;
+    i64 n0 = s.ndim ? s.len[0] : 1;
+    i64 segs = (total/n0)*((n0 + SEG - 1)/SEG);
+    k_convert_add<<<l1_grid(segs, L1_THREADS/32), L1_THREADS, 0, st>>>(src, dst, s, beta);
+    check_launch("k_convert_add");
+}
+
+template void l1_convert<float, double>(const float*, double*, const Strided&, cudaStream_t, const unsigned*, unsigned);
+template void l1_convert<double, float>(const double*, float*, const Strided&, cudaStream_t, const unsigned*, unsigned);
 
 // rows of same-order adds that a warp walks on its own
 constexpr i64 kLongRow = 128;

@@ -45,9 +45,14 @@ void l1_dot(const T* A, const T* B, const Strided2& ab, T* d_result, cudaStream_
             bool conj_b = false);
 
 // dst[o] = (D)src[o] for every offset o of the strided space (widening and
-// rounding copies between float and double storage of the same layout)
+// rounding copies between float and double storage of the same layout); with a
+// gate, only if the word there is above gate_above
 template <typename S, typename D>
-void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st);
+void l1_convert(const S* src, D* dst, const Strided& s, cudaStream_t st, const unsigned* gate = nullptr,
+                unsigned gate_above = 0);
+
+// dst[o] = (float)(src[o] + beta*dst[o])
+void l1_convert_add(const double* src, float* dst, const Strided& s, double beta, cudaStream_t st);
 
 // The same over many pieces in one launch (the stored blocks of a block-sparse
 // tensor): piece i is the index space ab[i] at offsets offa[i], offb[i]

@@ -246,7 +246,8 @@ static void dense_gemm(GemmF64Args& a, cudaStream_t st)
 // one contraction on device data (a GEMM view of device-resident operands)
 static void contract_device(const GemmView& v, const double* A, const double* B, double* C, double alpha,
                             double beta, int method, double tol, int slices, cudaStream_t st,
-                            int& used_slices, double& est_error, int* used_method = nullptr)
+                            int& used_slices, double& est_error, int* used_method = nullptr,
+                            const unsigned* gate = nullptr, unsigned gate_above = 0)
 {
     if (used_method) *used_method = method;
     if (method >= 2)
@@ -277,6 +278,7 @@ static void contract_device(const GemmView& v, const double* A, const double* B,
     a.M = v.m; a.N = v.n; a.K = v.k; a.L = v.l;
     a.alpha = alpha; a.beta = beta;
     a.amode = tab->amode; a.bmode = tab->bmode;
+    a.gate = gate; a.gate_above = gate_above;
     dense_gemm(a, st);
     used_slices = 0;
     est_error = 1.1e-16*std::sqrt((double)v.k);
@@ -535,6 +537,20 @@ static void mult_widened(const tblis_config* cfg,
     stage(sa, A, true, st, cx ? 8 : 4);
     stage(sb, B, true, st, cx ? 8 : 4);
 
+    // a large float contraction on the FP64 path takes the INT8 cores, verified
+    // (ozaki_verified): the FP64 pipe has a tenth of their rate
+    GemmView v;
+    bool moduli = false;
+    if (!cx && (opts && opts->method ? opts->method : (cfg ? cfg->method : 1)) == 1 &&
+        (double)A->scalar.data.s*(double)B->scalar.data.s != 0.0)
+    {
+        v = gemm_view(mult_groups(A, idx_A, B, idx_B, C, idx_C));
+        // (every element of C is written: none of its labels repeats)
+        i64 elements = 1;
+        for (unsigned d = 0; d < C->ndim; d++) elements *= C->len[d];
+        moduli = v.k != 0 && v.m*v.n*v.l == elements && elements != 0 && ozaki_verified_pays(v);
+    }
+
     const tblis_tensor* src[3] = {A, B, C};
     StagedOp* sto[3] = {&sa, &sb, &sc};
     tblis_tensor wide[3];
@@ -555,11 +571,45 @@ static void mult_widened(const tblis_config* cfg,
         wbuf[t] = dbuf((size_t)rv[t]->count()*sizeof(double), st);
         double* base = wbuf[t].as<double>() - rv[t]->lo;          // element 0 of the widened tensor
         wide[t].data = base;
-        if (t < 2 || read_c)
+        if (!moduli && (t < 2 || read_c))
             l1_convert<float, double>(static_cast<const float*>(sto[t]->dptr), base, rv[t]->s, st);
     }
-    mult_dispatch(cfg, &wide[0], idx_A, &wide[1], idx_B, &wide[2], idx_C, opts, report);
-    if (C->data && rv[2]->s.len[0] != 0)
+    if (moduli)
+    {
+        const int kernels_before = (int)g_kernel_count.load();
+        const double alpha = wide[0].scalar.data.d*wide[1].scalar.data.d, beta = wide[2].scalar.data.d;
+        const float *a = static_cast<const float*>(sa.dptr), *b = static_cast<const float*>(sb.dptr);
+        double *wa = static_cast<double*>(wide[0].data), *wb = static_cast<double*>(wide[1].data);
+        double* c = static_cast<double*>(wide[2].data);
+        dbuf gate;
+        unsigned above = 0;
+        bool done = false;
+        try { ozaki_verified(v, a, b, c, alpha, st, gate, above); done = true; }
+        catch (const error&)
+        {
+            // no room for the residue planes: FP64 does all of it
+            cudaGetLastError();
+        }
+        int used = 0;
+        double est = 0;
+        const unsigned* g = done ? gate.as<unsigned>() : nullptr;
+        l1_convert<float, double>(a, wa, rv[0]->s, st, g, above);
+        l1_convert<float, double>(b, wb, rv[1]->s, st, g, above);
+        contract_device(v, wa, wb, c, alpha, 0.0, 1, 0.0, 0, st, used, est, nullptr, g, above);
+        if (read_c) l1_convert_add(c, static_cast<float*>(sc.dptr), rv[2]->s, beta, st);
+        else l1_convert<double, float>(c, static_cast<float*>(sc.dptr), rv[2]->s, st);
+        if (report)
+        {
+            report->method = 1;
+            report->slices = 0;
+            report->est_error = est;
+            report->m = v.m; report->n = v.n; report->k = v.k; report->l = v.l;
+            report->flops = 2.0*(double)v.m*(double)v.n*(double)v.k*(double)v.l;
+            report->kernels = (int)(g_kernel_count.load() - kernels_before);
+        }
+    }
+    else mult_dispatch(cfg, &wide[0], idx_A, &wide[1], idx_B, &wide[2], idx_C, opts, report);
+    if (!moduli && C->data && rv[2]->s.len[0] != 0)
         l1_convert<double, float>(static_cast<const double*>(wide[2].data), static_cast<float*>(sc.dptr), rv[2]->s,
                                   st);
     unstage(sc, st);

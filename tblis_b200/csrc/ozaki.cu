@@ -467,11 +467,12 @@ ozaki_gemm_kernel(const OzGemmArgs p)
 // view of one operand as rows x k (rows = m for A, n for B)
 struct OzOperand
 {
-    const double* X;
+    const void* X;                 // double, or float values where f32
     const i64 *r_off, *k_off, *l_off;
     i64 R, K, L;
     int rmode;                     // 0: gather along rows (rows contiguous), 1: along k
     i64 r_step, k_step;            // r_off[i] == i*r_step (k alike) for every i, or -1
+    bool f32;
 };
 
 constexpr int ST_THREADS = 256;
@@ -499,6 +500,7 @@ constexpr int ST_UNROLL = 8;     // independent loads in flight per thread
 
 // rows contiguous: a thread per row, k split over blockIdx.y; partial
 // (max exponent, sum of squares) per split
+template <typename E>
 __global__ void __launch_bounds__(ST_THREADS)
 oz_stats_rows(const OzOperand o, int ksplit, int* pexp, double* pss)
 {
@@ -508,7 +510,7 @@ oz_stats_rows(const OzOperand o, int ksplit, int* pexp, double* pss)
     if (r >= o.R) return;
     const i64 kchunk = (o.K + ksplit - 1)/ksplit;
     const i64 k0 = sp*kchunk, k1 = min(o.K, k0 + kchunk);
-    const double* X = o.X + o.l_off[l] + o.r_off[r];
+    const E* X = static_cast<const E*>(o.X) + o.l_off[l] + o.r_off[r];
     unsigned long long mb = 0;
     double ss = 0.0;
     i64 k = k0;
@@ -533,6 +535,7 @@ oz_stats_rows(const OzOperand o, int ksplit, int* pexp, double* pss)
 }
 
 // k contiguous: a warp per row, lanes along k
+template <typename E>
 __global__ void __launch_bounds__(ST_THREADS)
 oz_stats_k(const OzOperand o, int* pexp, double* pss)
 {
@@ -540,7 +543,7 @@ oz_stats_k(const OzOperand o, int* pexp, double* pss)
     const int lane = threadIdx.x & 31;
     const int l = blockIdx.z;
     if (r >= o.R) return;
-    const double* X = o.X + o.l_off[l] + o.r_off[r];
+    const E* X = static_cast<const E*>(o.X) + o.l_off[l] + o.r_off[r];
     unsigned long long mb = 0;
     double ss = 0.0;
     i64 k = lane;
@@ -696,11 +699,12 @@ __device__ __forceinline__ typename PlaneElem<KIND>::T single_elem(double xs)
     else return to_tf32_bits(xs);
 }
 
-__device__ __forceinline__ void sl_cp_async8(double* smem, const double* gmem, bool valid)
+template <typename E>
+__device__ __forceinline__ void sl_cp_async(E* smem, const E* gmem, bool valid)
 {
     const unsigned saddr = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n"
-                 :: "r"(saddr), "l"(gmem), "r"(valid ? 8 : 0) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n"
+                 :: "r"(saddr), "l"(gmem), "n"((int)sizeof(E)), "r"(valid ? (int)sizeof(E) : 0) : "memory");
 }
 
 // geometry of tiled planes: blocks [l][row tile][k step], each holding the S
@@ -712,27 +716,30 @@ struct PlaneGeom
     int S;
 };
 
-constexpr int SL_LD = SL_T + 1;            // padded smem row (doubles)
+constexpr int SL_LD = SL_T + 1;            // padded smem row (elements)
 // 128 registers a thread: more of the 16 elements' FP64 chains in flight (residues
 // with 3 blocks: 2.87 ms for 13 planes of 25600 x 25600 where 2 take 2.81)
 constexpr int SL_BLOCKS_PER_SM = 2;
-constexpr size_t SL_SMEM = 2*SL_T*SL_LD*sizeof(double);
+template <typename E> constexpr size_t sl_smem_bytes() { return 2*SL_T*SL_LD*sizeof(E); }
 
 // writes the S tiled planes (PlaneGeom) of 64x64 tiles of the operand:
 // digit planes, or (SINGLE, S = 1) x' rounded to the plane type. Rows and k
 // beyond the operand, up to whole tiles and k steps, get zeros.
 // Persistent blocks walk the tiles; the gather of the next tile (cp.async,
 // zero-filled outside the operand) runs while the current one is converted.
-template <int S, int KIND, bool SINGLE, bool CRT = false>
+// E: the operand's elements.
+template <int S, int KIND, bool SINGLE, bool CRT = false, typename E = double>
 __global__ void __launch_bounds__(256, SL_BLOCKS_PER_SM)
 oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, unsigned tiles_r, unsigned tiles_k,
-         const CrtConsts cc)
+         const CrtConsts cc, int* inexact)
 {
     using T = typename PlaneElem<KIND>::T;
     constexpr int KE = OZ_BK/(int)sizeof(T);         // elements per k step
     unsigned char* outb = static_cast<unsigned char*>(out_);
     const i64 tile_bytes = (i64)pg.tile_rows*OZ_BK;
-    extern __shared__ double sl_smem[];    // two [SL_T][SL_LD] buffers
+    extern __shared__ double sl_smem_raw[];
+    E* sl_smem = reinterpret_cast<E*>(sl_smem_raw);      // two [SL_T][SL_LD] buffers
+    const E* X = static_cast<const E*>(o.X);
     const unsigned per_l = tiles_r*tiles_k, ntiles = per_l*(unsigned)o.L;   // below 2^31 (host check)
     const int t = threadIdx.x;
 
@@ -755,20 +762,20 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
         const unsigned tr = rem/tiles_k;
         return At{(int)l, (i64)tr*SL_T, (i64)(rem - tr*tiles_k)*SL_T};
     };
-    auto load = [&](const At& w, double* buf) {
+    auto load = [&](const At& w, E* buf) {
         const i64 f = (by_rows ? w.r0 : w.k0) + fixed;
         const i64 v0 = (by_rows ? w.k0 : w.r0) + vary0;
         const bool fok = f < fixed_n;
-        const double* Xf = o.X + o.l_off[w.l] + (fok ? fixed_off[f] : 0);
+        const E* Xf = X + o.l_off[w.l] + (fok ? fixed_off[f] : 0);
         if (vary_step >= 0)
         {
             // a single stride: the addresses need no table reads
-            const double* Xv = Xf + v0*vary_step;
+            const E* Xv = Xf + v0*vary_step;
             #pragma unroll
             for (int j = 0; j < SL_T*SL_T/256; j++)
             {
                 const bool ok = fok && v0 + 4*j < vary_n;
-                sl_cp_async8(buf + s_base + j*s_step, ok ? Xv + 4*j*vary_step : o.X, ok);
+                sl_cp_async(buf + s_base + j*s_step, ok ? Xv + 4*j*vary_step : X, ok);
             }
         }
         else
@@ -778,7 +785,7 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
             {
                 const i64 v = v0 + 4*j;
                 const bool ok = fok && v < vary_n;
-                sl_cp_async8(buf + s_base + j*s_step, ok ? Xf + vary_off[v] : o.X, ok);
+                sl_cp_async(buf + s_base + j*s_step, ok ? Xf + vary_off[v] : X, ok);
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -796,7 +803,7 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
     if (tile < ntiles) { at = where(tile); load(at, sl_smem); }
     for (int it = 0; tile < ntiles; tile += gridDim.x, it++)
     {
-        const double* cur = sl_smem + (it & 1)*SL_T*SL_LD;
+        const E* cur = sl_smem + (it & 1)*SL_T*SL_LD;
         const unsigned nxt = tile + gridDim.x;
         At nat = at;
         if (nxt < ntiles) { nat = where(nxt); load(nat, sl_smem + ((it + 1) & 1)*SL_T*SL_LD); }
@@ -809,7 +816,7 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
         {
             // rows past the operand hold zeros: any exponent serves
             const int e = r < o.R ? e_rows[(i64)at.l*o.R + r] : 0;
-            const double* src = cur + rl*SL_LD + seg;
+            const E* src = cur + rl*SL_LD + seg;
             const i64 rt = r/pg.tile_rows;
             const int rin = (int)(r - rt*pg.tile_rows);
             // slice tile 0 of the block of row tile rt holding element k
@@ -842,6 +849,14 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
                     av[u] = __dsub_rn(y0, SH);
                     av[u + 1] = __dsub_rn(y1, SH);
                     ylo[u/2] = __byte_perm((uint32_t)__double2loint(y0), (uint32_t)__double2loint(y1), 0x0400) & 0x00ff00ffu;
+                }
+                if (inexact)
+                {
+                    // elements that the rounding to an integer changed, per row
+                    int n = 0;
+                    #pragma unroll
+                    for (int u = 0; u < 16; u++) n += __dmul_rn(__dmul_rn(src[u], sc1), sc2) != av[u];
+                    if (n && r < o.R) atomicAdd(inexact + (i64)at.l*o.R + r, n);
                 }
                 const i64 plane_stride = tile_bytes;
                 unsigned char* dst = block(kk);
@@ -932,9 +947,9 @@ oz_slice(const OzOperand o, const int* e_rows, void* out_, const PlaneGeom pg, u
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
-template <int S, int KIND, bool SINGLE, bool CRT = false>
+template <int S, int KIND, bool SINGLE, bool CRT = false, typename E = double>
 void launch_slice(const OzOperand& o, const int* e, void* out, const PlaneGeom& pg, cudaStream_t st,
-                  const CrtConsts* cc = nullptr)
+                  const CrtConsts* cc = nullptr, int* inexact = nullptr)
 {
     // every row of the row tiles (64-row slicing tiles may pass the last
     // one: the kernel stops at it), every k of the k steps
@@ -944,12 +959,13 @@ void launch_slice(const OzOperand& o, const int* e, void* out, const PlaneGeom& 
     if (ntiles == 0) return;
     TB_CHECK(ntiles < ((i64)1 << 31), TB_ERR_SIZE, "Ozaki operand above 2^31 tiles of 64x64");
     const i64 grid = std::min<i64>(ntiles, (i64)device_sm_count()*SL_BLOCKS_PER_SM);
-    TB_CUDA(cudaFuncSetAttribute(oz_slice<S, KIND, SINGLE, CRT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)SL_SMEM));
+    constexpr size_t bytes = sl_smem_bytes<E>();
+    TB_CUDA(cudaFuncSetAttribute(oz_slice<S, KIND, SINGLE, CRT, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)bytes));
     CrtConsts none = {};
     TimedLaunch t("oz_slice", st);
-    oz_slice<S, KIND, SINGLE, CRT><<<(unsigned)grid, 256, SL_SMEM, st>>>(o, e, out, pg, (unsigned)tiles_r,
-                                                                          (unsigned)tiles_k, cc ? *cc : none);
+    oz_slice<S, KIND, SINGLE, CRT, E><<<(unsigned)grid, 256, bytes, st>>>(o, e, out, pg, (unsigned)tiles_r,
+                                                                           (unsigned)tiles_k, cc ? *cc : none, inexact);
     check_launch("oz_slice");
 }
 
@@ -1276,6 +1292,8 @@ __global__ void oz_crt_shifts(const double* ss, i64 n, int P, int* s_out)
     s_out[i] = s;
 }
 
+constexpr int VERIFIED_MODULI = 13;    // P = 50: the most that the digit extraction takes
+
 struct CrtCombineArgs
 {
     const unsigned char* R;        // residues of the chunks, chunk_bytes apart
@@ -1287,7 +1305,53 @@ struct CrtCombineArgs
     i64 M, N, tiles_m, tiles_n;
     double alpha, beta;
     CrtConsts cc;
+    // VERIFY: bounds on what rounding row i of A and column j of B to integers can
+    // change in a product (0: nothing was rounded), and the elements of C left to
+    // be recomputed: their number and, up to cap, their linear indices
+    const double *dA, *dB;
+    unsigned* count;
+    unsigned cap;
+    unsigned long long* list;
 };
+
+// The bounds: with n of row a's integers rounded (by at most 1/2 each), the
+// product changes by at most half the sum of |b| there, 1/2 sqrt(n) ||b||, with
+// ||b|| <= 2^P, and where both were rounded by at most another 1/4 each. A row
+// with an infinity or a NaN: infinite.
+__global__ void oz_inexact_bounds(const int* n, const double* ss, i64 rows, double norm, double* d)
+{
+    const i64 i = blockIdx.x*(i64)blockDim.x + threadIdx.x;
+    if (i >= rows) return;
+    const double k = (double)n[i];
+    d[i] = !(ss[i] <= 1.7e308) ? __longlong_as_double(0x7ff0000000000000ll)
+                               : k > 0.0 ? 0.5*sqrt(k)*norm*(1.0 + 0x1p-20) + 0.25*k : 0.0;
+}
+
+// C elements from the list in FP64, a warp each; nothing when the list ran over.
+// A and B hold floats.
+__global__ void __launch_bounds__(256)
+oz_recompute(const float* A, const float* B, double* C, const i64* a_m, const i64* a_k, const i64* a_l, const i64* b_n,
+             const i64* b_k, const i64* b_l, const i64* c_m, const i64* c_n, const i64* c_l, i64 M, i64 N, i64 K,
+             double alpha, const unsigned* count, unsigned cap, const unsigned long long* list)
+{
+    const unsigned n = *count;
+    if (n > cap) return;
+    const int lane = threadIdx.x & 31;
+    for (unsigned e = (blockIdx.x*blockDim.x + threadIdx.x) >> 5; e < n; e += (gridDim.x*blockDim.x) >> 5)
+    {
+        const i64 x = (i64)list[e], l = x/(M*N), mn = x - l*M*N, i = mn/N, j = mn - i*N;
+        const float* a = A + a_l[l] + a_m[i];
+        const float* b = B + b_l[l] + b_n[j];
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (i64 k = lane; k < K; k += 128)
+            #pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k + 32*u < K) s[u] = fma((double)a[a_k[k + 32*u]], (double)b[b_k[k + 32*u]], s[u]);
+        double t = (s[0] + s[1]) + (s[2] + s[3]);
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) C[c_l[l] + c_m[i] + c_n[j]] = alpha*t;
+    }
+}
 
 // One block of 256 threads per (output tile, batch index, quarter of the
 // tile's columns): lane t of a warp takes rows 4t..4t+3 and warp w the
@@ -1303,7 +1367,7 @@ struct CrtCombineArgs
 // vectors (beta == 0: C is not read). Bound by FP64 issue, about 5 operations a
 // modulus; Garner's mixed radix digits in FP32 before took NM^2/2 more and 0.73
 // ms for the ladder's 59 M elements, against 0.19 ms for their bytes.
-template <int NM>
+template <int NM, bool VERIFY>
 __global__ void __launch_bounds__(256)
 oz_crt_combine(const CrtCombineArgs p)
 {
@@ -1379,6 +1443,7 @@ oz_crt_combine(const CrtCombineArgs p)
                 stl[r] = fma(d, tl, stl[r]);
             }
         }
+        const double db = VERIFY ? p.dB[(i64)l*p.N + n] : 0.0;
         const int sb = p.sB[(i64)l*p.N + n];
         const double csc = pow2i(-sb);
         const i64 cn = p.c_n[n];
@@ -1394,6 +1459,21 @@ oz_crt_combine(const CrtCombineArgs p)
             const double pl = fma(p.cc.Mh, fe + stl[r], fma(p.cc.Ml, f, fma(p.cc.Mh, f, -ph)));
             double x = ph + pl;
             if (NM <= 13 && fabs(x) < 2251799813685248.0) x = rint(x);
+            if (VERIFY)
+            {
+                // what the rounding can have changed is below 2^-30 of the value, or
+                // the element is recomputed
+                const double d = p.dA[(i64)l*p.M + m0 + r] + db;
+                if (d > 0.0 && fabs(x) < 0x1p30*d)
+                {
+                    if (*(volatile unsigned*)p.count <= p.cap)
+                    {
+                        const unsigned at = atomicAdd(p.count, 1u);
+                        if (at < p.cap) p.list[at] = (unsigned long long)(((i64)l*p.M + m0 + r)*p.N + n);
+                    }
+                    continue;
+                }
+            }
             // 2^-(sA+sB) as two normal powers of two where the shifts allow
             const double val = p.alpha*((fast && sb > -500 && sb < 500) ? x*rsc[r]*csc : ldexp(x, -(sa[r] + sb)));
             double* dst = C + cm[r] + cn;
@@ -1410,7 +1490,8 @@ void stats(const OzOperand& o, int* e_out, double* ss_out, cudaStream_t st)
         const int ksplit = (int)std::min<i64>(32, std::max<i64>(1, o.K/256));
         dbuf pe((size_t)o.L*ksplit*o.R*sizeof(int), st), ps((size_t)o.L*ksplit*o.R*sizeof(double), st);
         dim3 grid((unsigned)((o.R + ST_THREADS - 1)/ST_THREADS), (unsigned)ksplit, (unsigned)o.L);
-        oz_stats_rows<<<grid, ST_THREADS, 0, st>>>(o, ksplit, pe.as<int>(), ps.as<double>());
+        if (o.f32) oz_stats_rows<float><<<grid, ST_THREADS, 0, st>>>(o, ksplit, pe.as<int>(), ps.as<double>());
+        else oz_stats_rows<double><<<grid, ST_THREADS, 0, st>>>(o, ksplit, pe.as<int>(), ps.as<double>());
         check_launch("oz_stats_rows");
         oz_stats_final<<<(unsigned)((o.R*o.L + 255)/256), 256, 0, st>>>(o.R, o.L, ksplit, pe.as<int>(),
                                                                         ps.as<double>(), e_out, ss_out);
@@ -1420,7 +1501,8 @@ void stats(const OzOperand& o, int* e_out, double* ss_out, cudaStream_t st)
     {
         dbuf pe((size_t)o.L*o.R*sizeof(int), st), ps((size_t)o.L*o.R*sizeof(double), st);
         dim3 grid((unsigned)((o.R*32 + ST_THREADS - 1)/ST_THREADS), 1, (unsigned)o.L);
-        oz_stats_k<<<grid, ST_THREADS, 0, st>>>(o, pe.as<int>(), ps.as<double>());
+        if (o.f32) oz_stats_k<float><<<grid, ST_THREADS, 0, st>>>(o, pe.as<int>(), ps.as<double>());
+        else oz_stats_k<double><<<grid, ST_THREADS, 0, st>>>(o, pe.as<int>(), ps.as<double>());
         check_launch("oz_stats_k");
         oz_stats_final<<<(unsigned)((o.R*o.L + 255)/256), 256, 0, st>>>(o.R, o.L, 1, pe.as<int>(),
                                                                         ps.as<double>(), e_out, ss_out);
@@ -1739,52 +1821,73 @@ double scheme2_seconds(int N, double m, double n, double k)
 
 template <int NM>
 void launch_crt_slice(const OzOperand& o, const int* s, void* out, const PlaneGeom& pg, const CrtConsts& cc,
-                      cudaStream_t st)
+                      cudaStream_t st, int* inexact)
 {
-    launch_slice<NM, OZ_I8, false, true>(o, s, out, pg, st, &cc);
+    launch_slice<NM, OZ_I8, false, true>(o, s, out, pg, st, &cc, inexact);
 }
 
 void crt_slice_dispatch(int nm, const OzOperand& o, const int* s, void* out, const PlaneGeom& pg,
-                        const CrtConsts& cc, cudaStream_t st)
+                        const CrtConsts& cc, cudaStream_t st, int* inexact = nullptr)
 {
+    if (o.f32)
+    {
+        launch_slice<VERIFIED_MODULI, OZ_I8, false, true, float>(o, s, out, pg, st, &cc, inexact);
+        return;
+    }
     switch (nm)
     {
-        case 2: launch_crt_slice<2>(o, s, out, pg, cc, st); break;
-        case 3: launch_crt_slice<3>(o, s, out, pg, cc, st); break;
-        case 4: launch_crt_slice<4>(o, s, out, pg, cc, st); break;
-        case 5: launch_crt_slice<5>(o, s, out, pg, cc, st); break;
-        case 6: launch_crt_slice<6>(o, s, out, pg, cc, st); break;
-        case 7: launch_crt_slice<7>(o, s, out, pg, cc, st); break;
-        case 8: launch_crt_slice<8>(o, s, out, pg, cc, st); break;
-        case 9: launch_crt_slice<9>(o, s, out, pg, cc, st); break;
-        case 10: launch_crt_slice<10>(o, s, out, pg, cc, st); break;
-        case 11: launch_crt_slice<11>(o, s, out, pg, cc, st); break;
-        case 12: launch_crt_slice<12>(o, s, out, pg, cc, st); break;
-        case 13: launch_crt_slice<13>(o, s, out, pg, cc, st); break;
-        case 14: launch_crt_slice<14>(o, s, out, pg, cc, st); break;
-        case 15: launch_crt_slice<15>(o, s, out, pg, cc, st); break;
-        default: launch_crt_slice<16>(o, s, out, pg, cc, st); break;
+        case 2: launch_crt_slice<2>(o, s, out, pg, cc, st, inexact); break;
+        case 3: launch_crt_slice<3>(o, s, out, pg, cc, st, inexact); break;
+        case 4: launch_crt_slice<4>(o, s, out, pg, cc, st, inexact); break;
+        case 5: launch_crt_slice<5>(o, s, out, pg, cc, st, inexact); break;
+        case 6: launch_crt_slice<6>(o, s, out, pg, cc, st, inexact); break;
+        case 7: launch_crt_slice<7>(o, s, out, pg, cc, st, inexact); break;
+        case 8: launch_crt_slice<8>(o, s, out, pg, cc, st, inexact); break;
+        case 9: launch_crt_slice<9>(o, s, out, pg, cc, st, inexact); break;
+        case 10: launch_crt_slice<10>(o, s, out, pg, cc, st, inexact); break;
+        case 11: launch_crt_slice<11>(o, s, out, pg, cc, st, inexact); break;
+        case 12: launch_crt_slice<12>(o, s, out, pg, cc, st, inexact); break;
+        case 13: launch_crt_slice<13>(o, s, out, pg, cc, st, inexact); break;
+        case 14: launch_crt_slice<14>(o, s, out, pg, cc, st, inexact); break;
+        case 15: launch_crt_slice<15>(o, s, out, pg, cc, st, inexact); break;
+        default: launch_crt_slice<16>(o, s, out, pg, cc, st, inexact); break;
     }
 }
 
 void crt_combine_dispatch(const CrtCombineArgs& a, i64 tiles, i64 L, cudaStream_t st)
 {
     dim3 grid((unsigned)tiles, (unsigned)L, 4);
+    if (a.count)
+    {
+        oz_crt_combine<VERIFIED_MODULI, true><<<grid, 256, 0, st>>>(a);
+        check_launch("oz_crt_combine");
+        return;
+    }
     switch (a.cc.nm)
     {
-#define TB_CRT_CASE(n) case n: oz_crt_combine<n><<<grid, 256, 0, st>>>(a); break;
+#define TB_CRT_CASE(n) case n: oz_crt_combine<n, false><<<grid, 256, 0, st>>>(a); break;
         TB_CRT_CASE(2) TB_CRT_CASE(3) TB_CRT_CASE(4) TB_CRT_CASE(5) TB_CRT_CASE(6) TB_CRT_CASE(7)
         TB_CRT_CASE(8) TB_CRT_CASE(9) TB_CRT_CASE(10) TB_CRT_CASE(11) TB_CRT_CASE(12) TB_CRT_CASE(13)
         TB_CRT_CASE(14) TB_CRT_CASE(15)
-        default: oz_crt_combine<16><<<grid, 256, 0, st>>>(a); break;
+        default: oz_crt_combine<16, false><<<grid, 256, 0, st>>>(a); break;
 #undef TB_CRT_CASE
     }
     check_launch("oz_crt_combine");
 }
 
+// bounds and list of a verified run (CrtCombineArgs), all device memory
+struct CrtVerify
+{
+    int* inexact;                  // l*m counters for A, then l*n for B (zeroed)
+    double* bounds;                // the same shape
+    unsigned* count;
+    unsigned cap;
+    unsigned long long* list;
+};
+
 // scheme II on the statistics already computed: shifts, residue planes,
 // one INT8 GEMM per modulus (per exact run of k), CRT combination into C
-void crt_run(OzakiJob& j, int nm, cudaStream_t st)
+void crt_run(OzakiJob& j, int nm, cudaStream_t st, const CrtVerify* ver = nullptr)
 {
     const GemmView& v = j.v;
     TB_CHECK(nm >= 2 && nm <= CRT_MAX, TB_ERR_ARG, "Ozaki moduli count must be 2..16");
@@ -1802,9 +1905,9 @@ void crt_run(OzakiJob& j, int nm, cudaStream_t st)
         check_launch("oz_crt_shifts");
     }
     OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
-                    j.tab->a_m_step, j.tab->a_k_step};
+                    j.tab->a_m_step, j.tab->a_k_step, j.f32};
     OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
-                    j.tab->b_n_step, j.tab->b_k_step};
+                    j.tab->b_n_step, j.tab->b_k_step, j.f32};
     // 128-row tiles of A and B, an even number of each: a CTA pair takes
     // 256 rows of A and 256 columns (two B tiles) of the output
     const i64 k_steps = ((v.k + OZ_BK*CRT_KSUB - 1)/(OZ_BK*CRT_KSUB))*CRT_KSUB;   // a multiple of four
@@ -1813,8 +1916,18 @@ void crt_run(OzakiJob& j, int nm, cudaStream_t st)
     TB_CHECK(ga.k_steps < (1ll << 31), TB_ERR_SIZE, "Ozaki contraction length above 2^31");
     dbuf pa((size_t)(v.l*ga.tiles*ga.k_steps*nm*A_TILE), st);
     dbuf pb((size_t)(v.l*gb.tiles*gb.k_steps*nm*CRT2_TILE), st);
-    crt_slice_dispatch(nm, oa, shA.as<int>(), pa.ptr, ga, cc, st);
-    crt_slice_dispatch(nm, ob, shB.as<int>(), pb.ptr, gb, cc, st);
+    crt_slice_dispatch(nm, oa, shA.as<int>(), pa.ptr, ga, cc, st, ver ? ver->inexact : nullptr);
+    crt_slice_dispatch(nm, ob, shB.as<int>(), pb.ptr, gb, cc, st, ver ? ver->inexact + v.l*v.m : nullptr);
+    if (ver)
+    {
+        const double norm = std::ldexp(1.0, P);
+        oz_inexact_bounds<<<(unsigned)((v.l*v.m + 255)/256), 256, 0, st>>>(ver->inexact, j.sA.as<double>(), v.l*v.m, norm,
+                                                                          ver->bounds);
+        check_launch("oz_inexact_bounds");
+        oz_inexact_bounds<<<(unsigned)((v.l*v.n + 255)/256), 256, 0, st>>>(ver->inexact + v.l*v.m, j.sB.as<double>(),
+                                                                          v.l*v.n, norm, ver->bounds + v.l*v.m);
+        check_launch("oz_inexact_bounds");
+    }
 
     // one launch per exact run of k steps; each writes its own residues of
     // the 128 x 256 tiles
@@ -1857,6 +1970,11 @@ void crt_run(OzakiJob& j, int nm, cudaStream_t st)
     a.M = v.m; a.N = v.n; a.tiles_m = ga.tiles; a.tiles_n = tiles_n;
     a.alpha = j.alpha; a.beta = j.beta;
     a.cc = cc;
+    a.dA = ver ? ver->bounds : nullptr;
+    a.dB = ver ? ver->bounds + v.l*v.m : nullptr;
+    a.count = ver ? ver->count : nullptr;
+    a.cap = ver ? ver->cap : 0;
+    a.list = ver ? ver->list : nullptr;
     TimedLaunch t("oz_crt_combine", st);
     crt_combine_dispatch(a, tiles, v.l, st);
 }
@@ -1895,9 +2013,9 @@ void ozaki_begin(OzakiJob& j, cudaStream_t st)
     j.sA = dbuf((size_t)v.l*v.m*sizeof(double), st);
     j.sB = dbuf((size_t)v.l*v.n*sizeof(double), st);
     OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
-                    j.tab->a_m_step, j.tab->a_k_step};
+                    j.tab->a_m_step, j.tab->a_k_step, j.f32};
     OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
-                    j.tab->b_n_step, j.tab->b_k_step};
+                    j.tab->b_n_step, j.tab->b_k_step, j.f32};
     stats(oa, j.eA.as<int>(), j.sA.as<double>(), st);
     stats(ob, j.eB.as<int>(), j.sB.as<double>(), st);
     if (j.single) return;
@@ -1977,9 +2095,9 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
     j.res.slices = S;
 
     OzOperand oa = {j.A, j.tab->a_m, j.tab->a_k, j.tab->a_l, v.m, v.k, v.l, j.tab->amode,
-                    j.tab->a_m_step, j.tab->a_k_step};
+                    j.tab->a_m_step, j.tab->a_k_step, j.f32};
     OzOperand ob = {j.B, j.tab->b_n, j.tab->b_k, j.tab->b_l, v.n, v.k, v.l, j.tab->bmode,
-                    j.tab->b_n_step, j.tab->b_k_step};
+                    j.tab->b_n_step, j.tab->b_k_step, j.f32};
     const int esz = elem_bytes(kind);
     const i64 ke = OZ_BK/esz;              // k elements per MMA step
     const PlaneGeom ga = {OZ_BM, (v.m + OZ_BM - 1)/OZ_BM, (v.k + ke - 1)/ke, S};
@@ -2013,6 +2131,51 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
     for (int d = 2; d < OZ_SMAX + 2; d++)
         g.w[d - 2] = j.single ? 1.0 : diagonal_weight(kind, d);   // a single pass: weight 1
     gemm_dispatch(kind, S, g, st);
+}
+
+bool ozaki_verified_pays(const GemmView& v)
+{
+    // Fitted to measurements (us): 1600^3 279, 2600^3 546, 4000^3 1180, 10201 x
+    // 1369 x 10201 2250, against 406, 1395, 4595 and 9870 in FP64 with a widening
+    // pass over the operands; 1300^3 238 in FP64. Residue planes of C, and their
+    // combination, cost as much as 250 steps of k: 10000 x 10000 with k = 400 took
+    // 3440 where FP64 took 3190.
+    const double m = (double)v.m, n = (double)v.n, k = (double)v.k, l = (double)v.l;
+    const double mt = (double)((v.m + 255)/256*256), nt = (double)((v.n + 255)/256*256);     // whole tiles
+    const double moduli = l*(VERIFIED_MODULI*(2.0*mt*nt*k/2.8e15 + (mt + nt)*k*3.4e-13 + m*n*1.1e-12) +
+                             1.1e-11*m*n) + 130e-6;
+    const double fp64 = l*(2.0*m*n*k/33e12 + (m + n)*k*3e-12) + 60e-6;
+    return v.l <= 64 && v.m < (1ll << 31) && v.n < (1ll << 31) && v.k < (1ll << 31) && moduli < fp64;
+}
+
+void ozaki_verified(const GemmView& v, const float* A, const float* B, double* C, double alpha, cudaStream_t st,
+                    dbuf& gate, unsigned& gate_above)
+{
+    OzakiJob j;
+    j.v = v; j.A = A; j.B = B; j.C = C;
+    j.f32 = true;
+    j.alpha = alpha; j.beta = 0.0;
+    j.kind = OZ_I8; j.single = true;           // statistics only: the moduli count is fixed
+    const i64 rows = v.l*(v.m + v.n);
+    CrtVerify ver;
+    // recomputing an element reads 2k values a sector each, about 2500 times an
+    // element's share of the DMMA contraction
+    ver.cap = (unsigned)std::min<i64>(1 << 20, std::max<i64>(256, v.l*v.m*v.n/2500));
+    dbuf list((size_t)ver.cap*8, st), bounds((size_t)rows*sizeof(double), st);
+    gate = dbuf((size_t)(rows + 1)*sizeof(int), st);
+    TB_CUDA(cudaMemsetAsync(gate.ptr, 0, gate.bytes, st));
+    ver.count = gate.as<unsigned>();
+    ver.inexact = gate.as<int>() + 1;
+    ver.bounds = bounds.as<double>();
+    ver.list = list.as<unsigned long long>();
+    gate_above = ver.cap;
+    ozaki_begin(j, st);
+    crt_run(j, VERIFIED_MODULI, st, &ver);
+    const GemmTables& t = *j.tab;
+    oz_recompute<<<(unsigned)device_sm_count()*4, 256, 0, st>>>(A, B, C, t.a_m, t.a_k, t.a_l, t.b_n, t.b_k, t.b_l, t.c_m,
+                                                                t.c_n, t.c_l, v.m, v.n, v.k, alpha, ver.count, ver.cap,
+                                                                ver.list);
+    check_launch("oz_recompute");
 }
 
 OzakiResult ozaki_mult(const GemmView& v, const double* A, const double* B, double* C,

@@ -26,13 +26,32 @@ OzakiResult ozaki_mult(const GemmView& v, const double* A, const double* B, doub
                        double alpha, double beta, double tol, int slices, cudaStream_t st,
                        int kind = OZ_I8, bool single = false, int scheme = 0);
 
+// C = alpha*A*B (C is not read) for operands of floats, to float's accuracy and
+// beyond, on the INT8 tensor cores: scheme II with its largest integers (2^50). A
+// float has 24 bits, so almost every element is one of those integers and the
+// products are exact sums; where a row or column did have elements rounded, the
+// combination bounds what that can change, and an element of C for which it is not
+// below 2^-30 of the value is recomputed in FP64. More of them than *gate_above
+// (rows of a wide exponent range, infinities): nothing is recomputed, and the
+// caller's FP64 contraction, queued behind this with the gate, does all of C. The
+// gate's first word is the number; no host synchronisation.
+// Against exact sums (normal, graded and spread operands, k = 10201, 12 draws):
+// 0.5006 units in the last place at most, where rounding the FP64 contraction gave
+// 0.50 to 10.5 (elements that cancel). The list run over costs 12%: 11.0 ms against
+// 9.9.
+// pays: a modelled time below the FP64 contraction's.
+bool ozaki_verified_pays(const GemmView& v);
+void ozaki_verified(const GemmView& v, const float* A, const float* B, double* C, double alpha, cudaStream_t st,
+                    dbuf& gate, unsigned& gate_above);
+
 // the same contraction in two phases, so a caller can queue the statistics
 // of several contractions, do other work, and wait only for the statistics
 struct OzakiJob
 {
     GemmView v;
-    const double* A = nullptr;
-    const double* B = nullptr;
+    const void* A = nullptr;         // double, or float values where f32
+    const void* B = nullptr;
+    bool f32 = false;
     double* C = nullptr;
     double alpha = 1, beta = 0, tol = 1e-12;
     int slices = 0;
