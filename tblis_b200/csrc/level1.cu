@@ -681,30 +681,33 @@ static unsigned pieces_grid(i64 tiles)
 }
 
 template <typename T>
-static void pieces_launch(int op, const T* A, T* B, const std::vector<PieceSpec>& specs, T alpha, T beta, bool conj_a,
+static void pieces_launch(int op, const T* A, T* B, const PieceSpec* specs, size_t nspecs, T alpha, T beta, bool conj_a,
                           bool conj_b, int red_op, typename PcAcc<T>::type* partial, cudaStream_t st)
 {
-    std::vector<Piece> pieces;
+    Piece one{};                             // the only or first piece
+    std::vector<Piece> pieces;               // all, where there are several
+    int np = 0;
     i64 tiles = 0, elements = 0;
-    for (const PieceSpec& sp : specs) elements += total_of(sp.ab);
+    for (size_t i = 0; i < nspecs; i++) elements += total_of(specs[i].ab);
     const i64 size = pc_size<T>(elements);
-    for (const PieceSpec& sp : specs)
+    if (nspecs > 1) pieces.reserve(nspecs);
+    for (size_t i = 0; i < nspecs; i++)
     {
         Piece c;
-        if (!make_piece(sp, c)) continue;
+        if (!make_piece(specs[i], c)) continue;
         if (op == 3) { c.turn = 0; }
         const i64 n = pc_tiles<T>(c, size);
         c.first = (unsigned)tiles;
         tiles += n;
         TB_CHECK(tiles < ((i64)1 << 32), TB_ERR_SIZE, "too many tiles");
-        pieces.push_back(c);
+        if (np++ == 0) one = c;
+        if (nspecs > 1) pieces.push_back(c);
     }
-    if (pieces.empty() && op < 2) return;
-    const Piece one = pieces.empty() ? Piece{} : pieces[0];
+    if (np == 0 && op < 2) return;
     dbuf dev;
     const Piece* many = nullptr;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (pieces.size() > 1 && op < 2 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+    if (np > 1 && op < 2 && cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
         capture == cudaStreamCaptureStatusActive)
     {
         // a replay would read the table's source after this call: a launch per piece
@@ -723,14 +726,13 @@ static void pieces_launch(int op, const T* A, T* B, const std::vector<PieceSpec>
         check_launch("k_pieces");
         return;
     }
-    if (pieces.size() > 1)
+    if (np > 1)
     {
         dev = dbuf(pieces.size()*sizeof(Piece), st);
         // pageable source: staged by the driver before the call returns
         TB_CUDA(cudaMemcpyAsync(dev.ptr, pieces.data(), pieces.size()*sizeof(Piece), cudaMemcpyHostToDevice, st));
         many = dev.as<Piece>();
     }
-    const int np = (int)pieces.size();
     const unsigned nt = (unsigned)tiles;
     if (op == 0)
         k_pieces<T, 0><<<pieces_grid<0>(tiles), PC_THREADS, 0, st>>>(
@@ -751,7 +753,8 @@ template <typename T>
 void l1_add_pieces(const T* A, T* B, const std::vector<PieceSpec>& pieces, T alpha, T beta, cudaStream_t st,
                    bool conj_a, bool conj_b)
 {
-    pieces_launch<T>(beta == T(0) ? 0 : 1, A, B, pieces, alpha, beta, conj_a, conj_b, 0, nullptr, st);
+    pieces_launch<T>(beta == T(0) ? 0 : 1, A, B, pieces.data(), pieces.size(), alpha, beta, conj_a, conj_b, 0, nullptr,
+                     st);
 }
 
 template <typename T, typename Acc>
@@ -759,7 +762,8 @@ static void pieces_sum(int op, int red_op, const T* A, const T* B, const std::ve
                        cudaStream_t st, bool conj_a, bool conj_b)
 {
     dbuf part(kPieceBlocks*sizeof(Acc), st);
-    pieces_launch<T>(op, A, const_cast<T*>(B), pieces, T(0), T(0), conj_a, conj_b, red_op, part.as<Acc>(), st);
+    pieces_launch<T>(op, A, const_cast<T*>(B), pieces.data(), pieces.size(), T(0), T(0), conj_a, conj_b, red_op,
+                     part.as<Acc>(), st);
     k_sum_partials<Acc><<<1, 32, 0, st>>>(part.as<Acc>(), kPieceBlocks, d_result);
     check_launch("k_sum_partials");
 }
@@ -853,7 +857,8 @@ void l1_add(const T* A, T* B, const Strided2& ab, const Strided& ao, const Strid
             }
         }
         TimedLaunch t(rows ? "k_add_rows" : "k_transpose", st);
-        pieces_launch<T>(b0 ? 0 : 1, A, B, {{ab, 0, 0}}, alpha, beta, conj_a, conj_b, 0, nullptr, st);
+        const PieceSpec whole = {ab, 0, 0};
+        pieces_launch<T>(b0 ? 0 : 1, A, B, &whole, 1, alpha, beta, conj_a, conj_b, 0, nullptr, st);
         return;
     }
 

@@ -78,7 +78,8 @@ i64 pc_tiles(Piece& c, i64 E)
     else
     {
         // a few widths, the first that fills the tile (a few hundred pieces a call:
-        // 32-bit divisions)
+        // 32-bit divisions); for a small problem one width, since the call costs more
+        // than the kernel
         typedef unsigned u32;
         auto evenly = [](i64 n, u32 w) -> u32        // n in the fewest equal parts of at most w
         {
@@ -89,8 +90,10 @@ i64 pc_tiles(Piece& c, i64 E)
         };
         double best = -1;
         u32 seen = 0;
-        for (const u32 w : {48u, 64u, 32u, 96u, 24u, 16u})
+        const bool small = E < pc_tile<T>()/2;
+        for (u32 w : {48u, 64u, 32u, 96u, 24u, 16u})
         {
+            if (small) w = E < 512 ? 16 : 28;
             const u32 a = evenly(c.np, w);
             if (a == seen) continue;
             seen = a;
@@ -101,7 +104,7 @@ i64 pc_tiles(Piece& c, i64 E)
             auto run = [](u32 x, i64 all) { return x >= 32 || all <= 32 ? 1.0 : (double)x*(1.0/32.0); };
             const double fill = (double)(a*b*r)*run(a, c.np)*run(b, c.nq);
             if (fill > best) { best = fill; tp = a; tq = b; tr = r; }
-            if (fill >= 0.85*(double)E) break;
+            if (small || fill >= 0.85*(double)E) break;
         }
     }
     // offsets within a tile are kept in 32 bits
