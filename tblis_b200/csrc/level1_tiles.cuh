@@ -23,8 +23,8 @@
 //
 // Measured (FP64): B[baji] = A[abij] - B, extents 97, 97, 31, 31, 43.6 us = 5.0
 // TB/s (113 us with 64 x 64 tiles); without reading B 32.7 us = 4.4 TB/s (64.7). The
-// 512 blocks of an 8-irrep tensor of 30M elements: add 134 us, with beta 167, dot
-// 140, norm 74 (a launch a block: 25 ms and more); their runs of 3 to 60 elements
+// 512 blocks of an 8-irrep tensor of 30M elements: add 128 us, with beta 166, dot
+// 140, norm 73 (a launch a block: 25 ms and more); their runs of 3 to 60 elements
 // leave a tenth of the fetched sectors unused and the last CTAs a sixth behind.
 #pragma once
 
