@@ -601,15 +601,20 @@ __device__ __forceinline__ double flip(double x, unsigned mask)
     return __hiloint2double(__double2hiint(x) ^ (int)mask, __double2loint(x));
 }
 
-// alpha*x + beta*op(c) over a complex element of C (beta == 0: c is not read)
+// alpha*x + beta*op(c) over a complex element of C (beta == 0: c is not read). A
+// factor of zero leaves its product out, so that a real alpha or beta scales
+// each part by itself: 0 times an infinite part would be NaN in the other one.
 __device__ __forceinline__ void update_z(const GemmF64Args& p, double* dst, double re, double im)
 {
-    double vr = p.alpha*re - p.alpha_im*im, vi = p.alpha*im + p.alpha_im*re;
+    double vr, vi;
+    if (p.alpha_im == 0.0) { vr = p.alpha*re; vi = p.alpha*im; }
+    else if (p.alpha == 0.0) { vr = -p.alpha_im*im; vi = p.alpha_im*re; }
+    else { vr = p.alpha*re - p.alpha_im*im; vi = p.alpha*im + p.alpha_im*re; }
     if (p.beta != 0.0 || p.beta_im != 0.0)
     {
         const double cr = dst[0], ci = p.conj_c ? -dst[1] : dst[1];
-        vr += p.beta*cr - p.beta_im*ci;
-        vi += p.beta*ci + p.beta_im*cr;
+        if (p.beta != 0.0) { vr += p.beta*cr; vi += p.beta*ci; }
+        if (p.beta_im != 0.0) { vr -= p.beta_im*ci; vi += p.beta_im*cr; }
     }
     *reinterpret_cast<double2*>(dst) = make_double2(vr, vi);
 }
