@@ -1060,7 +1060,7 @@ __global__ void __launch_bounds__(DN_CT*GROUPS)
 gemm_f64_fixup(const GemmF64Args p)
 {
     constexpr int BM = WGM*MF*16, BN = WGN*NF*8;
-    if (p.gate && *p.gate <= p.gate_above) return;
+    const bool off = p.gate && *p.gate <= p.gate_above;
     __shared__ double sums[GROUPS][2][DN_CT];
     const int tc = threadIdx.x % DN_CT, grp = threadIdx.x/DN_CT;
     const int lane = tc & 31;
@@ -1071,13 +1071,16 @@ gemm_f64_fixup(const GemmF64Args p)
     // the CTAs [c0, c1) whose runs meet this tile's k steps [ub, ue)
     const unsigned kt = (unsigned)p.kt, ub = blockIdx.x*kt, ue = ub + kt;
     const unsigned c0 = cta_of_unit(p, ub), c1 = cta_of_unit(p, ue - 1) + 1;
-    if (c1 - c0 == 1) return;                        // one CTA did the whole tile
     // the CTA's second slot when its first run is part of an earlier tile
     // (whole tiles take no slot); only the first CTA can have such a run
     const unsigned uf = first_unit(p, c0);
     const double* first = p.partial + (i64)(c0*2 + (uf < ub && uf % kt != 0 ? 1 : 0))*(BM*BN) + tc;
-    // launched while the kernel above runs: its sums are complete from here on
+    // launched while the kernel above runs: its sums are complete from here on.
+    // Every block waits, also one with nothing to add: else a launch whose blocks
+    // all return could end, and the next kernel start, before that kernel's writes
+    // to C are visible.
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (off || c1 - c0 == 1) return;                 // one CTA did the whole tile
     for (int e = blockIdx.y; e < MF*NF*2; e += gridDim.y)
     {
         // elements 2e and 2e + 1: neighbouring columns of one row (complex: the
