@@ -984,18 +984,46 @@ __device__ __forceinline__ void dn_body(const Work& work)
             const bool two = n + 1 < t.nrem;
             double* C0 = C + __ldg(c.c_n + t.n0 + n);
             double* C1 = C + (two ? __ldg(c.c_n + t.n0 + n + 1) : 0);
+            // The old values of a fragment's two rows are loaded before the first of
+            // them is stored: one by one, each load behind the store before it, the
+            // update took a memory latency an element. (Registers for more
+            // fragments at once spill.)
             #pragma unroll
             for (int i = 0; i < MF; i++)
+            {
+                const int m = (i*WGM + wm)*16 + fr;
+                const bool in[2] = {m < t.mrem, m + 8 < t.mrem};
+                i64 ro[2];
+                double v[2][2];
+                #pragma unroll
+                for (int hh = 0; hh < 2; hh++) ro[hh] = in[hh] ? __ldg(c.c_m + t.m0 + m + 8*hh) : 0;
+                if (beta != 0.0)
+                {
+                    #pragma unroll
+                    for (int hh = 0; hh < 2; hh++)
+                    {
+                        v[hh][0] = in[hh] ? C0[ro[hh]] : 0.0;
+                        v[hh][1] = in[hh] && two ? C1[ro[hh]] : 0.0;
+                    }
+                    #pragma unroll
+                    for (int hh = 0; hh < 2; hh++)
+                        #pragma unroll
+                        for (int q = 0; q < 2; q++) v[hh][q] = alpha*acc[i][j][2*hh + q] + beta*v[hh][q];
+                }
+                else
+                {
+                    #pragma unroll
+                    for (int hh = 0; hh < 2; hh++)
+                        #pragma unroll
+                        for (int q = 0; q < 2; q++) v[hh][q] = alpha*acc[i][j][2*hh + q];
+                }
                 #pragma unroll
                 for (int hh = 0; hh < 2; hh++)
                 {
-                    const int m = (i*WGM + wm)*16 + 8*hh + fr;
-                    if (m >= t.mrem) continue;
-                    const i64 ro = __ldg(c.c_m + t.m0 + m);
-                    const double v0 = alpha*acc[i][j][2*hh], v1 = alpha*acc[i][j][2*hh + 1];
-                    C0[ro] = beta == 0.0 ? v0 : v0 + beta*C0[ro];
-                    if (two) C1[ro] = beta == 0.0 ? v1 : v1 + beta*C1[ro];
+                    if (in[hh]) C0[ro[hh]] = v[hh][0];
+                    if (in[hh] && two) C1[ro[hh]] = v[hh][1];
                 }
+            }
         }
     }
 }
