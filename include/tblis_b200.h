@@ -244,6 +244,14 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
                            char* idx_AB, char* idx_AC, char* idx_BC, char* idx_ABC,
                            int64_t* mnkl);
 
+/* The work split of the dense FP64 kernel for an m x n x k contraction of l
+ * batch indices on `sms` SMs (host only; for tests): out[0] tile (0: 128 x 128,
+ * 1: 64 x 64, 2: 128 x 32), out[1] whether the operands are exchanged, out[2]
+ * whether tiles are cut along k, out[3] tiles done whole, out[4] tiles cut,
+ * out[5] CTAs. Returns 0 or an error code. */
+int tblis_b200_dense_plan(int64_t m, int64_t n, int64_t k, int64_t l, int complex_elements, int read_c, int sms,
+                          int64_t* out);
+
 /* Number of kernels this library launched since the process started. */
 int64_t tblis_b200_kernel_count(void);
 

@@ -336,6 +336,18 @@ def _scalar_value(s, code):
     return f[0]
 
 
+def dense_plan(m, n, k, l=1, cplx=False, beta=0.0, sms=148):
+    """The dense FP64 kernel's work split for an m x n x k contraction of l batch
+    indices (host only): tile extents, whether the operands are exchanged and
+    tiles are cut along k, tiles done whole, tiles cut, CTAs."""
+    out = (ctypes.c_int64 * 6)()
+    lib.tblis_b200_dense_plan(ctypes.c_int64(m), ctypes.c_int64(n), ctypes.c_int64(k), ctypes.c_int64(l),
+                              int(cplx), int(beta != 0), int(sms), out)
+    _check()
+    return {"tile": ((128, 128), (64, 64), (128, 32))[out[0]], "exchanged": bool(out[1]), "cut": bool(out[2]),
+            "whole": out[3], "cut_tiles": out[4], "ctas": out[5]}
+
+
 def kernel_count():
     """Kernels this library launched in this process."""
     return lib.tblis_b200_kernel_count()

@@ -614,6 +614,26 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
     });
 }
 
+int tblis_b200_dense_plan(int64_t m, int64_t n, int64_t k, int64_t l, int complex_elements, int read_c, int sms,
+                          int64_t* out)
+{
+    return guarded([&]
+    {
+        TB_CHECK(out && m > 0 && n > 0 && k > 0 && l > 0 && sms > 0, TB_ERR_ARG, "dense plan: empty contraction");
+        GemmF64Args a = {};
+        a.M = m; a.N = n; a.K = k; a.L = l;
+        a.beta = read_c ? 1.0 : 0.0;
+        a.cplx = complex_elements != 0;
+        gemm_f64_dense_plan(a, sms, SIZE_MAX);
+        out[0] = a.tile;
+        out[1] = a.M != m || a.N != n;
+        out[2] = a.cut;
+        out[3] = a.dp_tiles;
+        out[4] = a.sk_tiles;
+        out[5] = a.grid;
+    });
+}
+
 int64_t tblis_b200_kernel_count(void) { return g_kernel_count.load(); }
 
 int tblis_b200_kernel_timer(int enable)

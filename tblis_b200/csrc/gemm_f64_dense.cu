@@ -1237,35 +1237,49 @@ double step_cycles(int m, int n)
 template <typename T>
 double split_work(GemmF64Args& a, int sms, size_t ws_limit)
 {
-    // cutting adds a second launch, the partial sums' way through L2 (about
-    // 1.2 KB per cycle) and another pipeline start; kRun: a tile's C update
-    constexpr double kCutCycles = 10000, kRun = 2000, kUnit = 32;
+    // A tile's C update, or the way of its partial sums to the workspace, takes
+    // kOut bytes per cycle and SM after its last step (its warps do nothing else
+    // meanwhile) and kRun for its tables; the fixup starts kFixup late and moves
+    // kChip bytes per cycle. Fitted to forced splits (us, uncut and cut): 4000 x
+    // 4000 with k 16 64 and 64, k 64 109 and 135, k 500 557 and 559; 2000 x 2000 with k
+    // 200 77 and 98; 40000 x 100 with k 500 217 and 190. (2000 cycles a tile and 26000 a
+    // cut, as assumed before, cut 2000 x 2000 from k 200 on.)
+    constexpr double kOut = 9, kRun = 700, kFixup = 9000, kChip = 1700, kUnit = 32;
     constexpr size_t kSlot = (size_t)T::BM*T::BN*sizeof(double);
     const i64 N = a.cplx ? 2*a.N : a.N;
     const i64 fm = a.M/T::BM, fn = N/T::BN, L = a.L;
     const int rm = (int)(a.M - fm*T::BM), rn = (int)(N - fn*T::BN);
     const i64 count[4] = {fm*fn*L, rm ? fn*L : 0, rn ? fm*L : 0, rm && rn ? L : 0};
-    const double cyc[4] = {step_cycles<T>(T::BM, T::BN), step_cycles<T>(std::max(rm, 1), T::BN),
-                           step_cycles<T>(T::BM, std::max(rn, 1)), step_cycles<T>(std::max(rm, 1), std::max(rn, 1))};
+    const int rows[4] = {T::BM, std::max(rm, 1), T::BM, std::max(rm, 1)};
+    const int cols[4] = {T::BN, T::BN, std::max(rn, 1), std::max(rn, 1)};
+    const double elem = a.beta != 0.0 || a.beta_im != 0.0 ? 16.0 : 8.0;      // C is read too
     const double kt = (double)a.kt;
+    double cyc[4], update[4];
     i64 tiles = 0;
     double total = 0, longest = 0;
     for (int c = 0; c < 4; c++)
     {
+        cyc[c] = step_cycles<T>(rows[c], cols[c]);
+        update[c] = kRun + elem*rows[c]*cols[c]/kOut;
         tiles += count[c];
-        total += (double)count[c]*(kt*cyc[c] + kRun);
-        if (count[c]) longest = std::max(longest, kt*cyc[c] + kRun);
+        total += (double)count[c]*(kt*cyc[c] + update[c]);
+        if (count[c]) longest = std::max(longest, kt*cyc[c] + update[c]);
     }
     a.dp_tiles = tiles; a.sk_tiles = 0; a.sk_ctas = 0; a.cut = 0;
     a.sk_per = a.sk_extra = 0;
     a.grid = (int)std::min<i64>(tiles, sms);
     a.ws_bytes = 0;
-    // tiles dealt in turn: about one longest tile above the mean
+    // tiles dealt in turn: whole rounds of them, or a part of one above the mean
     const double whole = tiles <= sms ? longest : std::max((double)((tiles + sms - 1)/sms)*total/(double)tiles,
-                                                           total/sms + 0.5*longest);
+                                                           total/sms + 0.25*longest);
+    // A batch that fills the SMs is not cut: dealt in turn, neighbouring CTAs hold
+    // neighbouring batch indices at the same k, and what they share (32-byte sectors
+    // where the batch label is the fastest) is fetched once. Cut, every CTA has a run
+    // of its own: 100 matrices of 300 x 300 x 300 took 378 us where uncut ones take 238,
+    // and 1034 against 489 with the batch label fastest.
+    if (L > 1 && tiles > sms) return whole;
     // cut: all but the last whole wave of whole tiles stays uncut
     const i64 dp = std::max<i64>(0, (count[0]/sms - 1)*sms);
-    const double cut_total = total - (double)dp*(kt*cyc[0] + kRun);
     double units = 0;
     unsigned first = 0, wmax = 1;
     for (int c = 0; c < 4; c++)
@@ -1281,8 +1295,19 @@ double split_work(GemmF64Args& a, int sms, size_t ws_limit)
     // no run below 1500 cycles (its pipeline start) or two steps of any class
     i64 ctas = std::min<i64>({(i64)sms, (i64)(units*kUnit/1500.0), (i64)(units/(2.0*wmax)), (i64)(ws_limit/(2*kSlot))});
     if (units >= (double)(1ll << 31) || ctas < 2 || (dp > 0 && ctas < sms)) return whole;
-    const double cut = (double)(dp/sms)*(kt*cyc[0] + kRun) + cut_total/(double)ctas + kRun + kCutCycles +
-                       (double)ctas*(double)kSlot/1200.0;
+    const double sk = (double)(tiles - dp), fixed = std::min(sk, (double)ctas);      // tiles that the fixup sums
+    const double slots = std::min((double)ctas + sk, 2.0*(double)ctas);
+    double steps = 0, updates = 0, elements = 0;       // of the cut tiles
+    for (int c = 0; c < 4; c++)
+    {
+        const double n = (double)(count[c] - (c == 0 ? dp : 0));
+        steps += n*kt*cyc[c];
+        updates += n*update[c];
+        elements += n*rows[c]*cols[c];
+    }
+    const double mean = elements/sk;                   // elements of a tile
+    const double cut = (double)(dp/sms)*(kt*cyc[0] + update[0]) + (steps + (sk - fixed)*updates/sk)/(double)ctas +
+                       slots/(double)ctas*mean*8.0/kOut + kFixup + (slots*8.0 + fixed*elem)*mean/kChip;
     if (cut >= whole) return whole;
     a.dp_tiles = dp;
     a.sk_tiles = tiles - dp;
