@@ -243,6 +243,30 @@ static void dense_gemm(GemmF64Args& a, cudaStream_t st)
     gemm_f64_dense_launch(a, st);
 }
 
+// Contractions of one k step (up to 16 k) are the writing of C, with nothing to
+// overlap it: where they are large, three small CTAs per SM (gemm_f64.cu)
+// write faster than the dense kernel's one, and the tiny matrices of a batch cost
+// the dense kernel a pipeline start each. FP64, us, small CTAs / dense kernel:
+//   40000 x 100 x 16 21 / 29, 10000 x 1000 x 16 42 / 46, 4000 x 4000 x 1 58 / 66, but 500 x 500
+//   17 / 17, and with beta 178 / 145 (rows of C contiguous; 130 / 157 its columns)
+//   1000 matrices of 1000 x 60 x 3 221 / 298, 10000 of 64 x 64 x 3 150 / 188, 60000 of 4 x 4
+//   450 / 575, 30000 of 5 x 40 314 / 312; but 10000 of 32 x 32 x 16 128 / 117 and of 20 x
+//   200 x 16 448 / 300
+static bool one_step(const GemmView& v, double beta)
+{
+    if (v.k > gemm_f64_tile_k()) return false;
+    const double mn = (double)v.m*(double)v.n;
+    if (v.l == 1)
+    {
+        auto least = [](const ivec& s) { i64 x = INT64_MAX; for (i64 t : s) x = std::min<i64>(x, std::llabs(t)); return x; };
+        if (std::min(v.m, v.n) <= 32 || mn < 524288.0) return false;
+        return beta == 0.0 || (mn >= 8388608.0 && least(v.cN) < least(v.cM));
+    }
+    // how full the 64 x 64 tiles of one matrix are
+    const double fill = mn/(4096.0*(double)(((v.m + 63)/64)*((v.n + 63)/64)));
+    return fill < 0.07 || (beta == 0.0 && fill >= 0.5);
+}
+
 // one contraction on device data (a GEMM view of device-resident operands)
 static void contract_device(const GemmView& v, const double* A, const double* B, double* C, double alpha,
                             double beta, int method, double tol, int slices, cudaStream_t st,
@@ -279,7 +303,12 @@ static void contract_device(const GemmView& v, const double* A, const double* B,
     a.alpha = alpha; a.beta = beta;
     a.amode = tab->amode; a.bmode = tab->bmode;
     a.gate = gate; a.gate_above = gate_above;
-    dense_gemm(a, st);
+    if (!gate && one_step(v, beta))
+    {
+        a.splits = 1;
+        gemm_f64_launch(a, st);
+    }
+    else dense_gemm(a, st);
     used_slices = 0;
     est_error = 1.1e-16*std::sqrt((double)v.k);
 }
