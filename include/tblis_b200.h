@@ -149,11 +149,17 @@ unsigned tblis_get_num_threads(void);
 void tblis_set_num_threads(unsigned num_threads);
 
 /* src/util/configs.h:11: returns a GPU configuration by name, or NULL.
- * Names: "b200_fp64" (default; FP64 DMMA), "b200_ozaki_i8" (Ozaki INT8 on
+ * Names: "b200_fp64" (FP64 DMMA; what a call without a configuration takes too,
+ * but for large float contractions, below), "b200_ozaki_i8" (Ozaki INT8 on
  * tcgen05: slices or moduli, whichever needs less INT8 work for the
  * tolerance), "b200_ozaki_bf16" (Ozaki BF16 slices), "b200_ozaki_crt" (Ozaki
  * INT8 over pairwise-coprime moduli only, scheme II), "b200_tf32" and
- * "b200_bf16" (one low-precision pass with FP32 accumulation). */
+ * "b200_bf16" (one low-precision pass with FP32 accumulation).
+ * Float contractions compute in FP64 and round once at the end. Without a
+ * configuration and a method, those large enough for it to pay compute in exact
+ * integers of 50 bits a row on the INT8 cores instead: an element of C that
+ * rounding the operands to them could have changed by more than 2^-30 of its
+ * value is recomputed in FP64. "b200_fp64", or method 1, keeps FP64. */
 const tblis_config* tblis_get_config(const char* name);
 
 /* ---- extensions (no counterpart in the reference) ------------------------ */
@@ -199,7 +205,8 @@ double tblis_b200_config_get_tolerance(const tblis_config* cfg);
 /* Per-call options and report of the extended contraction entry point. */
 typedef struct tblis_b200_opts
 {
-    int method;          /* 0 = from cfg, 1 = FP64 DMMA, 2 = Ozaki INT8 (slices
+    int method;          /* 0 = from cfg (no cfg: FP64, large float contractions
+                            as at tblis_get_config), 1 = FP64 DMMA, 2 = Ozaki INT8 (slices
                             or moduli, whichever needs less INT8 work for the
                             tolerance), 3 = Ozaki BF16 slices, 4 = one TF32
                             pass, 5 = one BF16 pass (FP32 accumulation; no
@@ -211,9 +218,11 @@ typedef struct tblis_b200_opts
 
 typedef struct tblis_b200_report
 {
-    int method;          /* method that ran (6 when method 2 chose moduli) */
+    int method;          /* method that ran (6 when method 2, or a float
+                            contraction without a method, chose moduli) */
     int slices;          /* slice count, or moduli count for method 6 (0 for FP64) */
-    double est_error;    /* a-priori normwise error estimate */
+    double est_error;    /* a-priori normwise error estimate (of a float
+                            contraction: before C is rounded to float) */
     double flops;        /* algorithmic FLOPs, 2*m*n*k*l */
     int64_t m, n, k, l;  /* GEMM view of the contraction */
     int kernels;         /* kernels launched by this call */

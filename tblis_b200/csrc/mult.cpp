@@ -566,12 +566,12 @@ static void mult_widened(const tblis_config* cfg,
     stage(sa, A, true, st, cx ? 8 : 4);
     stage(sb, B, true, st, cx ? 8 : 4);
 
-    // a large float contraction on the FP64 path takes the INT8 cores, verified
-    // (ozaki_verified): the FP64 pipe has a tenth of their rate
+    // a large float contraction whose caller has named no method takes the INT8
+    // cores, verified (ozaki_verified): the FP64 pipe has a tenth of their rate. A
+    // named FP64 (method 1, b200_fp64) stays FP64.
     GemmView v;
     bool moduli = false;
-    if (!cx && (opts && opts->method ? opts->method : (cfg ? cfg->method : 1)) == 1 &&
-        (double)A->scalar.data.s*(double)B->scalar.data.s != 0.0)
+    if (!cx && !(opts && opts->method) && !cfg && (double)A->scalar.data.s*(double)B->scalar.data.s != 0.0)
     {
         v = gemm_view(mult_groups(A, idx_A, B, idx_B, C, idx_C));
         // (every element of C is written: none of its labels repeats)
@@ -629,9 +629,10 @@ static void mult_widened(const tblis_config* cfg,
         else l1_convert<double, float>(c, static_cast<float*>(sc.dptr), rv[2]->s, st);
         if (report)
         {
-            report->method = 1;
-            report->slices = 0;
-            report->est_error = est;
+            report->method = done ? 6 : 1;
+            report->slices = done ? ozaki_verified_moduli() : 0;
+            // what the verification lets pass, in every element (the others are FP64)
+            report->est_error = done ? std::max(est, ozaki_verified_error()) : est;
             report->m = v.m; report->n = v.n; report->k = v.k; report->l = v.l;
             report->flops = 2.0*(double)v.m*(double)v.n*(double)v.k*(double)v.l;
             report->kernels = (int)(g_kernel_count.load() - kernels_before);

@@ -1293,6 +1293,7 @@ __global__ void oz_crt_shifts(const double* ss, i64 n, int P, int* s_out)
 }
 
 constexpr int VERIFIED_MODULI = 13;    // P = 50: the most that the digit extraction takes
+constexpr double VERIFIED_ERROR = 0x1p-30;     // of an element's value
 
 struct CrtCombineArgs
 {
@@ -1461,10 +1462,10 @@ oz_crt_combine(const CrtCombineArgs p)
             if (NM <= 13 && fabs(x) < 2251799813685248.0) x = rint(x);
             if (VERIFY)
             {
-                // what the rounding can have changed is below 2^-30 of the value, or
-                // the element is recomputed
+                // what the rounding can have changed is below VERIFIED_ERROR of the
+                // value, or the element is recomputed
                 const double d = p.dA[(i64)l*p.M + m0 + r] + db;
-                if (d > 0.0 && fabs(x) < 0x1p30*d)
+                if (d > 0.0 && fabs(x) < d*(1.0/VERIFIED_ERROR))
                 {
                     if (*(volatile unsigned*)p.count <= p.cap)
                     {
@@ -2132,6 +2133,9 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
         g.w[d - 2] = j.single ? 1.0 : diagonal_weight(kind, d);   // a single pass: weight 1
     gemm_dispatch(kind, S, g, st);
 }
+
+int ozaki_verified_moduli() { return VERIFIED_MODULI; }
+double ozaki_verified_error() { return VERIFIED_ERROR; }
 
 bool ozaki_verified_pays(const GemmView& v)
 {

@@ -41,6 +41,8 @@ OzakiResult ozaki_mult(const GemmView& v, const double* A, const double* B, doub
 // 9.9.
 // pays: a modelled time below the FP64 contraction's.
 bool ozaki_verified_pays(const GemmView& v);
+int ozaki_verified_moduli();
+double ozaki_verified_error();     // relative, of an element that is not recomputed
 void ozaki_verified(const GemmView& v, const float* A, const float* B, double* C, double alpha, cudaStream_t st,
                     dbuf& gate, unsigned& gate_above);
 
