@@ -253,6 +253,10 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
                            char* idx_AB, char* idx_AC, char* idx_BC, char* idx_ABC,
                            int64_t* mnkl);
 
+/* Test support: device allocations above `bytes` (0: no limit) fail as if there
+ * were no room, so that the ways taken without their scratch can be run. */
+void tblis_b200_limit_allocations(size_t bytes);
+
 /* The work split of the dense FP64 kernel for an m x n x k contraction of l
  * batch indices on `sms` SMs (host only; for tests): out[0] tile (0: 128 x 128,
  * 1: 64 x 64, 2: 128 x 32), out[1] whether the operands are exchanged, out[2]

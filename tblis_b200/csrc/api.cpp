@@ -22,6 +22,7 @@ namespace tb
 
 std::atomic<int64_t> g_kernel_count{0};
 std::atomic<bool> g_ktimer_on{false};
+std::atomic<size_t> g_alloc_limit{SIZE_MAX};
 
 namespace
 {
@@ -613,6 +614,8 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
         mnkl[0] = v.m; mnkl[1] = v.n; mnkl[2] = v.k; mnkl[3] = v.l;
     });
 }
+
+void tblis_b200_limit_allocations(size_t bytes) { g_alloc_limit.store(bytes ? bytes : SIZE_MAX); }
 
 int tblis_b200_dense_plan(int64_t m, int64_t n, int64_t k, int64_t l, int complex_elements, int read_c, int sms,
                           int64_t* out)

@@ -47,6 +47,13 @@ struct error : std::runtime_error
     error(int c, const std::string& msg) : std::runtime_error(msg), code(c) {}
 };
 
+// a device allocation that found no room (callers with a way that needs less catch
+// this one only)
+struct alloc_error : error
+{
+    alloc_error(const std::string& msg) : error(TB_ERR_CUDA, msg) {}
+};
+
 void set_last_error(int code, const char* msg);
 
 #define TB_CUDA(call)                                                               \
@@ -133,6 +140,10 @@ inline void check_launch(const char* what)
     count_launch();
 }
 
+// device allocations above this many bytes fail as if there were no room (test
+// support: tblis_b200_limit_allocations)
+extern std::atomic<size_t> g_alloc_limit;
+
 // Stream-ordered device allocation from the device's default memory pool
 // (the GPU counterpart of TBLIS's MemoryPool, src/memory/memory_pool.hpp:18-166).
 struct dbuf
@@ -144,7 +155,11 @@ struct dbuf
     dbuf() {}
     dbuf(size_t n, cudaStream_t s) : bytes(n), stream(s)
     {
-        if (n) TB_CUDA(cudaMallocAsync(&ptr, n, s));
+        if (!n) return;
+        const cudaError_t e = n > g_alloc_limit.load(std::memory_order_relaxed) ? cudaErrorMemoryAllocation
+                                                                                : cudaMallocAsync(&ptr, n, s);
+        if (e == cudaErrorMemoryAllocation) throw alloc_error("no device memory for " + std::to_string(n) + " bytes");
+        TB_CUDA(e);
     }
     dbuf(const dbuf&) = delete;
     dbuf& operator=(const dbuf&) = delete;

@@ -232,7 +232,7 @@ static void dense_gemm(GemmF64Args& a, cudaStream_t st)
     if (a.ws_bytes)
     {
         try { ws = dbuf(a.ws_bytes, st); }
-        catch (const error&)
+        catch (const alloc_error&)
         {
             cudaGetLastError();
             a = unplanned;
@@ -614,7 +614,7 @@ static void mult_widened(const tblis_config* cfg,
         unsigned above = 0;
         bool done = false;
         try { ozaki_verified(v, a, b, c, alpha, st, gate, above); done = true; }
-        catch (const error&)
+        catch (const alloc_error&)
         {
             // no room for the residue planes: FP64 does all of it
             cudaGetLastError();

@@ -1,10 +1,13 @@
-"""Which method a large float contraction runs, and what its report says.
+"""Which method a large float contraction runs, what its report says, and what it
+does without room for the residue planes.
 
 A caller that names FP64 (method 1 or the b200_fp64 configuration) gets FP64; one
 that names nothing gets verified moduli, reported as method 6 with 13 moduli and
 the 2^-30 that they may differ by. Tolerance: one rounding to float with that, and
 k * 2^-53 of the absolute values (FP64).
 """
+import ctypes
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +55,45 @@ def test_unnamed_reports_moduli(cuda):
     assert launches == 1 and r["method"] == 6 and r["slices"] == 13 and r["est_error"] >= 2.0 ** -30
     assert (r["m"] * r["n"], r["k"], r["l"]) == (M * N, K, 1) and r["flops"] == 2.0 * M * N * K
     check(*ops, 2.0 ** -29)
+
+
+def test_without_room(cuda):
+    """No room for the residue planes (13 bytes an element of A): FP64, and the
+    report says so; no room for the widened operands either is an error."""
+    import tblis_b200 as tb
+    limit = tb.lib.tblis_b200_limit_allocations
+    limit.argtypes, limit.restype = [ctypes.c_size_t], None
+    limit(8 * max(M * K, K * N, M * N))
+    try:
+        ops, r, launches = run(tb, cuda)
+        assert launches == 0 and r["method"] == 1 and r["slices"] == 0
+        check(*ops, 0.0)
+        limit(4 * M * N)
+        with pytest.raises(tb.TblisError) as e:
+            run(tb, cuda)
+        assert e.value.code == 3
+    finally:
+        limit(0)
+        tb.kernel_timer(False)
+    ops, r, launches = run(tb, cuda)
+    assert launches == 1 and r["method"] == 6
+    check(*ops, 2.0 ** -29)
+
+
+def test_dense_without_workspace(cuda):
+    """A contraction whose plan cuts tiles, without room for their sums."""
+    import torch
+    import tblis_b200 as tb
+    limit = tb.lib.tblis_b200_limit_allocations
+    limit.argtypes, limit.restype = [ctypes.c_size_t], None
+    for dtype in (torch.float64, torch.complex128):
+        m, n, k = 97, 90, 20000
+        assert tb.dense_plan(m, n, k, 1, dtype == torch.complex128)["cut"]
+        A, B = torch.randn(m, k, dtype=dtype, device=cuda), torch.randn(k, n, dtype=dtype, device=cuda)
+        C = torch.full((m, n), float("nan"), dtype=dtype, device=cuda)
+        limit(1 << 10)
+        try:
+            tb.mult(1.0, A, "ik", B, "kj", 0.0, C, "ij")
+        finally:
+            limit(0)
+        assert bool(((C - A @ B).abs() <= 4 * k * 2.0 ** -53 * (A.abs() @ B.abs())).all())
