@@ -573,11 +573,15 @@ static void mult_widened(const tblis_config* cfg,
     bool moduli = false;
     if (!cx && !(opts && opts->method) && !cfg && (double)A->scalar.data.s*(double)B->scalar.data.s != 0.0)
     {
-        v = gemm_view(mult_groups(A, idx_A, B, idx_B, C, idx_C));
-        // (every element of C is written: none of its labels repeats)
-        i64 elements = 1;
-        for (unsigned d = 0; d < C->ndim; d++) elements *= C->len[d];
-        moduli = v.k != 0 && v.m*v.n*v.l == elements && elements != 0 && ozaki_verified_pays(v);
+        auto elements = [](const tblis_tensor* X) { i64 n = 1; for (unsigned d = 0; d < X->ndim; d++) n *= X->len[d]; return n; };
+        const i64 c = elements(C);
+        // m n k l <= sqrt(|A| |B| |C|): most calls are too small to need the GEMM view
+        if ((double)elements(A)*(double)elements(B)*(double)c >= 1e18)
+        {
+            v = gemm_view(mult_groups(A, idx_A, B, idx_B, C, idx_C));
+            // (every element of C is written: none of its labels repeats)
+            moduli = v.k != 0 && v.m*v.n*v.l == c && c != 0 && ozaki_verified_pays(v);
+        }
     }
 
     const tblis_tensor* src[3] = {A, B, C};
