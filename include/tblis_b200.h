@@ -175,9 +175,10 @@ void tblis_b200_clear_error(void);
 void tblis_b200_set_stream(void* stream);
 void* tblis_b200_get_stream(void);
 /* Waits for all work this library enqueued on the current stream. Records
- * TB_ERR_TIMEOUT (6) as the last error when an Ozaki kernel or the packed
- * grouped FP64 kernel gave up one of its bounded waits since the previous
- * check (the flag is then cleared). */
+ * TB_ERR_TIMEOUT (6) as the last error when an Ozaki kernel, the dense FP64
+ * kernel or a grouped FP64 kernel gave up one of its bounded waits since the
+ * previous check (the flags are the process's and are then cleared): part of a
+ * result was then not written. */
 void tblis_b200_synchronize(void);
 
 /* Test support for the failure detection of the Ozaki kernels (no reference
@@ -188,6 +189,12 @@ void tblis_b200_synchronize(void);
  * and returns, and tblis_b200_synchronize reports it. step = -1 and
  * wait_seconds <= 0 restore normal operation. Returns 0 or an error code. */
 int tblis_b200_ozaki_inject_wait_timeout(int step, double wait_seconds);
+
+/* The same for the dense FP64 kernel, also over the groups of a plan: the ring
+ * stage `stage` (0 to 5) of every CTA never becomes full, and every bounded wait
+ * gives up after wait_seconds; the CTAs wait for the copies that they issued and
+ * return. stage = -1 and wait_seconds <= 0 restore normal operation. */
+int tblis_b200_dense_inject_wait_timeout(int stage, double wait_seconds);
 
 /* The same for the packed grouped FP64 GEMM (DPD, indexed DPD and batches on
  * the packed path; no reference counterpart): its producer issues no copy for

@@ -54,6 +54,17 @@ tblis_config_s g_cfgs[] = {
 };
 }
 
+void finish_stream(cudaStream_t st, int waits)
+{
+    TB_CUDA(cudaStreamSynchronize(st));
+    const bool dense = (waits & WAITS_DENSE) && gemm_f64_dense_error_flag() != 0;
+    const bool grouped = (waits & WAITS_GROUPED) && gemm_f64_error_flag() != 0;
+    const bool oz = (waits & WAITS_OZAKI) && ozaki_error_flag() != 0;
+    TB_CHECK(!oz, TB_ERR_TIMEOUT, "an Ozaki kernel gave up a bounded wait");
+    TB_CHECK(!grouped, TB_ERR_TIMEOUT, "a grouped FP64 kernel gave up a bounded wait");
+    TB_CHECK(!dense, TB_ERR_TIMEOUT, "a dense FP64 kernel gave up a bounded wait");
+}
+
 void set_last_error(int code, const char* msg)
 {
     t_err_code = code;
@@ -564,18 +575,17 @@ void tblis_b200_set_stream(void* stream) { t_stream = static_cast<cudaStream_t>(
 void* tblis_b200_get_stream(void) { return t_stream; }
 void tblis_b200_synchronize(void)
 {
-    guarded([&]
-    {
-        TB_CUDA(cudaStreamSynchronize(t_stream));
-        TB_CHECK(ozaki_error_flag() == 0, TB_ERR_TIMEOUT, "an Ozaki kernel gave up a bounded wait");
-        TB_CHECK(gemm_f64_error_flag() == 0, TB_ERR_TIMEOUT, "a grouped FP64 kernel gave up a bounded wait");
-        TB_CHECK(gemm_f64_dense_error_flag() == 0, TB_ERR_TIMEOUT, "a dense FP64 kernel gave up a bounded wait");
-    });
+    guarded([&] { finish_stream(t_stream, WAITS_ALL); });
 }
 
 int tblis_b200_ozaki_inject_wait_timeout(int step, double wait_seconds)
 {
     return guarded([&] { ensure_device(); ozaki_inject_wait_timeout(step, wait_seconds); });
+}
+
+int tblis_b200_dense_inject_wait_timeout(int stage, double wait_seconds)
+{
+    return guarded([&] { ensure_device(); gemm_f64_dense_inject_wait_timeout(stage, wait_seconds); });
 }
 
 int tblis_b200_grouped_inject_wait_timeout(int step, double wait_seconds)

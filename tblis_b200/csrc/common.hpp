@@ -100,6 +100,12 @@ void checked(F&& f)
     if (c) throw error(c, tblis_b200_last_error_string());
 }
 
+// Waits for the stream, then throws TB_ERR_TIMEOUT if a kernel of the given kinds
+// gave up a bounded wait since the last check (its results are incomplete). Calls
+// on host data end with it; the flags are the process's and are cleared.
+enum { WAITS_DENSE = 1, WAITS_GROUPED = 2, WAITS_OZAKI = 4, WAITS_ALL = 7 };
+void finish_stream(cudaStream_t st, int waits);
+
 cudaStream_t current_stream();
 void ensure_device();
 

@@ -6,6 +6,18 @@
 namespace tb
 {
 
+// the bounded waits of the dense kernel: the host's flag of one that gave up, their
+// limit, and a ring stage that never fills up (test support, -1: none)
+struct WaitControl
+{
+    int* error;
+    unsigned long long wait_ns;
+    int hold_stage;
+};
+
+// A kernel argument: 376 bytes took the host 0.7 us a launch more than 352 (11.6 and
+// 10.9 us for the whole call of a small contraction), so the fields that only one
+// of the launchers uses share their place.
 struct GemmF64Args
 {
     const double* A;
@@ -13,13 +25,17 @@ struct GemmF64Args
     double* C;
     // scatter vectors (device): element offsets per GEMM index
     const i64 *a_m, *a_k, *b_k, *b_n, *c_m, *c_n, *a_l, *b_l, *c_l;
-    // per-BK-block common k strides of A and B (0 = irregular block)
-    const i64 *a_kbs, *b_kbs;
+    union
+    {
+        // gemm_f64_launch: per-BK-block common k strides of A and B (0 = irregular
+        // block), and its own share of k
+        struct { const i64 *a_kbs, *b_kbs; i64 k_per_split; };
+        WaitControl ctl;     // the dense kernel's launcher sets it
+    };
     i64 M, N, K, L;
     double alpha, beta;
     int amode, bmode;        // gather directions (see GemmView)
     int splits;              // split-K factor
-    i64 k_per_split;         // set by the launcher
     double* partial;         // split-K workspace (splits*L*M*N doubles)
     int variant;             // tile configuration, 0 = automatic
     // complex contraction (dense kernel only; offsets and extents in complex
@@ -39,6 +55,8 @@ struct GemmF64Args
     unsigned sk_per, sk_extra, cls_first[5], cls_w[4];
     size_t ws_bytes;
 };
+
+static_assert(sizeof(GemmF64Args) <= 352, "GemmF64Args as a kernel argument");
 
 // one K segment of a grouped GEMM: the rows of A / columns of B it reads
 // and its k range (all segments of a group accumulate into the same C tile)
@@ -149,7 +167,11 @@ void gemm_f64_launch(GemmF64Args a, cudaStream_t stream);
 // and a.ws_bytes, at most ws_limit bytes of workspace for a.partial; launch
 // runs it.
 void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit);
-void gemm_f64_dense_launch(const GemmF64Args& a, cudaStream_t stream);
+void gemm_f64_dense_launch(GemmF64Args& a, cudaStream_t stream);
+// nonzero once after a dense kernel (also a grouped one) gave up a wait
 int gemm_f64_dense_error_flag();
+// test support: ring stage `stage` never fills (-1: none) and waits give up after wait_seconds (0: 2 s)
+void gemm_f64_dense_inject_wait_timeout(int stage, double wait_seconds);
+int gemm_f64_dense_control_changes();      // times that was called: a captured launch holds older values
 
 } // namespace tb

@@ -35,7 +35,8 @@
 // scheduling, and no kernel waits for another CTA.
 //
 // Every wait is bounded (2 s of wall clock): one that gives up ends the CTA's
-// work and records the error for the host (gemm_f64_dense_error_flag).
+// work and records the error for the host (gemm_f64_dense_error_flag); part of C
+// is then not written.
 #include "gemm_f64.hpp"
 #include "gemm_f64_dev.cuh"
 
@@ -54,6 +55,7 @@ using namespace f64dev;
 constexpr int DN_PRODUCERS = 4, DN_CONSUMERS = 8;           // warps (per team of producers)
 constexpr int DN_PT = DN_PRODUCERS*32, DN_CT = DN_CONSUMERS*32;
 constexpr unsigned long long DN_WAIT_NS = 2000000000ull;    // 2 s
+constexpr unsigned long long DN_WAIT_MIN_NS = 10000000ull;  // no limit is below 10 ms: short waits need not read theirs
 // registers per thread at launch, and after the split between the roles (a sum
 // over the warps above the launch's would wait forever)
 constexpr int dn_threads(int teams) { return teams*DN_PT + DN_CT; }
@@ -63,7 +65,20 @@ constexpr int dn_reg_c(int teams) { return teams == 1 ? 200 : 184; }
 static_assert(DN_PT*dn_reg_p(1) + DN_CT*dn_reg_c(1) <= dn_threads(1)*dn_reg_launch(1), "register split");
 static_assert(2*DN_PT*dn_reg_p(2) + DN_CT*dn_reg_c(2) <= dn_threads(2)*dn_reg_launch(2), "register split");
 
-__device__ int g_dn_error = 0;
+// the CTA's state of failure, in shared memory: its waits give up together
+struct DnFail
+{
+    int abort;
+    unsigned long long limit; // of a wait, ns
+};
+
+// records for the host that this CTA gave up (once, at a role's end: the waits are
+// inlined in many places, and a longer kernel starts later)
+__device__ __forceinline__ void dn_report(int* error)
+{
+    *(volatile int*)error = 1;            // mapped host memory
+    __threadfence_system();
+}
 
 // smem position of element (row, k) of an operand tile of R rows and 16 k.
 // MODE 0 (gathered along the rows): k rows of R doubles; MODE 1 (along k):
@@ -75,7 +90,7 @@ __device__ __forceinline__ int tile_pos(int row, int k)
     return MODE == 0 ? k*R + (row ^ ((k & 3) << 2)) : row*BK + (k ^ ((row & 3) << 2));
 }
 
-__device__ __forceinline__ bool dn_wait_slow(uint64_t* b, uint32_t parity, volatile int* abort_flag)
+__device__ __forceinline__ bool dn_wait_slow(uint64_t* b, uint32_t parity, volatile DnFail* fail)
 {
     const unsigned long long t0 = gtimer();
     for (unsigned it = 0;; it++)
@@ -83,20 +98,20 @@ __device__ __forceinline__ bool dn_wait_slow(uint64_t* b, uint32_t parity, volat
         if (mb_try(b, parity)) return true;
         if ((it & 63) == 0)
         {
-            if (*abort_flag) return false;
-            if (gtimer() - t0 > DN_WAIT_NS)
+            if (fail->abort) return false;
+            const unsigned long long waited = gtimer() - t0;
+            if (waited > DN_WAIT_MIN_NS && waited > fail->limit)
             {
-                *abort_flag = 1;
-                atomicExch(&g_dn_error, 1);
+                fail->abort = 1;
                 return false;
             }
         }
     }
 }
 
-__device__ __forceinline__ bool dn_wait(uint64_t* b, uint32_t parity, volatile int* abort_flag)
+__device__ __forceinline__ bool dn_wait(uint64_t* b, uint32_t parity, volatile DnFail* fail)
 {
-    const bool ok = mb_try(b, parity) || dn_wait_slow(b, parity, abort_flag);
+    const bool ok = mb_try(b, parity) || dn_wait_slow(b, parity, fail);
     return __all_sync(0xffffffffu, ok) != 0;
 }
 
@@ -586,7 +601,7 @@ template <int STAGES>
 struct DnShared
 {
     uint64_t full[STAGES], empty[STAGES];
-    int abort;
+    DnFail fail;
 };
 
 template <int WGM, int WGN, int MF, int NF, int STAGES, int TEAMS>
@@ -657,6 +672,7 @@ struct DenseWork
         return Target{p.C + (CPLX ? 2 : 1)*p.c_l[t.l], p.c_m, p.c_n, p.alpha, p.beta};
     }
     __device__ __forceinline__ double* partial() const { return p.partial; }
+    __device__ __forceinline__ const WaitControl& control() const { return p.ctl; }
 };
 
 // The GEMMs of a grouped plan: tiles listed by the plan (group by group), the k
@@ -675,6 +691,8 @@ struct GroupWork
     const GroupTile* tiles;
     const GroupStart* start;
     double* w;
+    const WaitControl& ctl;
+    __device__ __forceinline__ const WaitControl& control() const { return ctl; }
     __device__ __forceinline__ GemmF64Args args() const { return GemmF64Args(); }     // complex groups do not occur
     __device__ __forceinline__ bool run(unsigned r, Run& out) const
     {
@@ -759,17 +777,19 @@ __device__ __forceinline__ void dn_body(const Work& work)
     extern __shared__ __align__(128) double smem[];
     i64* sro = reinterpret_cast<i64*>(smem + STAGES*STAGE);        // each team's row offsets of A, then of B
     DnShared<STAGES>& sh = *reinterpret_cast<DnShared<STAGES>*>(sro + TEAMS*(BM + BN));
-    volatile int* abort_flag = &sh.abort;
+    volatile DnFail* fail = &sh.fail;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0)
     {
         for (int s = 0; s < STAGES; s++)
         {
-            mb_init(&sh.full[s], DN_PRODUCERS);       // one arrival per producer warp, its copies landed
+            // one arrival per producer warp, its copies landed
+            mb_init(&sh.full[s], DN_PRODUCERS + (s == work.control().hold_stage ? 1 : 0));
             mb_init(&sh.empty[s], DN_CONSUMERS);      // one arrival per consumer warp
         }
-        sh.abort = 0;
+        sh.fail.abort = 0;
+        sh.fail.limit = work.control().wait_ns;
     }
     __syncthreads();
     // from here on the roles never wait on a CTA-wide barrier
@@ -824,7 +844,7 @@ __device__ __forceinline__ void dn_body(const Work& work)
                 }
                 if (turn == team)
                 {
-                    if (wrapped && !dn_wait(&sh.empty[st], phase ^ 1, abort_flag))
+                    if (wrapped && !dn_wait(&sh.empty[st], phase ^ 1, fail))
                     {
                         ok = false;
                         break;
@@ -854,6 +874,7 @@ __device__ __forceinline__ void dn_body(const Work& work)
         // the last stages (also after a wait that gave up: the copies land before
         // the CTA is gone)
         cp_async_wait<0>();
+        if (!ok) dn_report(work.control().error);
         __syncwarp();
         for (; ok && lag > 0; lag--)
         {
@@ -896,7 +917,7 @@ __device__ __forceinline__ void dn_body(const Work& work)
             constexpr int NI = decltype(ni_)::value, NJ = decltype(nj_)::value;
             for (int left = run.s1 - run.s0; left > 0; left--)
             {
-                if (!dn_wait(&sh.full[st], phase, abort_flag)) return false;
+                if (!dn_wait(&sh.full[st], phase, fail)) return false;
                 if (NI*NJ > 0)
                 {
                     const double* As = smem + st*STAGE;
@@ -938,7 +959,11 @@ __device__ __forceinline__ void dn_body(const Work& work)
             }
             return true;
         });
-        if (!ok) break;
+        if (!ok)
+        {
+            dn_report(work.control().error);
+            break;
+        }
 
         // the run and its tile again (not kept over the loop above)
         asm volatile("" : "+r"(r));
@@ -1044,9 +1069,9 @@ constexpr int GD_BM = 128, GD_BN = 128;
 template <int AMODE, int BMODE>
 __global__ void __launch_bounds__(dn_threads(1), 1)
 gemm_f64_group_dense_kernel(const GroupDesc* __restrict__ groups, const GroupTile* __restrict__ tiles,
-                            const GroupStart* __restrict__ start, double* __restrict__ partial)
+                            const GroupStart* __restrict__ start, double* __restrict__ partial, const WaitControl ctl)
 {
-    const GroupWork<GD_BM, GD_BN> work{groups, tiles, start, partial};
+    const GroupWork<GD_BM, GD_BN> work{groups, tiles, start, partial, ctl};
     dn_body<2, 4, 4, 4, 6, 1, 1, AMODE, BMODE, false>(work);
 }
 
@@ -1158,6 +1183,18 @@ gemm_f64_fixup(const GemmF64Args p)
     }
 }
 
+// a kernel's shared memory above 48 KB is allowed once per device (asked for before
+// every launch it took 0.3 us of them)
+static void dn_allow(std::atomic<unsigned long long>& done, const void* kern, size_t bytes)
+{
+    int dev = 0;
+    TB_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_relaxed) & bit) return;
+    TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    done |= bit;
+}
+
 template <int WGM, int WGN, int MF, int NF, int STAGES, int LAG, int TEAMS>
 struct DenseTile
 {
@@ -1167,7 +1204,8 @@ struct DenseTile
     {
         auto kern = gemm_f64_dense_kernel<WGM, WGN, MF, NF, STAGES, LAG, TEAMS, AM, BMd, CPLX>;
         constexpr size_t bytes = dn_smem<WGM, WGN, MF, NF, STAGES, TEAMS>();
-        TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        static std::atomic<unsigned long long> done{0};
+        dn_allow(done, (const void*)kern, bytes);
         TimedLaunch t("gemm_f64_kernel", s);
         kern<<<(unsigned)a.grid, dn_threads(TEAMS), bytes, s>>>(a);
         check_launch("gemm_f64_dense_kernel");
@@ -1347,8 +1385,29 @@ void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit)
     else if (tall < t128) a = c;
 }
 
-void gemm_f64_dense_launch(const GemmF64Args& a, cudaStream_t stream)
+// what gemm_f64_dense_inject_wait_timeout has set, and how often
+static std::atomic<int> g_dn_hold{-1}, g_dn_changes{0};
+static std::atomic<unsigned long long> g_dn_wait_ns{DN_WAIT_NS};
+
+// The host's flag: one int of pinned memory that every device can write, so that
+// reading it costs nothing.
+static int* dn_error()
 {
+    static int* const flag = []
+    {
+        int* p = nullptr;
+        TB_CUDA(cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+        *p = 0;
+        return p;
+    }();
+    return flag;
+}
+
+static WaitControl wait_control() { return {dn_error(), g_dn_wait_ns.load(), g_dn_hold.load()}; }
+
+void gemm_f64_dense_launch(GemmF64Args& a, cudaStream_t stream)
+{
+    a.ctl = wait_control();
     if (a.M == 0 || a.N == 0 || a.L == 0 || a.K == 0) return;
     TB_CHECK(a.L <= 65535, TB_ERR_SIZE, "batch extent too large");
     TB_CHECK(((a.M + 63)/64)*((a.N + 63)/64) < (1ll << 31), TB_ERR_SIZE, "tile grid too large");
@@ -1430,7 +1489,7 @@ void gemm_f64_group_dense_launch(const GroupDesc* d_groups, const GroupTile* d_t
     {
         TB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         TimedLaunch t("gemm_f64_group_dense_kernel", s);
-        kern<<<(unsigned)ctas, dn_threads(1), bytes, s>>>(d_groups, d_tiles, d_start, partial);
+        kern<<<(unsigned)ctas, dn_threads(1), bytes, s>>>(d_groups, d_tiles, d_start, partial, wait_control());
         check_launch("gemm_f64_group_dense_kernel");
     };
     switch (modes)
@@ -1450,14 +1509,18 @@ void gemm_f64_group_dense_launch(const GroupDesc* d_groups, const GroupTile* d_t
 
 int gemm_f64_dense_error_flag()
 {
-    int v = 0;
-    cudaMemcpyFromSymbol(&v, g_dn_error, sizeof(int));
-    if (v)
-    {
-        const int zero = 0;
-        cudaMemcpyToSymbol(g_dn_error, &zero, sizeof(int));
-    }
-    return v;
+    // reported once: the next check starts clean
+    return __atomic_exchange_n(dn_error(), 0, __ATOMIC_ACQ_REL);
 }
+
+void gemm_f64_dense_inject_wait_timeout(int stage, double wait_seconds)
+{
+    const unsigned long long ns = wait_seconds > 0.0 ? (unsigned long long)(wait_seconds*1e9) : DN_WAIT_NS;
+    g_dn_hold.store(stage);
+    g_dn_wait_ns.store(ns);
+    g_dn_changes++;
+}
+
+int gemm_f64_dense_control_changes() { return g_dn_changes.load(std::memory_order_relaxed); }
 
 } // namespace tb

@@ -553,8 +553,16 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
 
     if (grouped_use_graphs() && !plan.graph_failed)
     {
+        if (plan.graph && plan.graph_control != gemm_f64_dense_control_changes())
+        {
+            // captured with other arguments (test support): once its launch is over
+            TB_CUDA(cudaEventSynchronize(plan.last_use));
+            cudaGraphExecDestroy(plan.graph);
+            plan.graph = nullptr;
+        }
         if (!plan.graph)
         {
+            plan.graph_control = gemm_f64_dense_control_changes();
             cudaStream_t cs;
             TB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
             cudaGraph_t g;

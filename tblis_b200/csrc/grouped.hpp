@@ -57,6 +57,7 @@ struct GroupedPlan
     int variant = 0;                          // tuned tile configuration
     cudaGraphExec_t graph = nullptr;
     bool graph_failed = false;
+    int graph_control = 0;                    // gemm_f64_dense_control_changes at its capture
     cudaEvent_t last_use = nullptr;
     // the pointers and scalars the pinned descriptors were last built from
     std::vector<const double*> last_ptrs;
