@@ -178,7 +178,8 @@ void* tblis_b200_get_stream(void);
  * TB_ERR_TIMEOUT (6) as the last error when an Ozaki kernel, the dense FP64
  * kernel or a grouped FP64 kernel gave up one of its bounded waits since the
  * previous check (the flags are the process's and are then cleared): part of a
- * result was then not written. */
+ * result was then not written. A contraction of host data, which waits for its
+ * own result, makes the same check for the kernels that it runs. */
 void tblis_b200_synchronize(void);
 
 /* Test support for the failure detection of the Ozaki kernels (no reference

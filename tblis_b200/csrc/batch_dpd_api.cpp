@@ -115,7 +115,7 @@ void run_dpd_mult(const Desc* A, const label_type* idx_A, const Desc* B, const l
         dpd_narrow_blocks(c.lay, cx, wc.as<double>(), reinterpret_cast<float*>(sc.dev), st);
     }
     sc.out(st);
-    if (sa.host || sb.host || sc.host) TB_CUDA(cudaStreamSynchronize(st));
+    if (sa.host || sb.host || sc.host) finish_stream(st, WAITS_DENSE | WAITS_GROUPED);
     scalar_put(C->scalar, type, 1.0);
     C->conj = 0;
     if (report)
@@ -353,7 +353,7 @@ int tblis_b200_dpd_mult_shard(const tblis_b200_dpd_tensor* A, const label_type* 
         DpdMultReport r;
         dpd_mult_shard(a, idx_A, b, idx_B, c, idx_C, alpha, beta, nranks, rank, st, &r);
         sc.out(st);
-        if (sa.host || sb.host || sc.host) TB_CUDA(cudaStreamSynchronize(st));
+        if (sa.host || sb.host || sc.host) finish_stream(st, WAITS_DENSE | WAITS_GROUPED);
         C->scalar.data.d = 1.0;
         C->scalar.type = TYPE_DOUBLE;
         C->conj = 0;

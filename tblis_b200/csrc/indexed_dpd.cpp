@@ -453,7 +453,7 @@ void indexed_dpd_mult(const tblis_b200_indexed_dpd_tensor* A_, const label_type*
 
     if (widened) wc.narrow(C, st);
     sc.out(st);
-    if (sa.staged() || sb.staged() || sc.staged() || widened) TB_CUDA(cudaStreamSynchronize(st));
+    if (sa.staged() || sb.staged() || sc.staged() || widened) finish_stream(st, WAITS_DENSE | WAITS_GROUPED);
     scalar_put(C_->scalar, type, 1.0);
     if (report)
     {

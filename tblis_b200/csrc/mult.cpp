@@ -399,7 +399,7 @@ static void mult_complex(const tblis_config* cfg,
             a.amode = tab->amode; a.bmode = tab->bmode;
             dense_gemm(a, st);
             unstage(sC, st);
-            if (sA.staged || sB.staged || sC.staged) TB_CUDA(cudaStreamSynchronize(st));
+            if (sA.staged || sB.staged || sC.staged) finish_stream(st, WAITS_DENSE);
             C->scalar.type = TYPE_DCOMPLEX;
             C->scalar.data.z[0] = 1.0;
             C->scalar.data.z[1] = 0.0;
@@ -493,7 +493,7 @@ static void mult_complex(const tblis_config* cfg,
         else checked([&] { tblis_tensor_scale(nullptr, cfg, &z, idx_C); });
     }
     unstage(sC, st);
-    if (sA.staged || sB.staged || sC.staged) TB_CUDA(cudaStreamSynchronize(st));
+    if (sA.staged || sB.staged || sC.staged) finish_stream(st, method >= 2 ? WAITS_DENSE | WAITS_OZAKI : WAITS_DENSE);
     C->scalar.type = TYPE_DCOMPLEX;
     C->scalar.data.z[0] = 1.0;
     C->scalar.data.z[1] = 0.0;
@@ -647,7 +647,9 @@ static void mult_widened(const tblis_config* cfg,
         l1_convert<double, float>(static_cast<const double*>(wide[2].data), static_cast<float*>(sc.dptr), rv[2]->s,
                                   st);
     unstage(sc, st);
-    if (sa.staged || sb.staged || sc.staged) TB_CUDA(cudaStreamSynchronize(st));
+    if (sa.staged || sb.staged || sc.staged)
+        finish_stream(st, moduli || (opts && opts->method >= 2) || (cfg && cfg->method >= 2) ? WAITS_DENSE | WAITS_OZAKI
+                                                                                             : WAITS_DENSE);
     if (cx) { C->scalar.data.c[0] = 1.0f; C->scalar.data.c[1] = 0.0f; }
     else C->scalar.data.s = 1.0f;
     C->conj = 0;
@@ -871,7 +873,8 @@ void mult_dispatch(const tblis_config* cfg,
     }
 
     unstage(sc, st);
-    if (sa.staged || sb.staged || sc.staged || sc_back_done) TB_CUDA(cudaStreamSynchronize(st));
+    if (sa.staged || sb.staged || sc.staged || sc_back_done)
+        finish_stream(st, method >= 2 ? WAITS_DENSE | WAITS_OZAKI : WAITS_DENSE);
 
     C->scalar.data.d = 1.0;
     C->scalar.type = TYPE_DOUBLE;

@@ -3,8 +3,8 @@
 Every wait of the kernel is bounded. tblis_b200_dense_inject_wait_timeout keeps one
 ring stage from ever becoming full and shortens the bound, so that the wait for
 it runs out: the CTAs record it, wait for the copies that they issued and return.
-tblis_b200_synchronize reports it once (TB_ERR_TIMEOUT, 6), and the same contraction
-is then right on the same context.
+tblis_b200_synchronize reports it once (TB_ERR_TIMEOUT, 6), a contraction of host
+data reports it itself, and the same contraction is then right on the same context.
 """
 import contextlib
 import ctypes
@@ -12,6 +12,7 @@ import os
 import subprocess
 import sys
 
+import numpy as np
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -53,6 +54,24 @@ def test_wait_runs_out_and_context_recovers(cuda, m, n, k, cplx):
     call()
     tb.synchronize()
     assert bool(((C - A @ B).abs() <= 4 * k * 2.0 ** -53 * (A.abs() @ B.abs())).all())
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_host_data_reports_it(cuda, cplx):
+    import tblis_b200 as tb
+    rng = np.random.default_rng(2)
+    A, B = rng.uniform(-1, 1, (300, 512)), rng.uniform(-1, 1, (512, 260))
+    if cplx:
+        A, B = A + 1j * A[::-1], B - 1j * B[::-1]
+    C = np.zeros((300, 260), dtype=A.dtype)
+    tb.synchronize()
+    with held_stage(tb):
+        with pytest.raises(tb.TblisError) as e:
+            tb.mult(1.0, A, "ik", B, "kj", 0.0, C, "ij")
+        assert e.value.code == 6
+    tb.synchronize()
+    tb.mult(1.0, A, "ik", B, "kj", 0.0, C, "ij")
+    assert (np.abs(C - A @ B) <= 4 * 512 * 2.0 ** -53 * (np.abs(A) @ np.abs(B))).all()
 
 
 GROUPED = r"""
