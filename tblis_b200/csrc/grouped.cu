@@ -413,32 +413,137 @@ static bool ensure_pack(GroupedPlan& plan)
     return true;
 }
 
-static void release_gpart(GroupedPlan& plan)
+// The dense path's workspaces (two tiles per CTA, 39 MB each). They are scratch, so
+// the plans share them (one a plan would be 10 GB for a full plan cache): at most
+// PART_SLOTS per device, an event each that marks its last use. They are counted
+// with the packed panels and freed with the last plan that uses them. The
+// mutex is held over a launch, from the choice of a slot to the record of its event.
+namespace
 {
-    if (!plan.d_gpart) return;
-    cudaFree(plan.d_gpart);
-    plan.d_gpart = nullptr;
-    g_pack_held -= plan.gpart_held;
-    plan.gpart_held = 0;
-}
+struct PartSlot
+{
+    int device;
+    double* ptr;
+    cudaEvent_t used;
+    cudaStream_t stream;          // of the last use
+};
+constexpr int PART_SLOTS = 4;
+std::mutex g_part_mtx;
+std::vector<PartSlot> g_part;
+int g_part_users = 0;
 
-// the dense path's workspace (two tiles per CTA, 39 MB), allocated on first
-// use and counted with the packed panels; false when it would pass the cap or
-// the device has no room
-static bool ensure_gpart(GroupedPlan& plan)
+size_t part_bytes() { return gemm_f64_group_dense_bytes(device_sm_count()); }
+
+// a new slot for the current device, or null without room (mutex held)
+PartSlot* part_add()
 {
-    if (plan.d_gpart || plan.ngcuts == 0) return true;
-    if (plan.gpart_failed) return false;
-    const size_t bytes = gemm_f64_group_dense_bytes(plan.gctas);
-    if (g_pack_held.load() + bytes > pack_cap() || cudaMalloc(&plan.d_gpart, bytes) != cudaSuccess)
+    PartSlot s = {};
+    TB_CUDA(cudaGetDevice(&s.device));
+    const size_t bytes = part_bytes();
+    if (g_pack_held.load() + bytes > pack_cap() || cudaMalloc(&s.ptr, bytes) != cudaSuccess)
     {
         cudaGetLastError();
-        plan.d_gpart = nullptr;
+        return nullptr;
+    }
+    if (cudaEventCreateWithFlags(&s.used, cudaEventDisableTiming) != cudaSuccess)
+    {
+        cudaGetLastError();
+        cudaFree(s.ptr);
+        return nullptr;
+    }
+    g_pack_held += bytes;
+    g_part.push_back(s);
+    return &g_part.back();
+}
+
+bool past(cudaEvent_t e)
+{
+    if (cudaEventQuery(e) == cudaSuccess) return true;
+    cudaGetLastError();                   // not ready: no error for the launches that follow
+    return false;
+}
+bool part_idle(const PartSlot& s) { return past(s.used); }
+
+// The slot for a launch of the plan on st (mutex held): the one its graph holds,
+// unless that is at work for another plan and there is another one; a plan that
+// is itself at work on another stream waits there in any case. Null without room.
+PartSlot* part_pick(const GroupedPlan& plan, cudaStream_t st)
+{
+    int dev = 0;
+    TB_CUDA(cudaGetDevice(&dev));
+    PartSlot *own = nullptr, *any = nullptr, *other = nullptr;
+    int n = 0;
+    for (PartSlot& s : g_part)
+    {
+        if (s.device != dev) continue;
+        n++;
+        any = &s;
+        if (plan.graph && s.ptr == plan.graph_part) own = &s;
+        else if (!other && (s.stream == st || part_idle(s))) other = &s;
+    }
+    if (own && (own->stream == st || part_idle(*own) || !past(plan.last_use))) other = own;
+    if (!other && n < PART_SLOTS) other = part_add();
+    return other ? other : own ? own : any;
+}
+}
+
+// a workspace for the scope's launches on st; ptr null where the plan needs none
+struct PartHold
+{
+    std::unique_lock<std::mutex> lk;
+    PartSlot* slot = nullptr;
+    cudaStream_t st = 0;
+    double* ptr = nullptr;
+    PartHold(const GroupedPlan& plan, int v, cudaStream_t s) : st(s)
+    {
+        if (!gemm_f64_is_dense_variant(v) || plan.ngcuts == 0) return;
+        lk = std::unique_lock<std::mutex>(g_part_mtx);
+        slot = part_pick(plan, s);
+        if (!slot) throw alloc_error("no workspace for the grouped dense path");
+        TB_CUDA(cudaStreamWaitEvent(s, slot->used, 0));
+        ptr = slot->ptr;
+    }
+    ~PartHold()
+    {
+        if (!slot) return;
+        cudaEventRecord(slot->used, st);
+        slot->stream = st;
+    }
+};
+
+static void release_gpart(GroupedPlan& plan)
+{
+    if (!plan.gpart_user) return;
+    plan.gpart_user = false;
+    std::lock_guard<std::mutex> lk(g_part_mtx);
+    if (--g_part_users > 0) return;
+    for (PartSlot& s : g_part)
+    {
+        cudaFree(s.ptr);                  // waits for its last use
+        cudaEventDestroy(s.used);
+        g_pack_held -= part_bytes();
+    }
+    g_part.clear();
+}
+
+// counts the plan among the workspaces' users; false when there is none on this
+// device and no room for one
+static bool ensure_gpart(GroupedPlan& plan)
+{
+    if (plan.gpart_user || plan.ngcuts == 0) return true;
+    if (plan.gpart_failed) return false;
+    int dev = 0;
+    TB_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_part_mtx);
+    bool have = false;
+    for (const PartSlot& s : g_part) have = have || s.device == dev;
+    if (!have && !part_add())
+    {
         plan.gpart_failed = true;
         return false;
     }
-    plan.gpart_held = bytes;
-    g_pack_held += bytes;
+    plan.gpart_user = true;
+    g_part_users++;
     return true;
 }
 
@@ -448,8 +553,9 @@ static bool ensure_variant(GroupedPlan& plan, int v)
     return gemm_f64_is_ws_variant(v) ? ensure_pack(plan) : gemm_f64_is_dense_variant(v) ? ensure_gpart(plan) : true;
 }
 
-// one run of variant v of the plan on the descriptors descs
-static void launch_variant(GroupedPlan& plan, const GroupDesc* descs, int v, cudaStream_t st)
+// one run of variant v of the plan on the descriptors descs; part: a workspace
+// where the variant needs one (PartHold)
+static void launch_variant(GroupedPlan& plan, const GroupDesc* descs, int v, cudaStream_t st, double* part)
 {
     const int ng = (int)plan.groups.size();
     if (gemm_f64_is_ws_variant(v))
@@ -462,7 +568,7 @@ static void launch_variant(GroupedPlan& plan, const GroupDesc* descs, int v, cud
     }
     else if (gemm_f64_is_dense_variant(v))
         gemm_f64_group_dense_launch(descs, plan.d_gtiles, plan.d_gstart, plan.gctas, plan.d_gcuts, plan.ngcuts,
-                                    plan.d_gpart, plan.gmodes, st);
+                                    part, plan.gmodes, st);
     else
         gemm_f64_grouped_launch(descs, variant_tile_begin(plan, v), ng, plan.total_tiles[v - 1], v, st,
                                 plan.d_counter);
@@ -497,10 +603,13 @@ static int autotune(GroupedPlan& plan, const double* const* ptrs, const double* 
     for (int v = 1; v <= gemm_f64_grouped_num_variants(); v++)
     {
         if (!ensure_variant(plan, v)) continue;
-        launch_variant(plan, dd.as<GroupDesc>(), v, st);     // warm-up
-        TB_CUDA(cudaEventRecord(e0, st));
-        launch_variant(plan, dd.as<GroupDesc>(), v, st);
-        TB_CUDA(cudaEventRecord(e1, st));
+        {
+            const PartHold part(plan, v, st);
+            launch_variant(plan, dd.as<GroupDesc>(), v, st, part.ptr);     // warm-up
+            TB_CUDA(cudaEventRecord(e0, st));
+            launch_variant(plan, dd.as<GroupDesc>(), v, st, part.ptr);
+            TB_CUDA(cudaEventRecord(e1, st));
+        }
         TB_CUDA(cudaEventSynchronize(e1));
         float ms = 0;
         TB_CUDA(cudaEventElapsedTime(&ms, e0, e1));
@@ -551,11 +660,13 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
         plan.descs_valid = true;
     }
 
+    const PartHold part(plan, v, st);
     if (grouped_use_graphs() && !plan.graph_failed)
     {
-        if (plan.graph && plan.graph_control != gemm_f64_dense_control_changes())
+        if (plan.graph && (plan.graph_part != part.ptr || plan.graph_control != gemm_f64_dense_control_changes()))
         {
-            // captured with other arguments (test support): once its launch is over
+            // captured with another workspace (or, test support, other waits): once
+            // its launch is over
             TB_CUDA(cudaEventSynchronize(plan.last_use));
             cudaGraphExecDestroy(plan.graph);
             plan.graph = nullptr;
@@ -563,6 +674,7 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
         if (!plan.graph)
         {
             plan.graph_control = gemm_f64_dense_control_changes();
+            plan.graph_part = part.ptr;
             cudaStream_t cs;
             TB_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
             cudaGraph_t g;
@@ -574,7 +686,7 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
             {
                 try
                 {
-                    launch_variant(plan, plan.d_descs, v, cs);
+                    launch_variant(plan, plan.d_descs, v, cs, part.ptr);
                 }
                 catch (const error&) { ok = false; }
             }
@@ -605,7 +717,7 @@ void grouped_run(GroupedPlan& plan, const double* const* ptrs, const double* alp
     {
         TB_CUDA(cudaMemcpyAsync(plan.d_descs, plan.h_descs, plan.groups.size()*sizeof(GroupDesc),
                                 cudaMemcpyHostToDevice, st));
-        launch_variant(plan, plan.d_descs, v, st);
+        launch_variant(plan, plan.d_descs, v, st, part.ptr);
     }
     TB_CUDA(cudaEventRecord(plan.last_use, st));
 }

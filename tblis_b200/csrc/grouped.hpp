@@ -72,16 +72,15 @@ struct GroupedPlan
     double* d_pack = nullptr;
     size_t pack_held = 0;                     // bytes of d_pack counted against the cap
     bool pack_failed = false;
-    // dense path: its tiles, their division over CTAs, and the partial sums'
-    // workspace (allocated on first use)
+    // dense path: its tiles and their division over CTAs (the partial sums' workspace
+    // is shared by all plans, grouped.cu)
     GroupTile* d_gtiles = nullptr;
     GroupStart* d_gstart = nullptr;
     GroupCut* d_gcuts = nullptr;
     int gctas = 0, ngcuts = 0;
     int gmodes = 4;                           // gather directions shared by all groups (2*amode + bmode), or 4
-    double* d_gpart = nullptr;
-    size_t gpart_held = 0;
-    bool gpart_failed = false;
+    bool gpart_user = false, gpart_failed = false;      // counted among the workspaces' users
+    double* graph_part = nullptr;             // the workspace its graph was captured with
     std::string histogram;
     std::vector<std::shared_ptr<GroupedPlan>> parts;   // plans whose groups this one merges (kept alive)
 
