@@ -217,33 +217,45 @@ void scale_all(int type, const DpdLayout& X, void* base, zd beta, bool conj, con
     });
 }
 
-// the index space of a pair of blocks: dimensions of extent 1 dropped, those
-// that continue one another in both tensors merged
-PieceSpec piece_of(const std::vector<i64>& len, const std::vector<i64>& sa, const std::vector<i64>& sb, i64 offa,
-                   i64 offb)
+// The index space of a pair of blocks: dimensions of extent 1 dropped, those
+// that continue one another in both tensors merged. False where the kernels over
+// pieces cannot hold it: more dimensions left than they take, or 2^32 indices and
+// more outside the two fastest dimensions (such tensors go block by block through
+// the dense entry points).
+bool piece_of(const std::vector<i64>& len, const std::vector<i64>& sa, const std::vector<i64>& sb, i64 offa,
+              i64 offb, PieceSpec& p)
 {
-    TB_CHECK(len.size() <= (size_t)L1_MAX_DIM, TB_ERR_SIZE, "DPD: too many dimensions");
-    PieceSpec p;
-    p.offa = offa; p.offb = offb;
-    Strided2& s = p.ab;
+    struct Dim { i64 len, sa, sb; } dims[32];
+    if (len.size() > 32) return false;
+    size_t nd = 0, n = 0;
     for (size_t d = 0; d < len.size(); d++)
     {
         if (len[d] == 1) continue;
-        int at = s.ndim++;
-        for (; at > 0 && s.sa[at - 1] > sa[d]; at--)
-        {
-            s.len[at] = s.len[at - 1]; s.sa[at] = s.sa[at - 1]; s.sb[at] = s.sb[at - 1];
-        }
-        s.len[at] = len[d]; s.sa[at] = sa[d]; s.sb[at] = sb[d];
+        size_t at = nd++;
+        for (; at > 0 && dims[at - 1].sa > sa[d]; at--) dims[at] = dims[at - 1];
+        dims[at] = {len[d], sa[d], sb[d]};
     }
-    int n = 0;
-    for (int d = 0; d < s.ndim; d++)
+    for (size_t i = 0; i < nd; i++)
     {
-        if (n > 0 && s.sa[d] == s.sa[n - 1]*s.len[n - 1] && s.sb[d] == s.sb[n - 1]*s.len[n - 1]) s.len[n - 1] *= s.len[d];
-        else { s.len[n] = s.len[d]; s.sa[n] = s.sa[d]; s.sb[n] = s.sb[d]; n++; }
+        const Dim d = dims[i];
+        if (n > 0 && d.sa == dims[n - 1].sa*dims[n - 1].len && d.sb == dims[n - 1].sb*dims[n - 1].len)
+            dims[n - 1].len *= d.len;
+        else dims[n++] = d;
     }
-    s.ndim = n;
-    return p;
+    if (n > (size_t)L1_MAX_DIM) return false;
+    p.offa = offa; p.offb = offb;
+    Strided2& s = p.ab;
+    s.ndim = (int)n;
+    size_t fast = 0;                     // B's fastest dimension (A's is the first)
+    for (size_t d = 0; d < n; d++)
+    {
+        s.len[d] = dims[d].len; s.sa[d] = dims[d].sa; s.sb[d] = dims[d].sb;
+        if (std::llabs(s.sb[d]) < std::llabs(s.sb[fast])) fast = d;
+    }
+    i64 outer = 1;
+    for (size_t d = 1; d < n; d++)
+        if (d != fast) outer *= s.len[d];
+    return outer < ((i64)1 << 32);
 }
 
 // block irr of X: its extents and strides into len and stride (in X's dimension
@@ -329,6 +341,7 @@ void dpd_add_dev_t(int type, zd alpha, const DpdLayout& A, const void* a, const 
         // (a launch per block cost 2 us each, 512 of them for 8 irreps)
         std::vector<PieceSpec> pieces;
         std::vector<i64> la, sa, sb(A.ndim);
+        bool fit = true;
         B.for_each_block([&](const std::vector<unsigned>& irrB, const std::vector<i64>&, const std::vector<i64>& bs,
                              i64 offb)
         {
@@ -336,18 +349,22 @@ void dpd_add_dev_t(int type, zd alpha, const DpdLayout& A, const void* a, const 
             for (size_t i = 0; i < AB.size(); i++) irrA[pA_AB[i]] = irrB[pB_AB[i]];
             if (!block_at(A, irrA, la, sa, offa)) return;
             for (size_t i = 0; i < AB.size(); i++) sb[pA_AB[i]] = bs[pB_AB[i]];
-            pieces.push_back(piece_of(la, sa, sb, offa, offb));
+            pieces.emplace_back();
+            fit = piece_of(la, sa, sb, offa, offb, pieces.back()) && fit;
         });
-        with_element(type, [&](auto t)
+        if (fit)
         {
-            typedef decltype(t) T;
-            T al, be;
-            element(alpha, al);
-            element(beta, be);
-            l1_add_pieces<T>(static_cast<const T*>(a), static_cast<T*>(b), pieces, al, be, current_stream(), conj_a,
-                             conj_b);
-        });
-        return;
+            with_element(type, [&](auto t)
+            {
+                typedef decltype(t) T;
+                T al, be;
+                element(alpha, al);
+                element(beta, be);
+                l1_add_pieces<T>(static_cast<const T*>(a), static_cast<T*>(b), pieces, al, be, current_stream(), conj_a,
+                                 conj_b);
+            });
+            return;
+        }
     }
     B.for_each_block([&](const std::vector<unsigned>& irrB, const std::vector<i64>&, const std::vector<i64>&, i64)
     {
@@ -398,9 +415,24 @@ zd dpd_dot_dev_t(int type, const DpdLayout& A, const void* a, const std::string&
     const auto pB = positions(iA, iB);
     std::vector<unsigned> irrB(B.ndim), all(A.ndim), irrA(A.ndim, 0);
     for (unsigned d = 0; d < A.ndim; d++) all[d] = d;
-    if (repeats(iA) || repeats(iB))
+    // every stored block pair in one launch, the sum in double precision
+    std::vector<PieceSpec> pieces;
+    std::vector<i64> la, sa, lb, sb, sbA(A.ndim);
+    bool fit = !repeats(iA) && !repeats(iB);
+    if (fit)
+        for_each_combo(all, A.irrep, A.nirrep, irrA, [&]
+        {
+            for (unsigned d = 0; d < A.ndim; d++) irrB[pB[d]] = irrA[d];
+            i64 offa = 0, offb = 0;
+            if (!block_at(A, irrA, la, sa, offa) || !block_at(B, irrB, lb, sb, offb)) return;
+            for (unsigned d = 0; d < A.ndim; d++) sbA[d] = sb[pB[d]];
+            pieces.emplace_back();
+            fit = piece_of(la, sa, sbA, offa, offb, pieces.back()) && fit;
+        });
+    if (!fit)
     {
-        // diagonals: block by block through the dense entry point
+        // diagonals, and what a launch cannot hold: block by block through the dense
+        // entry point
         for_each_combo(all, A.irrep, A.nirrep, irrA, [&]
         {
             for (unsigned d = 0; d < A.ndim; d++) irrB[pB[d]] = irrA[d];
@@ -413,17 +445,6 @@ zd dpd_dot_dev_t(int type, const DpdLayout& A, const void* a, const std::string&
         });
         return sum;
     }
-    // every stored block pair in one launch, the sum in double precision
-    std::vector<PieceSpec> pieces;
-    std::vector<i64> la, sa, lb, sb, sbA(A.ndim);
-    for_each_combo(all, A.irrep, A.nirrep, irrA, [&]
-    {
-        for (unsigned d = 0; d < A.ndim; d++) irrB[pB[d]] = irrA[d];
-        i64 offa = 0, offb = 0;
-        if (!block_at(A, irrA, la, sa, offa) || !block_at(B, irrB, lb, sb, offb)) return;
-        for (unsigned d = 0; d < A.ndim; d++) sbA[d] = sb[pB[d]];
-        pieces.push_back(piece_of(la, sa, sbA, offa, offb));
-    });
     cudaStream_t st = current_stream();
     with_element(type, [&](auto t)
     {
@@ -460,26 +481,32 @@ void dpd_reduce_dev_t(int type, int op, const DpdLayout& A, const void* a, const
         // sums: every stored block in one launch, in double precision
         std::vector<PieceSpec> pieces;
         std::vector<i64> la, sa;
+        bool fit = true;
         for_each_combo(all, A.irrep, A.nirrep, irr, [&]
         {
             i64 off = 0;
-            if (block_at(A, irr, la, sa, off)) pieces.push_back(piece_of(la, sa, sa, off, off));
+            if (!block_at(A, irr, la, sa, off)) return;
+            pieces.emplace_back();
+            fit = piece_of(la, sa, sa, off, off, pieces.back()) && fit;
         });
         cudaStream_t st = current_stream();
-        with_element(type, [&](auto t)
+        if (fit)
         {
-            typedef decltype(t) T;
-            typedef typename SumOf<T>::type Acc;
-            dbuf out(sizeof(Acc), st);
-            l1_sum_pieces<T, Acc>(op, static_cast<const T*>(a), pieces, out.as<Acc>(), st);
-            Acc v;
-            TB_CUDA(cudaMemcpyAsync(&v, out.ptr, sizeof(Acc), cudaMemcpyDeviceToHost, st));
-            TB_CUDA(cudaStreamSynchronize(st));
-            acc = to_zd(v);
-        });
-        result = op == REDUCE_NORM_2 ? zd(std::sqrt(acc.real())) : acc;
-        idx = -1;
-        return;
+            with_element(type, [&](auto t)
+            {
+                typedef decltype(t) T;
+                typedef typename SumOf<T>::type Acc;
+                dbuf out(sizeof(Acc), st);
+                l1_sum_pieces<T, Acc>(op, static_cast<const T*>(a), pieces, out.as<Acc>(), st);
+                Acc v;
+                TB_CUDA(cudaMemcpyAsync(&v, out.ptr, sizeof(Acc), cudaMemcpyDeviceToHost, st));
+                TB_CUDA(cudaStreamSynchronize(st));
+                acc = to_zd(v);
+            });
+            result = op == REDUCE_NORM_2 ? zd(std::sqrt(acc.real())) : acc;
+            idx = -1;
+            return;
+        }
     }
     for_each_combo(all, A.irrep, A.nirrep, irr, [&]
     {
