@@ -221,7 +221,7 @@ __device__ __forceinline__ void pc_copy(T* to, const T* from)
 }
 
 // OP 0: B = alpha*op(A) (B not read), 1: B = alpha*op(A) + beta*op(B),
-// 2: sum of op(A)*op(B), 3: sum of red_val(op, A)
+// 2: sum of op(A)*op(B), 3: sum of red_val(op, A), both in at least double precision
 template <typename T, int OP>
 __global__ void __launch_bounds__(PC_THREADS, pc_blocks<OP>())
 k_pieces(const T* __restrict__ A, T* __restrict__ B, const Piece one, const Piece* __restrict__ many, int npieces,
@@ -298,7 +298,7 @@ k_pieces(const T* __restrict__ A, T* __restrict__ B, const Piece one, const Piec
                 if (!(m >> u & 1)) continue;
                 const T x = buf[b][w.at[u] >> 8];
                 if (OP == 2) acc += pc_widen(cj(x, conj_a))*pc_widen(cj(y[u], conj_b));
-                else if (OP == 3) acc += pc_widen(red_val(red_op, x));
+                else if (OP == 3) acc += red_val(red_op, pc_widen(x));     // float squares leave its range
                 else
                 {
                     const T v = alpha*cj(x, conj_a);
