@@ -261,6 +261,11 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
                            char* idx_AB, char* idx_AC, char* idx_BC, char* idx_ABC,
                            int64_t* mnkl);
 
+/* Elements that the last large float contraction on this device left to FP64
+ * after verification (-1 on error; for tests, waits for the device): each was
+ * recomputed, or, where they were more than one in 2500 (and 256), FP64 did all of C. */
+int64_t tblis_b200_verified_listed(void);
+
 /* Test support: device allocations above `bytes` (0: no limit) fail as if there
  * were no room, so that the ways taken without their scratch can be run. */
 void tblis_b200_limit_allocations(size_t bytes);

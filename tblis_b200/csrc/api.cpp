@@ -625,6 +625,13 @@ int tblis_b200_mult_groups(const tblis_tensor* A, const label_type* idx_A,
     });
 }
 
+int64_t tblis_b200_verified_listed(void)
+{
+    int64_t n = -1;
+    guarded([&] { ensure_device(); n = ozaki_verified_listed(); });
+    return n;
+}
+
 void tblis_b200_limit_allocations(size_t bytes) { g_alloc_limit.store(bytes ? bytes : SIZE_MAX); }
 
 int tblis_b200_dense_plan(int64_t m, int64_t n, int64_t k, int64_t l, int complex_elements, int read_c, int sms,

@@ -1328,6 +1328,9 @@ __global__ void oz_inexact_bounds(const int* n, const double* ss, i64 rows, doub
                                : k > 0.0 ? 0.5*sqrt(k)*norm*(1.0 + 0x1p-20) + 0.25*k : 0.0;
 }
 
+// elements that the last verified run left to FP64 (tests)
+__device__ unsigned g_oz_listed = 0;
+
 // C elements from the list in FP64, a warp each; nothing when the list ran over.
 // A and B hold floats.
 __global__ void __launch_bounds__(256)
@@ -1336,6 +1339,7 @@ oz_recompute(const float* A, const float* B, double* C, const i64* a_m, const i6
              double alpha, const unsigned* count, unsigned cap, const unsigned long long* list)
 {
     const unsigned n = *count;
+    if (blockIdx.x == 0 && threadIdx.x == 0) g_oz_listed = n;
     if (n > cap) return;
     const int lane = threadIdx.x & 31;
     for (unsigned e = (blockIdx.x*blockDim.x + threadIdx.x) >> 5; e < n; e += (gridDim.x*blockDim.x) >> 5)
@@ -2132,6 +2136,13 @@ void ozaki_end(OzakiJob& j, cudaStream_t st, bool stats_ready)
     for (int d = 2; d < OZ_SMAX + 2; d++)
         g.w[d - 2] = j.single ? 1.0 : diagonal_weight(kind, d);   // a single pass: weight 1
     gemm_dispatch(kind, S, g, st);
+}
+
+i64 ozaki_verified_listed()
+{
+    unsigned n = 0;
+    TB_CUDA(cudaMemcpyFromSymbol(&n, g_oz_listed, sizeof(n)));
+    return n;
 }
 
 int ozaki_verified_moduli() { return VERIFIED_MODULI; }

@@ -42,6 +42,7 @@ OzakiResult ozaki_mult(const GemmView& v, const double* A, const double* B, doub
 // pays: a modelled time below the FP64 contraction's.
 bool ozaki_verified_pays(const GemmView& v);
 int ozaki_verified_moduli();
+i64 ozaki_verified_listed();       // gate's number of the last run on this device (tests; synchronises)
 double ozaki_verified_error();     // relative, of an element that is not recomputed
 void ozaki_verified(const GemmView& v, const float* A, const float* B, double* C, double alpha, cudaStream_t st,
                     dbuf& gate, unsigned& gate_above);
