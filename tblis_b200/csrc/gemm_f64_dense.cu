@@ -1113,7 +1113,11 @@ __global__ void __launch_bounds__(DN_CT*GROUPS)
 gemm_f64_fixup(const GemmF64Args p)
 {
     constexpr int BM = WGM*MF*16, BN = WGN*NF*8;
-    const bool off = p.gate && *p.gate <= p.gate_above;
+    if (p.gate && *p.gate <= p.gate_above)
+    {
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // as below
+        return;
+    }
     __shared__ double sums[GROUPS][2][DN_CT];
     const int tc = threadIdx.x % DN_CT, grp = threadIdx.x/DN_CT;
     const int lane = tc & 31;
@@ -1133,7 +1137,7 @@ gemm_f64_fixup(const GemmF64Args p)
     // all return could end, and the next kernel start, before that kernel's writes
     // to C are visible.
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if (off || c1 - c0 == 1) return;                 // one CTA did the whole tile
+    if (c1 - c0 == 1) return;                        // one CTA did the whole tile
     for (int e = blockIdx.y; e < MF*NF*2; e += gridDim.y)
     {
         // elements 2e and 2e + 1: neighbouring columns of one row (complex: the
