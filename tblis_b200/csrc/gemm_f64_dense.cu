@@ -619,17 +619,19 @@ __device__ __forceinline__ double flip(double x, unsigned mask)
 // alpha*x + beta*op(c) over a complex element of C (beta == 0: c is not read). A
 // factor of zero leaves its product out, so that a real alpha or beta scales
 // each part by itself: 0 times an infinite part would be NaN in the other one.
+// REAL: both are real (tested an element at a time, 4000 x 4000 x 8 took 143 us, not 128).
+template <bool REAL>
 __device__ __forceinline__ void update_z(const GemmF64Args& p, double* dst, double re, double im)
 {
     double vr, vi;
-    if (p.alpha_im == 0.0) { vr = p.alpha*re; vi = p.alpha*im; }
+    if (REAL || p.alpha_im == 0.0) { vr = p.alpha*re; vi = p.alpha*im; }
     else if (p.alpha == 0.0) { vr = -p.alpha_im*im; vi = p.alpha_im*re; }
     else { vr = p.alpha*re - p.alpha_im*im; vi = p.alpha*im + p.alpha_im*re; }
-    if (p.beta != 0.0 || p.beta_im != 0.0)
+    if (p.beta != 0.0 || (!REAL && p.beta_im != 0.0))
     {
         const double cr = dst[0], ci = p.conj_c ? -dst[1] : dst[1];
-        if (p.beta != 0.0) { vr += p.beta*cr; vi += p.beta*ci; }
-        if (p.beta_im != 0.0) { vr -= p.beta_im*ci; vi += p.beta_im*cr; }
+        if (REAL || p.beta != 0.0) { vr += p.beta*cr; vi += p.beta*ci; }
+        if (!REAL && p.beta_im != 0.0) { vr -= p.beta_im*ci; vi += p.beta_im*cr; }
     }
     *reinterpret_cast<double2*>(dst) = make_double2(vr, vi);
 }
@@ -995,15 +997,22 @@ __device__ __forceinline__ void dn_body(const Work& work)
             if (CPLX)
             {
                 double* C0 = C + 2*__ldg(c.c_n + (t.n0 + n)/2);
-                #pragma unroll
-                for (int i = 0; i < MF; i++)
+                const GemmF64Args& p = work.args();
+                auto rows = [&](auto real)
+                {
                     #pragma unroll
-                    for (int hh = 0; hh < 2; hh++)
-                    {
-                        const int m = (i*WGM + wm)*16 + 8*hh + fr;
-                        if (m < t.mrem)
-                            update_z(work.args(), C0 + 2*__ldg(c.c_m + t.m0 + m), acc[i][j][2*hh], acc[i][j][2*hh + 1]);
-                    }
+                    for (int i = 0; i < MF; i++)
+                        #pragma unroll
+                        for (int hh = 0; hh < 2; hh++)
+                        {
+                            const int m = (i*WGM + wm)*16 + 8*hh + fr;
+                            if (m < t.mrem)
+                                update_z<decltype(real)::value>(p, C0 + 2*__ldg(c.c_m + t.m0 + m), acc[i][j][2*hh],
+                                                                acc[i][j][2*hh + 1]);
+                        }
+                };
+                if (p.alpha_im == 0.0 && p.beta_im == 0.0) rows(std::true_type());
+                else rows(std::false_type());
                 continue;
             }
             const bool two = n + 1 < t.nrem;
@@ -1171,7 +1180,7 @@ gemm_f64_fixup(const GemmF64Args p)
         if (!in) continue;
         if (CPLX)
         {
-            update_z(p, p.C + 2*(p.c_l[t.l] + __ldg(p.c_m + t.m0 + m) + __ldg(p.c_n + (t.n0 + n)/2)), s0, s1);
+            update_z<false>(p, p.C + 2*(p.c_l[t.l] + __ldg(p.c_m + t.m0 + m) + __ldg(p.c_n + (t.n0 + n)/2)), s0, s1);
             continue;
         }
         double* Cm = p.C + p.c_l[t.l] + __ldg(p.c_m + t.m0 + m);
