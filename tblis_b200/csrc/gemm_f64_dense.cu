@@ -1295,7 +1295,7 @@ double split_work(GemmF64Args& a, int sms, size_t ws_limit)
     // 4000 with k 16 64 and 64, k 64 109 and 135, k 500 557 and 559; 2000 x 2000 with k
     // 200 77 and 98; 40000 x 100 with k 500 217 and 190. (2000 cycles a tile and 26000 a
     // cut, as assumed before, cut 2000 x 2000 from k 200 on.)
-    constexpr double kOut = 9, kRun = 700, kFixup = 9000, kChip = 1700, kUnit = 32;
+    constexpr double kOut = 9, kRun = 700, kFixup = 12000, kChip = 1700, kUnit = 32;
     constexpr size_t kSlot = (size_t)T::BM*T::BN*sizeof(double);
     const i64 N = a.cplx ? 2*a.N : a.N;
     const i64 fm = a.M/T::BM, fn = N/T::BN, L = a.L;
@@ -1394,7 +1394,11 @@ void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit)
     a.tile = 0; b.tile = 1; c.tile = 2;
     const double t128 = split_work<Tile128>(a, sms, ws_limit), t64 = split_work<Tile64>(b, sms, ws_limit);
     const double tall = per*a.N <= TileTall::BN ? split_work<TileTall>(c, sms, ws_limit) : 1e300;
-    if (t64 < t128 && t64 <= tall) a = b;
+    // equal steps of a thin real GEMM: 128 x 32 where it fills more than 32 rows (us, 64 x
+    // 64 and 128 x 32 tiles: 100 of 20 x 200 x 1000 103 and 87, 30000 of 5 x 40 x 40 506
+    // and 457; 10000 of 32 x 32 x 40 171 and 217, 30000 complex of 5 x 40 x 3 574 and 683)
+    const double bias = a.M > 32 && !a.cplx ? 1.03 : 1.0;
+    if (t64 < t128 && t64*bias <= tall) a = b;
     else if (tall < t128) a = c;
 }
 

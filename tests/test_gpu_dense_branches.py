@@ -29,7 +29,7 @@ CASES = [
     (2000, 1301, 300, True, T128, False, True, True),
     (1301, 601, 1100, True, T128, False, True, False),
     (30000, 20, 60, True, T128, False, False, None),
-    (700, 700, 300, True, T64, False, True, False),
+    (400, 400, 300, True, T64, False, True, False),
     (1300, 1100, 48, True, T64, False, False, None),
     (2500, 12, 900, True, TALL, False, True, False),
     (12, 2500, 900, True, TALL, True, True, False),
