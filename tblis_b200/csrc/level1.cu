@@ -19,7 +19,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
-#include <cstring>
 
 namespace tb
 {
@@ -662,7 +661,7 @@ static bool make_piece(const PieceSpec& sp, Piece& c)
     for (int d = 0; d < ab.ndim; d++)
     {
         if (d == pa || d == pb || ab.len[d] == 1) continue;
-        c.d[c.nd] = PieceDim{ab.sa[d], ab.sb[d], (unsigned)ab.len[d], 0};
+        c.len[c.nd] = ab.len[d]; c.sa[c.nd] = ab.sa[d]; c.sb[c.nd] = ab.sb[d];
         c.nd++;
         outer *= ab.len[d];
     }
@@ -679,23 +678,6 @@ template <int OP>
 static unsigned pieces_grid(i64 tiles)
 {
     return (unsigned)std::min<i64>(tiles, (i64)device_sm_count()*pc_blocks<OP>());
-}
-
-// one launch, over the pieces of a table or over one alone
-template <typename T, int OP>
-static void pieces_go(unsigned grid, const T* A, T* B, const Piece& one, const Piece* many, int np, unsigned nt, T alpha,
-                      T beta, bool conj_a, bool conj_b, int red_op, typename PcAcc<T>::type* partial, cudaStream_t st)
-{
-    if (many || one.nd <= PC_FEW_DIMS)
-    {
-        PieceFew few;
-        memcpy(&few, &one, sizeof(few));
-        k_pieces<T, OP, PieceFew><<<grid, PC_THREADS, 0, st>>>(A, B, few, many, np, nt, alpha, beta, conj_a, conj_b, red_op,
-                                                               partial);
-    }
-    else
-        k_pieces<T, OP, Piece><<<grid, PC_THREADS, 0, st>>>(A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, red_op,
-                                                            partial);
 }
 
 template <typename T>
@@ -735,11 +717,11 @@ static void pieces_launch(int op, const T* A, T* B, const PieceSpec* specs, size
             alone.first = 0;
             const i64 n = pc_tiles<T>(alone, size);
             if (op == 0)
-                pieces_go<T, 0>(pieces_grid<0>(n), A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0,
-                                nullptr, st);
+                k_pieces<T, 0><<<pieces_grid<0>(n), PC_THREADS, 0, st>>>(
+                    A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0, nullptr);
             else
-                pieces_go<T, 1>(pieces_grid<1>(n), A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0,
-                                nullptr, st);
+                k_pieces<T, 1><<<pieces_grid<1>(n), PC_THREADS, 0, st>>>(
+                    A, B, alone, nullptr, 1, (unsigned)n, alpha, beta, conj_a, conj_b, 0, nullptr);
         }
         check_launch("k_pieces");
         return;
@@ -753,13 +735,17 @@ static void pieces_launch(int op, const T* A, T* B, const PieceSpec* specs, size
     }
     const unsigned nt = (unsigned)tiles;
     if (op == 0)
-        pieces_go<T, 0>(pieces_grid<0>(tiles), A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr, st);
+        k_pieces<T, 0><<<pieces_grid<0>(tiles), PC_THREADS, 0, st>>>(
+            A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr);
     else if (op == 1)
-        pieces_go<T, 1>(pieces_grid<1>(tiles), A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr, st);
+        k_pieces<T, 1><<<pieces_grid<1>(tiles), PC_THREADS, 0, st>>>(
+            A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, nullptr);
     else if (op == 2)
-        pieces_go<T, 2>(kPieceBlocks, A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0, partial, st);
+        k_pieces<T, 2><<<kPieceBlocks, PC_THREADS, 0, st>>>(A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, 0,
+                                                            partial);
     else
-        pieces_go<T, 3>(kPieceBlocks, A, B, one, many, np, nt, alpha, beta, conj_a, conj_b, red_op, partial, st);
+        k_pieces<T, 3><<<kPieceBlocks, PC_THREADS, 0, st>>>(A, B, one, many, np, nt, alpha, beta, conj_a, conj_b,
+                                                            red_op, partial);
     check_launch("k_pieces");
 }
 

@@ -28,22 +28,15 @@
 // leave a tenth of the fetched sectors unused and the last CTAs a sixth behind.
 #pragma once
 
-struct PieceDim { i64 sa, sb; unsigned len, unused; };
-template <int D>
-struct PieceOf
+struct Piece
 {
     i64 np, nq, sap, saq, sbp, sbq;          // extents and strides (elements) of p and q
     i64 offa, offb;
+    int nd;                                  // outer dimensions
+    i64 len[L1_MAX_DIM], sa[L1_MAX_DIM], sb[L1_MAX_DIM];
     unsigned outer, tiles_p, tiles_q, first; // tiles: p fastest, then q, then outer; first tile of the piece
     int tp, tq, tr, turn;                    // turn: q present, through shared memory
-    int nd;                                  // outer dimensions
-    PieceDim d[D];
 };
-typedef PieceOf<L1_MAX_DIM> Piece;
-// A single piece is a kernel argument, most often with few outer dimensions: an
-// argument block above 352 bytes costs the host time at every launch.
-constexpr int PC_FEW_DIMS = 5;
-typedef PieceOf<PC_FEW_DIMS> PieceFew;       // the beginning of a Piece
 
 constexpr int PC_THREADS = 256;
 template <int OP> constexpr int pc_blocks() { return OP == 1 || OP == 2 ? 2 : 3; }  // CTAs an SM (B's elements in registers too)
@@ -151,9 +144,9 @@ __device__ __forceinline__ void pc_setup(const Piece& c, unsigned tile, PcTile& 
         i64 oa = c.offa + p0*c.sap + q0*c.saq, ob = c.offb + p0*c.sbp + q0*c.sbq;
         for (int d = 0; d < c.nd; d++)
         {
-            const unsigned ld = c.d[d].len, qq = o/ld, i = o - qq*ld;
-            oa += (i64)i*c.d[d].sa;
-            ob += (i64)i*c.d[d].sb;
+            const unsigned ld = (unsigned)c.len[d], qq = o/ld, i = o - qq*ld;
+            oa += (i64)i*c.sa[d];
+            ob += (i64)i*c.sb[d];
             o = qq;
         }
         t.oa[r] = oa;
@@ -229,9 +222,9 @@ __device__ __forceinline__ void pc_copy(T* to, const T* from)
 
 // OP 0: B = alpha*op(A) (B not read), 1: B = alpha*op(A) + beta*op(B),
 // 2: sum of op(A)*op(B), 3: sum of red_val(op, A), both in at least double precision
-template <typename T, int OP, typename One>
+template <typename T, int OP>
 __global__ void __launch_bounds__(PC_THREADS, pc_blocks<OP>())
-k_pieces(const T* __restrict__ A, T* __restrict__ B, const __grid_constant__ One one, const Piece* __restrict__ many, int npieces,
+k_pieces(const T* __restrict__ A, T* __restrict__ B, const Piece one, const Piece* __restrict__ many, int npieces,
          unsigned ntiles, T alpha, T beta, bool conj_a, bool conj_b, int red_op, typename PcAcc<T>::type* partial)
 {
     constexpr int NE = pc_ne<T>();
@@ -260,8 +253,7 @@ k_pieces(const T* __restrict__ A, T* __restrict__ B, const __grid_constant__ One
     {
         // the piece into shared memory (the last tile's readers are past their barrier)
         const int* src = many ? reinterpret_cast<const int*>(many + pi) : reinterpret_cast<const int*>(&one);
-        const int words = many ? (int)(sizeof(Piece)/4) : (int)(sizeof(One)/4);
-        for (int w = threadIdx.x; w < words; w += PC_THREADS) reinterpret_cast<int*>(&held)[w] = src[w];
+        for (int w = threadIdx.x; w < (int)(sizeof(Piece)/4); w += PC_THREADS) reinterpret_cast<int*>(&held)[w] = src[w];
         __syncthreads();
         const unsigned first = c.first, end = pi + 1 < npieces ? min(t1, many[pi + 1].first) : t1;
         pc_spots(c, false, c.sap, c.saq, wa);
