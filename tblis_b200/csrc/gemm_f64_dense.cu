@@ -16,9 +16,10 @@
 // ring of 16-wide k stages whose mbarriers they alone feed, and eight consumer
 // warps (two per SM sub-core, so one's fragment loads hide behind the other's
 // MMAs) release each stage as soon as its fragments are in registers. No
-// barrier spans the CTA after the start. Measured: 7680^3 in 27.4 ms (30.4 before,
-// cuBLAS 25.3), 97 x 97 x 93217 in 102 us (283), 3007^3 with permuted operands in
-// 1.95 ms (2.97), complex 1728^3 in 1.38 ms (2.58 as four real contractions).
+// barrier spans the CTA after the start. Measured against the 64 x 64 kernel: 7680^3
+// in 26.6 ms (30.2; cuBLAS 25.3), 97 x 97 x 93217 in 100 us (283), 3007^3 with permuted
+// operands in 1.77 ms (2.88; 1.92 and 2.97 with the copy of a residual before it),
+// complex 1728^3 in 1.31 ms (2.50 as four real contractions).
 //
 // Fragments are dealt to the warps cyclically (16-row fragment f of the tile
 // to row-warp f % WGM, 8-column fragment g to column-warp g % WGN), and
