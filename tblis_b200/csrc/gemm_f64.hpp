@@ -168,6 +168,7 @@ void gemm_f64_launch(GemmF64Args a, cudaStream_t stream);
 // runs it.
 void gemm_f64_dense_plan(GemmF64Args& a, int sms, size_t ws_limit);
 void gemm_f64_dense_launch(GemmF64Args& a, cudaStream_t stream);
+void gemm_f64_dense_prepare();             // the launches' one allocation, made once
 // nonzero once after a dense kernel (also a grouped one) gave up a wait
 int gemm_f64_dense_error_flag();
 // test support: ring stage `stage` never fills (-1: none) and waits give up after wait_seconds (0: 2 s)

@@ -1421,6 +1421,8 @@ static int* dn_error()
     return flag;
 }
 
+void gemm_f64_dense_prepare() { dn_error(); }
+
 static WaitControl wait_control() { return {dn_error(), g_dn_wait_ns.load(), g_dn_hold.load()}; }
 
 void gemm_f64_dense_launch(GemmF64Args& a, cudaStream_t stream)

@@ -1,5 +1,6 @@
 // planner.cpp -- see planner.hpp. Paths cited are relative to the TBLIS tree.
 #include "planner.hpp"
+#include "gemm_f64.hpp"
 
 #include <algorithm>
 #include <cstring>
@@ -559,6 +560,9 @@ std::shared_ptr<GemmTables> gemm_tables(const GemmView& v, i64 BM, i64 BN, i64 B
     fill_block_scatter(v.lenL, v.bL, 1, 0, v.l, b_l, bs.data(), false);
     fill_block_scatter(v.lenL, v.cL, 1, 0, v.l, c_l, bs.data(), false);
 
+    // what else a later call of this shape would allocate: with its tables cached it
+    // can be captured
+    gemm_f64_dense_prepare();
     auto t = std::make_shared<GemmTables>();
     t->amode = amode;
     t->bmode = bmode;

@@ -35,3 +35,35 @@ def test_against_numpy(cuda, l, m, n, k, beta):
         want = 1.5 * np.einsum(spec, T[0], T[1], optimize=True) + (beta * T[2] if beta else 0.0)
         size = 1.5 * np.einsum(spec, abs(T[0]), abs(T[1]), optimize=True) + abs(beta * T[2])
         assert (np.abs(D[2].cpu().numpy() - want) <= (k + 4) * 2.0 ** -52 * size).all(), (ia, ib, ic)
+
+
+CAPTURED = r"""
+import torch
+import tblis_b200 as tb
+A, B, C = (torch.rand(*s, dtype=torch.float64, device="cuda") for s in ((800, 8), (8, 800), (800, 800)))
+s = torch.cuda.Stream()
+tb.set_stream(s.cuda_stream)
+with torch.cuda.stream(s):
+    tb.mult(1.0, A, "ik", B, "kj", 0.0, C, "ij")       # small CTAs; the shape's tables are cached from here on
+torch.cuda.synchronize()
+C.fill_(1.0)
+torch.cuda.synchronize()
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g, stream=s):
+    tb.mult(1.0, A, "ik", B, "kj", 0.5, C, "ij")       # the process's first call of the dense kernel
+g.replay()
+torch.cuda.synchronize()
+assert bool(((C - (A @ B + 0.5)).abs() <= 12 * 2.0 ** -52 * (A @ B + 0.5)).all())
+print("captured ok")
+"""
+
+
+def test_first_dense_call_under_capture(cuda):
+    """With the shape's tables cached a call is capturable, whichever kernel it takes."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    p = subprocess.run([sys.executable, "-c", CAPTURED], cwd=root, env=dict(os.environ, PYTHONPATH=root),
+                       capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0 and "captured ok" in p.stdout, p.stdout[-500:] + p.stderr[-1500:]
