@@ -1019,45 +1019,63 @@ __device__ __forceinline__ void dn_body(const Work& work)
             const bool two = n + 1 < t.nrem;
             double* C0 = C + __ldg(c.c_n + t.n0 + n);
             double* C1 = C + (two ? __ldg(c.c_n + t.n0 + n + 1) : 0);
-            // The old values of a fragment's two rows are loaded before the first of
-            // them is stored: one by one, each load behind the store before it, the
-            // update took a memory latency an element. (Registers for more
-            // fragments at once spill.)
+            // The old values of IB fragments' rows are loaded before the first of them is
+            // stored: one by one, each load behind the store before it, the update
+            // took a memory latency an element, and a load from a sector just stored to
+            // waits for the store. With small accumulators all rows of a column pair
+            // go together (656^3 with permuted operands and beta: 51 us, 59 a fragment at
+            // a time); with 128 x 128 tiles the registers for more would spill. Past L1,
+            // which has no room for that many lines beside the stages.
+            constexpr int IB = MF*NF > 4 ? 1 : MF;
             #pragma unroll
-            for (int i = 0; i < MF; i++)
+            for (int i0 = 0; i0 < MF; i0 += IB)
             {
-                const int m = (i*WGM + wm)*16 + fr;
-                const bool in[2] = {m < t.mrem, m + 8 < t.mrem};
-                i64 ro[2];
-                double v[2][2];
+                bool in[IB][2];
+                i64 ro[IB][2];
+                double v[IB][2][2];
                 #pragma unroll
-                for (int hh = 0; hh < 2; hh++) ro[hh] = in[hh] ? __ldg(c.c_m + t.m0 + m + 8*hh) : 0;
-                if (beta != 0.0)
-                {
+                for (int x = 0; x < IB; x++)
                     #pragma unroll
                     for (int hh = 0; hh < 2; hh++)
                     {
-                        v[hh][0] = in[hh] ? C0[ro[hh]] : 0.0;
-                        v[hh][1] = in[hh] && two ? C1[ro[hh]] : 0.0;
+                        const int m = ((i0 + x)*WGM + wm)*16 + 8*hh + fr;
+                        in[x][hh] = m < t.mrem;
+                        ro[x][hh] = in[x][hh] ? __ldg(c.c_m + t.m0 + m) : 0;
                     }
+                if (beta != 0.0)
+                {
                     #pragma unroll
-                    for (int hh = 0; hh < 2; hh++)
+                    for (int x = 0; x < IB; x++)
                         #pragma unroll
-                        for (int q = 0; q < 2; q++) v[hh][q] = alpha*acc[i][j][2*hh + q] + beta*v[hh][q];
+                        for (int hh = 0; hh < 2; hh++)
+                        {
+                            v[x][hh][0] = in[x][hh] ? __ldcg(C0 + ro[x][hh]) : 0.0;
+                            v[x][hh][1] = in[x][hh] && two ? __ldcg(C1 + ro[x][hh]) : 0.0;
+                        }
+                    #pragma unroll
+                    for (int x = 0; x < IB; x++)
+                        #pragma unroll
+                        for (int hh = 0; hh < 2; hh++)
+                            #pragma unroll
+                            for (int q = 0; q < 2; q++) v[x][hh][q] = alpha*acc[i0 + x][j][2*hh + q] + beta*v[x][hh][q];
                 }
                 else
                 {
                     #pragma unroll
-                    for (int hh = 0; hh < 2; hh++)
+                    for (int x = 0; x < IB; x++)
                         #pragma unroll
-                        for (int q = 0; q < 2; q++) v[hh][q] = alpha*acc[i][j][2*hh + q];
+                        for (int hh = 0; hh < 2; hh++)
+                            #pragma unroll
+                            for (int q = 0; q < 2; q++) v[x][hh][q] = alpha*acc[i0 + x][j][2*hh + q];
                 }
                 #pragma unroll
-                for (int hh = 0; hh < 2; hh++)
-                {
-                    if (in[hh]) C0[ro[hh]] = v[hh][0];
-                    if (in[hh] && two) C1[ro[hh]] = v[hh][1];
-                }
+                for (int x = 0; x < IB; x++)
+                    #pragma unroll
+                    for (int hh = 0; hh < 2; hh++)
+                    {
+                        if (in[x][hh]) C0[ro[x][hh]] = v[x][hh][0];
+                        if (in[x][hh] && two) C1[ro[x][hh]] = v[x][hh][1];
+                    }
             }
         }
     }
@@ -1296,7 +1314,7 @@ double split_work(GemmF64Args& a, int sms, size_t ws_limit)
     // 4000 with k 16 64 and 64, k 64 109 and 135, k 500 557 and 559; 2000 x 2000 with k
     // 200 77 and 98; 40000 x 100 with k 500 217 and 190. (2000 cycles a tile and 26000 a
     // cut, as assumed before, cut 2000 x 2000 from k 200 on.)
-    constexpr double kOut = 9, kRun = 700, kFixup = 12000, kChip = 1700, kUnit = 32;
+    constexpr double kOut = 9, kRun = 700, kFixup = 15000, kChip = 1700, kUnit = 32;
     constexpr size_t kSlot = (size_t)T::BM*T::BN*sizeof(double);
     const i64 N = a.cplx ? 2*a.N : a.N;
     const i64 fm = a.M/T::BM, fn = N/T::BN, L = a.L;
